@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "df64.cuh"
+#include "fx64.cuh"
 #include "lpg_common.cuh"
 #include "lpg_internal.hpp"
 
@@ -388,20 +389,341 @@ ax_hex_staged_kernel(const int64_t Nelements, const int32_t* __restrict__ elemen
   cp_async_wait<0>();
 }
 
-// ---------------------------------------------------------------- FP64 even-odd variant
-// GLL derivative matrices satisfy D[N-i][N-m] = -D[i][m], and so does D^T. Splitting a
-// line q_0..q_N into e_m = q_m + q_{N-m} and o_m = q_m - q_{N-m} (m < H = Nq/2), the two
-// outputs t and N-t of D q are A + B and B - A with A = sum_m Dp[t][m] e_m,
-// B = sum_m Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m]) / 2: Nq FMA for two
-// outputs instead of 2 Nq. GB300's FP64 operator is bound by the FP64 pipe, so the
-// operation count is the lever: 49 instead of 59 FP64 operations per node at N = 7.
+// Barrier over the threads of one element where they are whole warps, else over the CTA.
+// The barrier numbers are immediates: a number in a register reserves all 16 of a CTA's
+// barriers, and an SM's 64 then hold only 4 CTAs.
+template <int NQ, int EPB>
+__device__ __forceinline__ void ax_fx_sync(const int el) {
+  if constexpr ((NQ * NQ) % 32 == 0 && EPB == 2) {
+    if (el == 0) asm volatile("bar.sync 1, %0;\n" ::"n"(NQ * NQ) : "memory");
+    else asm volatile("bar.sync 2, %0;\n" ::"n"(NQ * NQ) : "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------- FP64 block fixed-point kernel
+// The FP64 operator with its contractions in block fixed point (fx64.cuh). Every 1-D line
+// of an element is converted once to 64-bit integers on the exponent of its largest entry,
+// contracted with D (or D^T) by integer multiply-adds, and converted back; the metric
+// product G . grad q and the mass term stay in FP64.
 //
-// Per layer k of an element, thread (i, j) forms one even/odd value of its row (partner
-// (N-i, j) is lane ^ (Nq-1)) and one of its column (partner (i, N-j) is lane ^ 2Nq: the
-// row map eo_row puts rows j and N-j in the same warp); then threads with i < H take
-// the r-derivative pair (i, N-i) of row j and threads with i >= H the s-derivative pair
-// (i-H, N-i+H) of column j. The t-direction works on the register pencil. The
-// transposed derivatives repeat the pattern with D^T. Nq = 4 or 8 (N = 3, 7).
+// One thread holds one line at a time: thread l of an element takes line l of the r, then
+// of the s, then of the t direction, through FP64 copies of the element in shared memory.
+// Line maxima, even/odd sums and all integers of a line are then the thread's own registers,
+// and an element needs 4 barriers.
+// What bounds it (N = 7): the FP64 pipe again, at the 9 FP64 operations a node of the metric
+// product and 1 of the mass term against 50 of the FP64 kernel it replaced, closely followed
+// by issue (570 instructions a node). 64^3, N = 7, lambda = 1: 3.25 ms against 11.31 ms;
+// 31 x 23 x 29, N = 5, lambda field: 143 us against 363 us; 64^3, N = 3: 363 us against 1037 us
+// of the direct kernel. Requesting the factors of a later element (one wave ahead) from L2
+// instead of this element's was slower (48^3: 1.53 against 1.37 ms).
+//   S[2] = q;  S[0..2] = D_r q, D_s q, D_t q (the last in place);  then the three rows of
+//   G . grad q;  then the transposed derivatives as integers (exponents in s_x), summed on
+//   their common exponent. q is gathered again for the mass term.
+// Nq = 4, 8: the GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
+// with e_m = q_m + q_{N-m}, o_m = q_m - q_{N-m} (m < H = Nq/2), outputs t and N-t are A + B
+// and B - A, A = sum Dp[t][m] e_m, B = sum Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m])/2.
+template <int NQ>
+struct FxLayout {
+  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ, H = NQ / 2;
+  static constexpr bool EO = (NQ == 4 || NQ == 8);
+  static constexpr int P = NQ | 1, PL = P * NQ;      // odd row pitch: conflict-free lines
+  static constexpr int ROWS = EO ? H : NQ;           // rows of a table
+  static constexpr int COLS = EO ? 2 * H : NQ;       // (Dp, Dm) interleaved, or D
+  // Bits S (fx64.cuh) of a line value (FS) and a table entry (DS): as many as keep the halves
+  // in 32 bits and, for any D, the sum of the middle quarters, COLS (EO: H per sum) products
+  // of each kind, and the sum of three transposed lines below 2^63. The mirror sums double a
+  // line value and a table entry (2 Dp).
+  static constexpr int FS = NQ <= 3 ? 8 : 7;
+  static constexpr int DS = NQ == 2 || NQ == 4 ? 8 : NQ == 9 ? 6 : 7;
+  static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
+  static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
+  static constexpr int NT = NL * EPB;
+  // resident CTAs per SM to compile for (registers): measured best of 5, 6, 7, 8
+  static constexpr int MINB = NQ == 9 ? 5 : 7;
+};
+
+// D (trans = false) or D^T in the layout's table: entry c of row t (2 Dp, 2 Dm)
+template <int NQ>
+__device__ __forceinline__ double fx_table_entry(const double* __restrict__ Dg, bool trans, int t, int c) {
+  using L = FxLayout<NQ>;
+  const int rs = trans ? 1 : NQ, cs = trans ? NQ : 1;
+  if constexpr (L::EO) {
+    const int m = c >> 1;
+    const double d0 = Dg[t * rs + m * cs], d1 = Dg[t * rs + (NQ - 1 - m) * cs];
+    return (c & 1) ? d0 - d1 : d0 + d1;
+  } else {
+    return Dg[t * rs + c * cs];
+  }
+}
+
+// emit(t, sum_m table[t][m] q[m]) for the outputs t of one line, as integers in units of
+// 2^(eL + eR[t] - EXP)
+template <int NQ, typename F>
+__device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, const fx_half* __restrict__ tab,
+                                        F&& emit) {
+  using L = FxLayout<NQ>;
+  constexpr int N = NQ - 1, H = L::H;
+  int64_t f[NQ];
+#pragma unroll
+  for (int m = 0; m < NQ; ++m) f[m] = fx_from_double<L::FS + 1>(q[m], eL);
+  fx_half x[NQ];
+  if constexpr (L::EO) {
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      x[2 * m] = fx_split(f[m] + f[N - m]);
+      x[2 * m + 1] = fx_split(f[m] - f[N - m]);
+    }
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      fx_acc A, B;
+      const int4* row = reinterpret_cast<const int4*>(tab + t * L::COLS);
+      fx_half dp[H], dm[H];
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const int4 v = row[m];
+        dp[m] = {v.x, v.y};
+        dm[m] = {v.z, v.w};
+        A.cross(x[2 * m], dp[m]);
+        B.cross(x[2 * m + 1], dm[m]);
+      }
+      A.fold();
+      B.fold();
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        A.high(x[2 * m], dp[m]);
+        B.high(x[2 * m + 1], dm[m]);
+      }
+      emit(t, A.v + B.v);
+      emit(N - t, B.v - A.v);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) x[m] = fx_split(f[m]);
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) {
+      fx_acc A;
+      fx_half d[NQ];
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) {
+        d[m] = tab[t * L::COLS + m];
+        A.cross(x[m], d[m]);
+      }
+      A.fold();
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) A.high(x[m], d[m]);
+      emit(t, A.v);
+    }
+  }
+}
+
+// a line of zeros (as the masked lines of Dirichlet faces are): no magnitude bit is set
+template <int NQ>
+__device__ __forceinline__ bool fx_zero(const double (&v)[NQ], const unsigned key) {
+  int lo = 0;
+#pragma unroll
+  for (int m = 0; m < NQ; ++m) lo |= __double2loint(v[m]);
+  return key == 0 && lo == 0;
+}
+
+// row of the table that output t of a line uses
+template <int NQ>
+__device__ __forceinline__ constexpr int fx_row(int t) {
+  return FxLayout<NQ>::EO && t >= NQ / 2 ? NQ - 1 - t : t;
+}
+
+// MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
+// UNIT: lambda == 1 without a lambda field, the mass term is wJ q
+template <int NQ, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+__global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB)
+ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
+                 const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
+                 const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
+                 const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
+                 double* __restrict__ out) {
+  using L = FxLayout<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, P = L::P, PL = L::PL, EPB = L::EPB, NT = L::NT;
+  constexpr int TAB = L::ROWS * L::COLS;
+  extern __shared__ __align__(16) unsigned char fx_smem[];
+  __shared__ __align__(16) fx_half s_tab[2][TAB];   // D, D^T
+  __shared__ int s_e[2][L::ROWS];                   // biased exponents of their rows
+  __shared__ int s_x[EPB][3][NL];                   // exponents of the transposed lines, -1: FP64 values
+  __shared__ int s_plain;                           // D beyond 2^63: every line in FP64
+  const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
+  if (tid == 0) s_plain = 0;
+  __syncthreads();
+  double* S = reinterpret_cast<double*>(fx_smem) + el * (3 * PL * NQ);
+  const int a = l % NQ, b = l / NQ;
+
+  int64_t e = (int64_t)blockIdx.x * EPB + el;
+  const bool active = e < Nelements;
+  if (active && elementList) e = elementList[e];
+  if (!active) e = 0;
+  const int64_t nodeBase = e * NP + l;
+  if (active && l == 0) {
+    prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(double));
+    if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(double));
+  }
+  {
+    double v[NQ];
+    if constexpr (INMODE == IN_GATHER) {
+      int32_t id[NQ];
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) v[k] = id[k] >= 0 ? q[id[k]] : 0.0;
+    } else {
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) v[k] = active ? q[nodeBase + k * NL] : 0.0;
+    }
+    // tables of D and D^T while the gather is in flight
+    for (int w = tid; w < 2 * TAB; w += NT) {
+      const int tr = w / TAB, t = (w % TAB) / L::COLS, c = w % L::COLS;
+      unsigned key = 0;
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) key = max(key, fx_key(Dg[tr ? m * NQ + t : t * NQ + m]));
+      const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
+      s_tab[tr][t * L::COLS + c] = fx_split(fx_from_double<L::DS + 1>(fx_table_entry<NQ>(Dg, tr, t, c), eR));
+      if (c == 0) s_e[tr][t] = eR;
+      if (eR > 1086) s_plain = 1;
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) S[(2 * NQ + k) * PL + b * P + a] = v[k];
+  }
+  __syncthreads();
+
+  // D q along r, s, t
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    if (d == 2) ax_fx_sync<NQ, EPB>(el);   // the t-lines overwrite q
+    const int st = d == 0 ? 1 : d == 1 ? P : PL;
+    const int base = a * (d == 0 ? P : 1) + b * (d == 2 ? P : PL);
+    const double* in = S + 2 * PL * NQ + base;
+    double* o = S + d * PL * NQ + base;
+    double v[NQ];
+    unsigned key = 0;
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) {
+      v[m] = in[m * st];
+      key = max(key, fx_key(v[m]));
+    }
+    const int eL = (int)(key >> 20);
+    asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
+    if (fx_ordinary(eL) && !s_plain) {
+      fx_line<NQ>(v, eL, s_tab[0], [&](int t, int64_t r) {
+        o[t * st] = fx_to_double(r, fx_base(eL + s_e[0][fx_row<NQ>(t)] - (L::EXP - 1086)));
+      });
+    } else if (fx_zero<NQ>(v, key)) {
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) o[t * st] = 0.0;
+    } else {
+#pragma unroll 1
+      for (int t = 0; t < NQ; ++t) {
+        double r = 0;
+#pragma unroll
+        for (int m = 0; m < NQ; ++m) r += Dg[t * NQ + m] * v[m];
+        o[t * st] = r;
+      }
+    }
+  }
+  ax_fx_sync<NQ, EPB>(el);
+
+  // G . grad q
+  {
+    const double* gp = ggeo + e * geoStride + l;
+    double* s = S + b * P + a;
+#pragma unroll 4
+    for (int k = 0; k < NQ; ++k) {
+      double G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0;
+      if (active) {
+        G00 = gp[0 * NP + k * NL]; G01 = gp[1 * NP + k * NL]; G02 = gp[2 * NP + k * NL];
+        G11 = gp[3 * NP + k * NL]; G12 = gp[4 * NP + k * NL]; G22 = gp[5 * NP + k * NL];
+      }
+      double* c = s + k * PL;
+      const double qr = c[0], qs = c[PL * NQ], qt = c[2 * PL * NQ];
+      c[0] = G00 * qr + G01 * qs + G02 * qt;
+      c[PL * NQ] = G01 * qr + G11 * qs + G12 * qt;
+      c[2 * PL * NQ] = G02 * qr + G12 * qs + G22 * qt;
+    }
+  }
+  ax_fx_sync<NQ, EPB>(el);
+
+  // D^T along r, s, t, left as integers
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    const int st = d == 0 ? 1 : d == 1 ? P : PL;
+    double* in = S + d * PL * NQ + a * (d == 0 ? P : 1) + b * (d == 2 ? P : PL);
+    double v[NQ];
+    unsigned key = 0;
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) {
+      v[m] = in[m * st];
+      key = max(key, fx_key(v[m]));
+    }
+    const int eL = (int)(key >> 20);
+    int x = eL;
+    asm volatile("" ::: "memory");
+    if (fx_ordinary(eL) && !s_plain) {
+      fx_line<NQ>(v, eL, s_tab[1], [&](int t, int64_t r) { in[t * st] = __longlong_as_double(r); });
+    } else if (fx_zero<NQ>(v, key)) {
+      x = 128;
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) in[t * st] = 0.0;
+    } else {
+      x = -1;
+#pragma unroll 1
+      for (int t = 0; t < NQ; ++t) {
+        double r = 0;
+#pragma unroll
+        for (int m = 0; m < NQ; ++m) r += Dg[m * NQ + t] * v[m];
+        in[t * st] = r;
+      }
+    }
+    s_x[el][d][l] = x;
+  }
+  ax_fx_sync<NQ, EPB>(el);
+
+  if (!active) return;
+  const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
+  const double* wp = wJ + e * wJStride + l;
+  const int er = s_e[1][fx_row<NQ>(a)], es = s_e[1][fx_row<NQ>(b)];
+  const double* s = S + b * P + a;
+#pragma unroll 4
+  for (int k = 0; k < NQ; ++k) {
+    const double* c = s + k * PL;
+    const int lr = s_x[el][0][b + NQ * k], ls = s_x[el][1][a + NQ * k], lt = s_x[el][2][l];
+    const int xr = lr + er, xs = ls + es, xt = lt + s_e[1][fx_row<NQ>(k)];
+    const double vr = c[0], vs = c[PL * NQ], vt = c[2 * PL * NQ];
+    double r;
+    if ((lr | ls | lt) >= 0) {
+      const int X = max(xr, max(xs, xt));
+      const int64_t sum = fx_shr(__double_as_longlong(vr), X - xr) + fx_shr(__double_as_longlong(vs), X - xs) +
+                          fx_shr(__double_as_longlong(vt), X - xt);
+      r = fx_to_double(sum, fx_base(X - (L::EXP - 1086)));
+    } else {
+      r = (lr < 0 ? vr : fx_to_double(__double_as_longlong(vr), fx_base(xr - (L::EXP - 1086)))) +
+          (ls < 0 ? vs : fx_to_double(__double_as_longlong(vs), fx_base(xs - (L::EXP - 1086)))) +
+          (lt < 0 ? vt : fx_to_double(__double_as_longlong(vt), fx_base(xt - (L::EXP - 1086))));
+    }
+    int32_t id = 0;
+    if constexpr (OUTMODE == OUT_ASSEMBLE || (MASS && INMODE == IN_GATHER)) id = __ldg(g2l + nodeBase + k * NL);
+    if constexpr (MASS) {
+      double v = 0.0;
+      if constexpr (INMODE == IN_GATHER) v = id >= 0 ? q[id] : 0.0;
+      else v = q[nodeBase + k * NL];
+      r = fma(UNIT ? wp[k * NL] : wp[k * NL] * lam, v, r);
+    }
+    if constexpr (OUTMODE == OUT_ASSEMBLE) {
+      if (id >= 0) atomicAdd(out + id, r);
+    } else if constexpr (OUTMODE == OUT_LOCAL) {
+      out[nodeBase + k * NL] = r;
+    } else {
+      out[nodeBase + k * NL] -= r;
+    }
+  }
+}
+
 template <int NQ>
 __device__ __forceinline__ int eo_row(const int jj) {
   const int lo = 2 * (jj >> 2) + (jj & 1);
@@ -412,179 +734,6 @@ template <int NQ>
 __device__ __forceinline__ void eo_sync(const int el) {
   if constexpr ((NQ * NQ) % 32 == 0) elem_sync<NQ>(el);  // Nq = 8: the element's two warps
   else __syncwarp();                                    // Nq = 4: an element is half a warp
-}
-
-// MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
-// UNIT: lambda == 1 without a lambda field, the mass term is wJ q (one FP64 multiply fewer
-// per node, the same result: wJ * 1.0 is exact)
-template <int NQ, bool MASS = true, bool UNIT = false>
-__global__ void __launch_bounds__(NQ * NQ * elems_per_block<NQ>(), 3)
-ax_hex_eo_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
-                 const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
-                 const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
-                 const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
-                 double* __restrict__ out) {
-  static_assert(NQ == 4 || NQ == 8, "even-odd kernel: Nq = 4 or 8");
-  constexpr int NP = NQ * NQ * NQ, H = NQ / 2, N = NQ - 1;
-  constexpr int EPB = elems_per_block<NQ>();
-  constexpr unsigned FULL = 0xffffffffu;
-  __shared__ double s_Dp[H][H], s_Dm[H][H];   // even/odd tables of D
-  __shared__ double s_Tp[H][H], s_Tm[H][H];   // and of D^T
-  __shared__ double s_R[EPB][NQ][NQ];         // row j: e_0..e_{H-1}, o_0..o_{H-1} along i
-  __shared__ double s_S[EPB][NQ][NQ];         // column i: the same along j
-  __shared__ double s_dr[EPB][NQ][NQ];        // [j][i] r-derivative, then r-transposed term
-  __shared__ double s_ds[EPB][NQ][NQ];        // [j][i] s-derivative, then s-transposed term
-  // per-thread pencils of D_t q and of G_t . grad q, [k][thread] (kept out of registers so
-  // that three CTAs fit on an SM: the FP64 pipe needs the warps)
-  __shared__ double s_qt[NQ][NQ * NQ * EPB];
-  __shared__ double s_gt[NQ][NQ * NQ * EPB];
-
-  const int i = threadIdx.x, jj = threadIdx.y, el = threadIdx.z;
-  const int j = eo_row<NQ>(jj);
-  const int tid = i + NQ * (jj + NQ * el);
-  for (int t = tid; t < H * H; t += NQ * NQ * EPB) {
-    const int a = t / H, m = t % H;
-    const double d0 = Dg[a * NQ + m], d1 = Dg[a * NQ + N - m];     // D[a][m], D[a][N-m]
-    const double t0 = Dg[m * NQ + a], t1 = Dg[(N - m) * NQ + a];   // D^T[a][m], D^T[a][N-m]
-    s_Dp[a][m] = 0.5 * (d0 + d1);
-    s_Dm[a][m] = 0.5 * (d0 - d1);
-    s_Tp[a][m] = 0.5 * (t0 + t1);
-    s_Tm[a][m] = 0.5 * (t0 - t1);
-  }
-
-  int64_t e = (int64_t)blockIdx.x * EPB + el;
-  const bool active = e < Nelements;
-  if (active && elementList) e = elementList[e];
-  if (!active) e = 0;
-
-  double r_q[NQ], r_Aq[NQ];
-  int32_t r_id[NQ];
-  const int64_t nodeBase = e * NP + j * NQ + i;
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    const int32_t id = active ? __ldg(g2l + nodeBase + k * NQ * NQ) : -1;
-    r_id[k] = id;
-    r_q[k] = (id >= 0) ? q[id] : 0.0;
-  }
-  const double lam = (lambdaE && active) ? lambdaE[e] : lambda;
-  const double* gp = ggeo + e * geoStride + j * NQ + i;
-  const double* wp = wJ + e * wJStride + j * NQ + i;
-  __syncthreads();
-
-  // t-direction of the pencil, even/odd
-  {
-    double E[H], O[H];
-#pragma unroll
-    for (int m = 0; m < H; ++m) {
-      E[m] = r_q[m] + r_q[N - m];
-      O[m] = r_q[m] - r_q[N - m];
-    }
-#pragma unroll
-    for (int t = 0; t < H; ++t) {
-      double A = 0, B = 0;
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A += s_Dp[t][m] * E[m];
-        B += s_Dm[t][m] * O[m];
-      }
-      s_qt[t][tid] = A + B;
-      s_qt[N - t][tid] = B - A;
-    }
-  }
-
-  // the pair task of this thread: r-pair of row j (i < H) or s-pair of column j (i >= H)
-  const bool rtask = i < H;
-  const int pt = rtask ? i : i - H;
-  double* dst0 = rtask ? &s_dr[el][j][pt] : &s_ds[el][pt][j];
-  double* dst1 = rtask ? &s_dr[el][j][N - pt] : &s_ds[el][N - pt][j];
-  const double* line = rtask ? &s_R[el][j][0] : &s_S[el][j][0];
-  // even/odd slot of this thread's node in its row (along i) and column (along j): the
-  // value is partner + sign * own (e for the first half, o for the second), written
-  // without branches so that no FP64 instruction issues twice in a diverged warp
-  const int slotR = (i < H) ? i : H + N - i, slotS = (j < H) ? j : H + N - j;
-  const double sgnR = (i < H) ? 1.0 : -1.0, sgnS = (j < H) ? 1.0 : -1.0;
-
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    const int off = k * NQ * NQ;
-    double G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0, GwJ = 0;
-    if (active) {
-      G00 = gp[0 * NP + off]; G01 = gp[1 * NP + off]; G02 = gp[2 * NP + off];
-      G11 = gp[3 * NP + off]; G12 = gp[4 * NP + off]; G22 = gp[5 * NP + off];
-      if constexpr (MASS) GwJ = wp[off];
-    }
-    // even/odd values of q along i (row j) and along j (column i)
-    const double v = r_q[k];
-    const double pr = __shfl_xor_sync(FULL, v, NQ - 1);
-    const double ps = __shfl_xor_sync(FULL, v, 2 * NQ);
-    s_R[el][j][slotR] = fma(sgnR, v, pr);
-    s_S[el][i][slotS] = fma(sgnS, v, ps);
-    eo_sync<NQ>(el);
-    {
-      double A = 0, B = 0;
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A += s_Dp[pt][m] * line[m];
-        B += s_Dm[pt][m] * line[H + m];
-      }
-      *dst0 = A + B;
-      *dst1 = B - A;
-    }
-    eo_sync<NQ>(el);
-    const double qr = s_dr[el][j][i], qs = s_ds[el][j][i], qtk = s_qt[k][tid];
-    const double Gqr = G00 * qr + G01 * qs + G02 * qtk;
-    const double Gqs = G01 * qr + G11 * qs + G12 * qtk;
-    s_gt[k][tid] = G02 * qr + G12 * qs + G22 * qtk;
-    // even/odd values of Gqr along i and of Gqs along j for the transposed derivatives
-    const double pr2 = __shfl_xor_sync(FULL, Gqr, NQ - 1);
-    const double ps2 = __shfl_xor_sync(FULL, Gqs, 2 * NQ);
-    s_R[el][j][slotR] = fma(sgnR, Gqr, pr2);
-    s_S[el][i][slotS] = fma(sgnS, Gqs, ps2);
-    eo_sync<NQ>(el);
-    {
-      double A = 0, B = 0;
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A += s_Tp[pt][m] * line[m];
-        B += s_Tm[pt][m] * line[H + m];
-      }
-      *dst0 = A + B;
-      *dst1 = B - A;
-    }
-    eo_sync<NQ>(el);
-    // the mass term lambda wJ q folded into the sum as one FMA
-    const double sum = s_dr[el][j][i] + s_ds[el][j][i];
-    if constexpr (MASS && UNIT) r_Aq[k] = fma(GwJ, v, sum);
-    else if constexpr (MASS) r_Aq[k] = fma(GwJ * lam, v, sum);
-    else r_Aq[k] = sum;
-  }
-
-  // transposed t-direction: r_Aq[t] += sum_m D[m][t] Gqt[m], even/odd
-  {
-    double E[H], O[H];
-#pragma unroll
-    for (int m = 0; m < H; ++m) {
-      const double g0 = s_gt[m][tid], g1 = s_gt[N - m][tid];
-      E[m] = g0 + g1;
-      O[m] = g0 - g1;
-    }
-#pragma unroll
-    for (int t = 0; t < H; ++t) {
-      double A = 0, B = 0;
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A += s_Tp[t][m] * E[m];
-        B += s_Tm[t][m] * O[m];
-      }
-      r_Aq[t] += A + B;
-      r_Aq[N - t] += B - A;
-    }
-  }
-
-  if (!active) return;
-#pragma unroll
-  for (int k = 0; k < NQ; ++k)
-    if (r_id[k] >= 0) atomicAdd(out + r_id[k], r_Aq[k]);
 }
 
 // ---------------------------------------------------------------- double-word variant
@@ -1155,13 +1304,44 @@ static bool staged_ok(const AxArgs<T, G>& a) {
          ((a.wJStride * (int64_t)sizeof(G)) % 16 == 0);
 }
 
-// LPG_AX_FP64 = direct: tuning override back to the direct-contraction FP64 kernel
+// LPG_AX_FP64 = direct: tuning override back to the direct-contraction FP64 kernel (ax_hex_kernel)
 static bool fp64_direct_override() {
   static const bool direct = [] {
     const char* e = std::getenv("LPG_AX_FP64");
     return e && !std::strcmp(e, "direct");
   }();
   return direct;
+}
+
+template <int NQ, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+static int fx_config(KernelConfig* cfg, size_t* smem) {
+  using L = FxLayout<NQ>;
+  static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in, occupancy
+  auto kern = ax_hex_fx_kernel<NQ, INMODE, OUTMODE, MASS, UNIT>;
+  const size_t bytes = sizeof(double) * 3 * L::PL * NQ * L::EPB;
+  *smem = bytes;
+  return perDevice.get(
+      [&](int, KernelConfig& c) {
+        LPG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        LPG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.ctasPerSM, kern, L::NT, bytes));
+        return (int)LPG_OK;
+      },
+      cfg);
+}
+
+template <int NQ, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+static int launch_fx(const AxArgs<double, double>& a, cudaStream_t s) {
+  using L = FxLayout<NQ>;
+  KernelConfig cfg;
+  size_t smem;
+  const int rc = fx_config<NQ, INMODE, OUTMODE, MASS, UNIT>(&cfg, &smem);
+  if (rc) return rc;
+  const int64_t blocks = (a.Nelements + L::EPB - 1) / L::EPB;
+  if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
+  ax_hex_fx_kernel<NQ, INMODE, OUTMODE, MASS, UNIT><<<(unsigned)blocks, L::NT, smem, s>>>(
+      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out);
+  LPG_LAUNCH_CHECK("ax_hex_fx_kernel");
+  return LPG_OK;
 }
 
 template <int NQ, typename T, typename G, int INMODE, int OUTMODE>
@@ -1191,23 +1371,11 @@ static int launch_ax(const AxArgs<T, G>& a, cudaStream_t s) {
   const int64_t blocks = (a.Nelements + EPB - 1) / EPB;
   if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
   dim3 block(NQ, NQ, EPB);
-  if constexpr (std::is_same<T, double>::value && std::is_same<G, double>::value && INMODE == IN_GATHER &&
-                OUTMODE == OUT_ASSEMBLE && (NQ == 4 || NQ == 8)) {
+  if constexpr (std::is_same<T, double>::value) {
     if (!fp64_direct_override()) {
-      if (a.lambda == 0.0 && !a.lambdaE)
-        ax_hex_eo_kernel<NQ, false><<<(unsigned)blocks, block, 0, s>>>(a.Nelements, a.elementList, a.g2l, a.ggeo,
-                                                                      a.geoStride, a.wJ, a.wJStride, a.D, a.lambda,
-                                                                      a.lambdaE, a.q, a.out);
-      else if (a.lambda == 1.0 && !a.lambdaE)
-        ax_hex_eo_kernel<NQ, true, true><<<(unsigned)blocks, block, 0, s>>>(a.Nelements, a.elementList, a.g2l,
-                                                                           a.ggeo, a.geoStride, a.wJ, a.wJStride,
-                                                                           a.D, a.lambda, a.lambdaE, a.q, a.out);
-      else
-        ax_hex_eo_kernel<NQ, true><<<(unsigned)blocks, block, 0, s>>>(a.Nelements, a.elementList, a.g2l, a.ggeo,
-                                                                     a.geoStride, a.wJ, a.wJStride, a.D, a.lambda,
-                                                                     a.lambdaE, a.q, a.out);
-      LPG_LAUNCH_CHECK("ax_hex_eo_kernel");
-      return LPG_OK;
+      if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, INMODE, OUTMODE, false, false>(a, s);
+      if (a.lambda == 1.0 && !a.lambdaE) return launch_fx<NQ, INMODE, OUTMODE, true, true>(a, s);
+      return launch_fx<NQ, INMODE, OUTMODE, true, false>(a, s);
     }
   }
   ax_hex_kernel<NQ, T, G, INMODE, OUTMODE><<<(unsigned)blocks, block, 0, s>>>(
@@ -1252,42 +1420,40 @@ int ax_hex(const AxArgs<T, G>& a, AxMode mode, cudaStream_t s) {
 }
 
 template <int NQ>
-static cudaError_t fp64_occupancy(int* per, bool dw, bool mass, int epb) {
-  if (dw) {
-    if constexpr (NQ == 8) {
-      return dw7_classic()
-                 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, ax_hex_dw_kernel<8, true>, NQ * NQ * epb, 0)
-                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, ax_hex_dw_lean_kernel<8, true>, NQ * NQ * epb,
-                                                                 0);
-    } else {
-      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, ax_hex_dw_kernel<NQ>, NQ * NQ * epb, 0);
-    }
-  }
-  if (fp64_direct_override())
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        per, ax_hex_kernel<NQ, double, double, IN_GATHER, OUT_ASSEMBLE>, NQ * NQ * epb, 0);
-  return mass ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, ax_hex_eo_kernel<NQ, true>, NQ * NQ * epb, 0)
-              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, ax_hex_eo_kernel<NQ, false>, NQ * NQ * epb, 0);
-}
-
-int ax_wave_elements(int N, bool dw, bool mass) {
-  int dev = 0, sms = 0, per = 0;
+static int wave_elements(bool dw, bool mass) {
+  int dev = 0, sms = 0, per = 0, epb = elems_per_block<NQ>();
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 1;
-  cudaError_t e = cudaErrorInvalidValue;
-  int epb = 1;
-  if (N == 7) {
-    epb = elems_per_block<8>();
-    e = fp64_occupancy<8>(&per, dw, mass, epb);
-  } else if (N == 3) {
-    epb = elems_per_block<4>();
-    e = fp64_occupancy<4>(&per, dw, mass, epb);
+  cudaError_t e = cudaSuccess;
+  if (dw) {
+    if constexpr (NQ == 8)
+      e = dw7_classic()
+              ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_dw_kernel<8, true>, NQ * NQ * epb, 0)
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_dw_lean_kernel<8, true>, NQ * NQ * epb, 0);
+    else
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_dw_kernel<NQ>, NQ * NQ * epb, 0);
+  } else if (fp64_direct_override()) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_kernel<NQ, double, double, IN_GATHER, OUT_ASSEMBLE>,
+                                                      NQ * NQ * epb, 0);
+  } else {
+    KernelConfig cfg;
+    size_t smem;
+    const int rc = mass ? fx_config<NQ, IN_GATHER, OUT_ASSEMBLE, true, false>(&cfg, &smem)
+                        : fx_config<NQ, IN_GATHER, OUT_ASSEMBLE, false, false>(&cfg, &smem);
+    per = rc ? 0 : cfg.ctasPerSM;
+    epb = FxLayout<NQ>::EPB;
   }
   if (e != cudaSuccess || per < 1) {
     cudaGetLastError();
     return 1;
   }
   return sms * per * epb;
+}
+
+int ax_wave_elements(int N, bool dw, bool mass) {
+  if (N == 7) return wave_elements<8>(dw, mass);
+  if (N == 3) return wave_elements<4>(dw, mass);
+  return 1;
 }
 
 template int ax_hex<double, double>(const AxArgs<double, double>&, AxMode, cudaStream_t);
