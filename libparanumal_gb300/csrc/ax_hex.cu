@@ -389,16 +389,25 @@ ax_hex_staged_kernel(const int64_t Nelements, const int32_t* __restrict__ elemen
   cp_async_wait<0>();
 }
 
-// Barrier over the threads of one element where they are whole warps, else over the CTA.
-// The barrier numbers are immediates: a number in a register reserves all 16 of a CTA's
-// barriers, and an SM's 64 then hold only 4 CTAs.
+// Barrier over the threads of one element where they are whole warps, else over the CTA;
+// returns whether `any` was set by one of them. The barrier numbers are immediates: a number
+// in a register reserves all 16 of a CTA's barriers, and an SM's 64 then hold only 4 CTAs.
 template <int NQ, int EPB>
-__device__ __forceinline__ void ax_fx_sync(const int el) {
+__device__ __forceinline__ bool ax_fx_sync(const int el, const bool any = false) {
   if constexpr ((NQ * NQ) % 32 == 0 && EPB == 2) {
-    if (el == 0) asm volatile("bar.sync 1, %0;\n" ::"n"(NQ * NQ) : "memory");
-    else asm volatile("bar.sync 2, %0;\n" ::"n"(NQ * NQ) : "memory");
+    int r;
+#define LPG_FX_BARRIER(id)                                                                              \
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %2, 0;\nbarrier.cta.red.or.pred q, " #id ", %1, p;\n" \
+               "selp.s32 %0, 1, 0, q;\n}\n"                                                              \
+               : "=r"(r)                                                                                \
+               : "n"(NQ * NQ), "r"((int)any)                                                            \
+               : "memory")
+    if (el == 0) LPG_FX_BARRIER(1);
+    else LPG_FX_BARRIER(2);
+#undef LPG_FX_BARRIER
+    return r != 0;
   } else {
-    __syncthreads();
+    return __syncthreads_or(any);
   }
 }
 
@@ -414,13 +423,17 @@ __device__ __forceinline__ void ax_fx_sync(const int el) {
 // and an element needs 4 barriers.
 // What bounds it (N = 7): the FP64 pipe again, at the 9 FP64 operations a node of the metric
 // product and 1 of the mass term against 50 of the FP64 kernel it replaced, closely followed
-// by issue (570 instructions a node). 64^3, N = 7, lambda = 1: 3.25 ms against 11.31 ms;
-// 31 x 23 x 29, N = 5, lambda field: 143 us against 363 us; 64^3, N = 3: 363 us against 1037 us
-// of the direct kernel. Requesting the factors of a later element (one wave ahead) from L2
-// instead of this element's was slower (48^3: 1.53 against 1.37 ms).
-//   S[2] = q;  S[0..2] = D_r q, D_s q, D_t q (the last in place);  then the three rows of
-//   G . grad q;  then the transposed derivatives as integers (exponents in s_x), summed on
-//   their common exponent. q is gathered again for the mass term.
+// by the integer pipe (shifts, logic and multiply-adds share 64 lanes a clock; 520
+// instructions a node in all). 48^3, N = 7: 1.31 ms (lambda = 0: 1.20)
+// against 4.78 (4.56); 28^3, N = 5: 156 us against 406 us; 64^3, N = 3: 340 us against 1037 us
+// of the direct kernel. Measured and not kept at 48^3: L2 prefetch of a later element's factors
+// (one wave ahead) 1.53 against 1.37 ms; eight CTAs per SM with swizzled instead of pitched
+// lines 1.37 against 1.37 ms.
+// S holds three copies of the element, each with the lines of one direction contiguous, so
+// one piece of code with immediate offsets serves all three; every step works in place:
+//   q three times;  then D_r q, D_s q, D_t q;  then the three rows of G . grad q;  then the
+//   transposed derivatives as integers (exponents in s_x), summed on their common exponent.
+// q is gathered again for the mass term.
 // Nq = 4, 8: the GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
 // with e_m = q_m + q_{N-m}, o_m = q_m - q_{N-m} (m < H = Nq/2), outputs t and N-t are A + B
 // and B - A, A = sum Dp[t][m] e_m, B = sum Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m])/2.
@@ -477,7 +490,6 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
     }
 #pragma unroll
     for (int t = 0; t < H; ++t) {
-      fx_acc A, B;
       const int4* row = reinterpret_cast<const int4*>(tab + t * L::COLS);
       fx_half dp[H], dm[H];
 #pragma unroll
@@ -485,6 +497,10 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
         const int4 v = row[m];
         dp[m] = {v.x, v.y};
         dm[m] = {v.z, v.w};
+      }
+      fx_acc A(x[0], dp[0]), B(x[1], dm[0]);
+#pragma unroll
+      for (int m = 1; m < H; ++m) {
         A.cross(x[2 * m], dp[m]);
         B.cross(x[2 * m + 1], dm[m]);
       }
@@ -495,7 +511,7 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
         A.high(x[2 * m], dp[m]);
         B.high(x[2 * m + 1], dm[m]);
       }
-      emit(t, A.v + B.v);
+      emit(t, A.v + B.v + 1);   // both were rounded down
       emit(N - t, B.v - A.v);
     }
   } else {
@@ -503,7 +519,7 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
     for (int m = 0; m < NQ; ++m) x[m] = fx_split(f[m]);
 #pragma unroll
     for (int t = 0; t < NQ; ++t) {
-      fx_acc A;
+      fx_acc A(0x40000000ll);   // rounds to nearest
       fx_half d[NQ];
 #pragma unroll
       for (int m = 0; m < NQ; ++m) {
@@ -549,12 +565,14 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
   __shared__ __align__(16) fx_half s_tab[2][TAB];   // D, D^T
   __shared__ int s_e[2][L::ROWS];                   // biased exponents of their rows
   __shared__ int s_x[EPB][3][NL];                   // exponents of the transposed lines, -1: FP64 values
-  __shared__ int s_plain;                           // D beyond 2^63: every line in FP64
   const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
-  if (tid == 0) s_plain = 0;
-  __syncthreads();
   double* S = reinterpret_cast<double*>(fx_smem) + el * (3 * PL * NQ);
   const int a = l % NQ, b = l / NQ;
+  // line l of each copy, and node (a, b, 0) in each; node (a, b, k) is k PL, k PL, k further
+  double* const line = S + b * PL + a * P;
+  double* const nr = S + b * P + a;
+  double* const ns = S + PL * NQ + a * P + b;
+  double* const nt = S + 2 * PL * NQ + b * PL + a * P;
 
   int64_t e = (int64_t)blockIdx.x * EPB + el;
   const bool active = e < Nelements;
@@ -565,6 +583,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
     prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(double));
     if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(double));
   }
+  int plain = 0;
   {
     double v[NQ];
     if constexpr (INMODE == IN_GATHER) {
@@ -577,7 +596,8 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
 #pragma unroll
       for (int k = 0; k < NQ; ++k) v[k] = active ? q[nodeBase + k * NL] : 0.0;
     }
-    // tables of D and D^T while the gather is in flight
+    // tables of D and D^T while the gather is in flight; entries beyond 2^63 leave every
+    // line to FP64
     for (int w = tid; w < 2 * TAB; w += NT) {
       const int tr = w / TAB, t = (w % TAB) / L::COLS, c = w % L::COLS;
       unsigned key = 0;
@@ -586,44 +606,40 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
       const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
       s_tab[tr][t * L::COLS + c] = fx_split(fx_from_double<L::DS + 1>(fx_table_entry<NQ>(Dg, tr, t, c), eR));
       if (c == 0) s_e[tr][t] = eR;
-      if (eR > 1086) s_plain = 1;
+      plain |= eR > 1086;
     }
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) S[(2 * NQ + k) * PL + b * P + a] = v[k];
+    for (int k = 0; k < NQ; ++k) nr[k * PL] = ns[k * PL] = nt[k] = v[k];
   }
-  __syncthreads();
+  plain = __syncthreads_or(plain);
 
   // D q along r, s, t
 #pragma unroll 1
   for (int d = 0; d < 3; ++d) {
-    if (d == 2) ax_fx_sync<NQ, EPB>(el);   // the t-lines overwrite q
-    const int st = d == 0 ? 1 : d == 1 ? P : PL;
-    const int base = a * (d == 0 ? P : 1) + b * (d == 2 ? P : PL);
-    const double* in = S + 2 * PL * NQ + base;
-    double* o = S + d * PL * NQ + base;
+    double* const o = line + d * PL * NQ;
     double v[NQ];
     unsigned key = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) {
-      v[m] = in[m * st];
+      v[m] = o[m];
       key = max(key, fx_key(v[m]));
     }
     const int eL = (int)(key >> 20);
     asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
-    if (fx_ordinary(eL) && !s_plain) {
+    if (fx_ordinary(eL) && !plain) {
       fx_line<NQ>(v, eL, s_tab[0], [&](int t, int64_t r) {
-        o[t * st] = fx_to_double(r, fx_base(eL + s_e[0][fx_row<NQ>(t)] - (L::EXP - 1086)));
+        o[t] = fx_to_double(r, fx_base(eL + s_e[0][fx_row<NQ>(t)] - (L::EXP - 1086)));
       });
     } else if (fx_zero<NQ>(v, key)) {
 #pragma unroll
-      for (int t = 0; t < NQ; ++t) o[t * st] = 0.0;
+      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
     } else {
 #pragma unroll 1
       for (int t = 0; t < NQ; ++t) {
         double r = 0;
 #pragma unroll
         for (int m = 0; m < NQ; ++m) r += Dg[t * NQ + m] * v[m];
-        o[t * st] = r;
+        o[t] = r;
       }
     }
   }
@@ -632,7 +648,6 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
   // G . grad q
   {
     const double* gp = ggeo + e * geoStride + l;
-    double* s = S + b * P + a;
 #pragma unroll 4
     for (int k = 0; k < NQ; ++k) {
       double G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0;
@@ -640,63 +655,66 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
         G00 = gp[0 * NP + k * NL]; G01 = gp[1 * NP + k * NL]; G02 = gp[2 * NP + k * NL];
         G11 = gp[3 * NP + k * NL]; G12 = gp[4 * NP + k * NL]; G22 = gp[5 * NP + k * NL];
       }
-      double* c = s + k * PL;
-      const double qr = c[0], qs = c[PL * NQ], qt = c[2 * PL * NQ];
-      c[0] = G00 * qr + G01 * qs + G02 * qt;
-      c[PL * NQ] = G01 * qr + G11 * qs + G12 * qt;
-      c[2 * PL * NQ] = G02 * qr + G12 * qs + G22 * qt;
+      const double qr = nr[k * PL], qs = ns[k * PL], qt = nt[k];
+      nr[k * PL] = G00 * qr + G01 * qs + G02 * qt;
+      ns[k * PL] = G01 * qr + G11 * qs + G12 * qt;
+      nt[k] = G02 * qr + G12 * qs + G22 * qt;
     }
   }
   ax_fx_sync<NQ, EPB>(el);
 
   // D^T along r, s, t, left as integers
+  bool fp = false;   // a line of this thread kept FP64 values
 #pragma unroll 1
   for (int d = 0; d < 3; ++d) {
-    const int st = d == 0 ? 1 : d == 1 ? P : PL;
-    double* in = S + d * PL * NQ + a * (d == 0 ? P : 1) + b * (d == 2 ? P : PL);
+    double* const o = line + d * PL * NQ;
     double v[NQ];
     unsigned key = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) {
-      v[m] = in[m * st];
+      v[m] = o[m];
       key = max(key, fx_key(v[m]));
     }
     const int eL = (int)(key >> 20);
     int x = eL;
     asm volatile("" ::: "memory");
-    if (fx_ordinary(eL) && !s_plain) {
-      fx_line<NQ>(v, eL, s_tab[1], [&](int t, int64_t r) { in[t * st] = __longlong_as_double(r); });
+    if (fx_ordinary(eL) && !plain) {
+      fx_line<NQ>(v, eL, s_tab[1], [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
     } else if (fx_zero<NQ>(v, key)) {
       x = 128;
 #pragma unroll
-      for (int t = 0; t < NQ; ++t) in[t * st] = 0.0;
+      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
     } else {
       x = -1;
+      fp = true;
 #pragma unroll 1
       for (int t = 0; t < NQ; ++t) {
         double r = 0;
 #pragma unroll
         for (int m = 0; m < NQ; ++m) r += Dg[m * NQ + t] * v[m];
-        in[t * st] = r;
+        o[t] = r;
       }
     }
     s_x[el][d][l] = x;
   }
-  ax_fx_sync<NQ, EPB>(el);
+  int32_t id[NQ];   // in flight over the barrier
+  if constexpr (OUTMODE == OUT_ASSEMBLE || (MASS && INMODE == IN_GATHER)) {
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+  }
+  fp = ax_fx_sync<NQ, EPB>(el, fp);
 
   if (!active) return;
   const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
   const double* wp = wJ + e * wJStride + l;
   const int er = s_e[1][fx_row<NQ>(a)], es = s_e[1][fx_row<NQ>(b)];
-  const double* s = S + b * P + a;
-#pragma unroll 4
+#pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    const double* c = s + k * PL;
     const int lr = s_x[el][0][b + NQ * k], ls = s_x[el][1][a + NQ * k], lt = s_x[el][2][l];
     const int xr = lr + er, xs = ls + es, xt = lt + s_e[1][fx_row<NQ>(k)];
-    const double vr = c[0], vs = c[PL * NQ], vt = c[2 * PL * NQ];
+    const double vr = nr[k * PL], vs = ns[k * PL], vt = nt[k];
     double r;
-    if ((lr | ls | lt) >= 0) {
+    if (!fp || (lr | ls | lt) >= 0) {
       const int X = max(xr, max(xs, xt));
       const int64_t sum = fx_shr(__double_as_longlong(vr), X - xr) + fx_shr(__double_as_longlong(vs), X - xs) +
                           fx_shr(__double_as_longlong(vt), X - xt);
@@ -706,16 +724,14 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
           (ls < 0 ? vs : fx_to_double(__double_as_longlong(vs), fx_base(xs - (L::EXP - 1086)))) +
           (lt < 0 ? vt : fx_to_double(__double_as_longlong(vt), fx_base(xt - (L::EXP - 1086))));
     }
-    int32_t id = 0;
-    if constexpr (OUTMODE == OUT_ASSEMBLE || (MASS && INMODE == IN_GATHER)) id = __ldg(g2l + nodeBase + k * NL);
     if constexpr (MASS) {
       double v = 0.0;
-      if constexpr (INMODE == IN_GATHER) v = id >= 0 ? q[id] : 0.0;
+      if constexpr (INMODE == IN_GATHER) v = id[k] >= 0 ? q[id[k]] : 0.0;
       else v = q[nodeBase + k * NL];
       r = fma(UNIT ? wp[k * NL] : wp[k * NL] * lam, v, r);
     }
     if constexpr (OUTMODE == OUT_ASSEMBLE) {
-      if (id >= 0) atomicAdd(out + id, r);
+      if (id[k] >= 0) atomicAdd(out + id[k], r);
     } else if constexpr (OUTMODE == OUT_LOCAL) {
       out[nodeBase + k * NL] = r;
     } else {

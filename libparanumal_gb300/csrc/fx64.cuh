@@ -33,7 +33,8 @@ __device__ __forceinline__ bool fx_ordinary(int eL) { return (unsigned)(eL - 128
 
 // 2 F of v for S = SH - 1 on a line of biased exponent eL >= 128 (entries so small against
 // the line's largest that nothing is left, zeros and subnormals among them, shift to 0: the
-// PTX shift clamps its amount)
+// PTX shift clamps its amount). Negative values are complemented, not negated: one unit of
+// 2 F, the size of the cut.
 template <int SH>
 __device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
   const int hi = __double2hiint(v), lo = __double2loint(v);
@@ -42,14 +43,17 @@ __device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
   int64_t F;
   asm("{\n"
       ".reg .u32 h, l;\n"
+      ".reg .s32 s;\n"
       ".reg .u64 m;\n"
-      ".reg .pred p;\n"
       "shf.l.wrap.b32 h, %2, %1, %5;\n"
       "shl.b32 l, %2, %5;\n"
       "mov.b64 m, {l, h};\n"
-      "shr.u64 %0, m, %3;\n"
-      "setp.lt.s32 p, %4, 0;\n"
-      "@p neg.s64 %0, %0;\n"
+      "shr.u64 m, m, %3;\n"
+      "shr.s32 s, %4, 31;\n"
+      "mov.b64 {l, h}, m;\n"
+      "xor.b32 l, l, s;\n"
+      "xor.b32 h, h, s;\n"
+      "mov.b64 %0, {l, h};\n"
       "}\n"
       : "=l"(F)
       : "r"(mh), "r"(lo), "r"(n), "r"(hi), "n"(SH));
@@ -74,10 +78,11 @@ __device__ __forceinline__ double fx_to_double(int64_t R, int base) {
       "@p neg.s64 a, a;\n"
       "mov.b64 {l, h}, a;\n"
       "bfind.shiftamt.u32 n, h;\n"          // leading zeros; -1 for 0
-      "setp.eq.u32 z, h, 0;\n"
-      "@z bfind.shiftamt.u32 n, l;\n"
-      "@z add.s32 n, n, 32;\n"
-      "setp.eq.and.s64 z, a, 0, z;\n"
+      "bfind.shiftamt.u32 t, l;\n"
+      "add.s32 t, t, 32;\n"
+      "setp.eq.u32 p, h, 0;\n"
+      "selp.b32 n, t, n, p;\n"
+      "setp.eq.and.u32 z, n, 31, p;\n"     // only 0 has a leading -1 + 32 in its low word
       "shl.b64 a, a, n;\n"
       "mov.b64 {l, h}, a;\n"
       "shf.r.wrap.b32 x, l, h, 11;\n"
@@ -110,20 +115,29 @@ __device__ __forceinline__ fx_half fx_split(int64_t F2) { return {(int)((F2 + 0x
 
 // c + a * b with a 64-bit sum. As PTX: from C++ the halves of a 64-bit value are multiplied
 // as 64-bit integers, three instructions for one.
-__device__ __forceinline__ void fx_mad(int64_t& c, int a, int b) {
-  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(c) : "r"(a), "r"(b));
+__device__ __forceinline__ int64_t fx_mad(int a, int b, int64_t c) {
+  int64_t r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
 }
 
-// sum of products of split integers, in units of 2^62: middle quarters first, then the high
-// ones on top of them, shifted and rounded
+// a * b with a 64-bit product
+__device__ __forceinline__ int64_t fx_mul(int a, int b) {
+  int64_t r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+// sum of products of split integers, in units of 2^62: the middle quarters (started with the
+// first product's), then the high ones on top of them, shifted. The shift rounds down;
+// starting from 2^30 it rounds to nearest.
 struct fx_acc {
-  int64_t v = 0x40000000ll;
-  __device__ __forceinline__ void cross(fx_half a, fx_half b) {
-    fx_mad(v, a.h, b.l);
-    fx_mad(v, a.l, b.h);
-  }
+  int64_t v;
+  __device__ __forceinline__ fx_acc(fx_half a, fx_half b) { v = fx_mad(a.l, b.h, fx_mul(a.h, b.l)); }
+  __device__ __forceinline__ explicit fx_acc(int64_t v0) : v(v0) {}
+  __device__ __forceinline__ void cross(fx_half a, fx_half b) { v = fx_mad(a.l, b.h, fx_mad(a.h, b.l, v)); }
   __device__ __forceinline__ void fold() { v >>= 31; }
-  __device__ __forceinline__ void high(fx_half a, fx_half b) { fx_mad(v, a.h, b.h); }
+  __device__ __forceinline__ void high(fx_half a, fx_half b) { v = fx_mad(a.h, b.h, v); }
 };
 
 }  // namespace lpg
