@@ -50,8 +50,9 @@ def build_ref(force=False, verbose=False):
     oracle/_ref/ref_kernels.c is present."""
     from . import okl_translate as tr
     gen = tr.GENERATED
-    if os.path.isdir(REF_TREE) and (force or not os.path.exists(gen) or
-                                   os.path.getmtime(gen) < os.path.getmtime(tr.__file__)):
+    okl = os.path.join(REF_TREE, "solvers", "elliptic", "okl", "ellipticAxHex3D.okl")
+    if os.path.isfile(okl) and (force or not os.path.exists(gen) or
+                                os.path.getmtime(gen) < os.path.getmtime(tr.__file__)):
         tr.generate(REF_TREE)
     if not os.path.exists(gen):
         return None
