@@ -16,7 +16,7 @@
 #include <type_traits>
 
 #include "df64.cuh"
-#include "fx64.cuh"
+#include "fx_hex.cuh"
 #include "lpg_common.cuh"
 #include "lpg_internal.hpp"
 
@@ -145,12 +145,6 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-// L2 prefetch of `bytes` (a multiple of 16) from global memory; skipped unless the address
-// is 16-byte aligned, as the bulk prefetch requires
-__device__ __forceinline__ void prefetch_l2_bulk(const void* gmem, unsigned bytes) {
-  if (((uintptr_t)gmem & 15u) == 0 && (bytes & 15u) == 0)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(gmem), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -389,38 +383,18 @@ ax_hex_staged_kernel(const int64_t Nelements, const int32_t* __restrict__ elemen
   cp_async_wait<0>();
 }
 
-// Barrier over the threads of one element where they are whole warps, else over the CTA;
-// returns whether `any` was set by one of them. The barrier numbers are immediates: a number
-// in a register reserves all 16 of a CTA's barriers, and an SM's 64 then hold only 4 CTAs.
-template <int NQ, int EPB>
-__device__ __forceinline__ bool ax_fx_sync(const int el, const bool any = false) {
-  if constexpr ((NQ * NQ) % 32 == 0 && EPB == 2) {
-    int r;
-#define LPG_FX_BARRIER(id)                                                                              \
-  asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %2, 0;\nbarrier.cta.red.or.pred q, " #id ", %1, p;\n" \
-               "selp.s32 %0, 1, 0, q;\n}\n"                                                              \
-               : "=r"(r)                                                                                \
-               : "n"(NQ * NQ), "r"((int)any)                                                            \
-               : "memory")
-    if (el == 0) LPG_FX_BARRIER(1);
-    else LPG_FX_BARRIER(2);
-#undef LPG_FX_BARRIER
-    return r != 0;
-  } else {
-    return __syncthreads_or(any);
-  }
-}
-
 // ---------------------------------------------------------------- FP64 block fixed-point kernel
 // The FP64 operator with its contractions in block fixed point (fx64.cuh). Every 1-D line
 // of an element is converted once to 64-bit integers on the exponent of its largest entry,
 // contracted with D (or D^T) by integer multiply-adds, and converted back; the metric
 // product G . grad q and the mass term stay in FP64.
 //
-// One thread holds one line at a time: thread l of an element takes line l of the r, then
-// of the s, then of the t direction, through FP64 copies of the element in shared memory.
-// Line maxima, even/odd sums and all integers of a line are then the thread's own registers,
-// and an element needs 4 barriers.
+// The element sits in three line-contiguous FP64 copies in shared memory and every step works
+// in place, with 4 barriers (fx_hex.cuh):
+//   q three times;  then D_r q, D_s q, D_t q;  then the three rows of G . grad q;  then the
+//   transposed derivatives as integers (exponents in s_x), summed on their common exponent.
+// q is gathered again for the mass term.
+//
 // What bounds it (N = 7): the FP64 pipe again, at the 9 FP64 operations a node of the metric
 // product and 1 of the mass term against 50 of the FP64 kernel it replaced, closely followed
 // by the integer pipe (shifts, logic and multiply-adds share 64 lanes a clock; 520
@@ -429,126 +403,6 @@ __device__ __forceinline__ bool ax_fx_sync(const int el, const bool any = false)
 // of the direct kernel. Measured and not kept at 48^3: L2 prefetch of a later element's factors
 // (one wave ahead) 1.53 against 1.37 ms; eight CTAs per SM with swizzled instead of pitched
 // lines 1.37 against 1.37 ms.
-// S holds three copies of the element, each with the lines of one direction contiguous, so
-// one piece of code with immediate offsets serves all three; every step works in place:
-//   q three times;  then D_r q, D_s q, D_t q;  then the three rows of G . grad q;  then the
-//   transposed derivatives as integers (exponents in s_x), summed on their common exponent.
-// q is gathered again for the mass term.
-// Nq = 4, 8: the GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
-// with e_m = q_m + q_{N-m}, o_m = q_m - q_{N-m} (m < H = Nq/2), outputs t and N-t are A + B
-// and B - A, A = sum Dp[t][m] e_m, B = sum Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m])/2.
-template <int NQ>
-struct FxLayout {
-  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ, H = NQ / 2;
-  static constexpr bool EO = (NQ == 4 || NQ == 8);
-  static constexpr int P = NQ | 1, PL = P * NQ;      // odd row pitch: conflict-free lines
-  static constexpr int ROWS = EO ? H : NQ;           // rows of a table
-  static constexpr int COLS = EO ? 2 * H : NQ;       // (Dp, Dm) interleaved, or D
-  // Bits S (fx64.cuh) of a line value (FS) and a table entry (DS): as many as keep the halves
-  // in 32 bits and, for any D, the sum of the middle quarters, COLS (EO: H per sum) products
-  // of each kind, and the sum of three transposed lines below 2^63. The mirror sums double a
-  // line value and a table entry (2 Dp).
-  static constexpr int FS = NQ <= 3 ? 8 : 7;
-  static constexpr int DS = NQ == 2 || NQ == 4 ? 8 : NQ == 9 ? 6 : 7;
-  static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
-  static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
-  static constexpr int NT = NL * EPB;
-  // resident CTAs per SM to compile for (registers): measured best of 5, 6, 7, 8
-  static constexpr int MINB = NQ == 9 ? 5 : 7;
-};
-
-// D (trans = false) or D^T in the layout's table: entry c of row t (2 Dp, 2 Dm)
-template <int NQ>
-__device__ __forceinline__ double fx_table_entry(const double* __restrict__ Dg, bool trans, int t, int c) {
-  using L = FxLayout<NQ>;
-  const int rs = trans ? 1 : NQ, cs = trans ? NQ : 1;
-  if constexpr (L::EO) {
-    const int m = c >> 1;
-    const double d0 = Dg[t * rs + m * cs], d1 = Dg[t * rs + (NQ - 1 - m) * cs];
-    return (c & 1) ? d0 - d1 : d0 + d1;
-  } else {
-    return Dg[t * rs + c * cs];
-  }
-}
-
-// emit(t, sum_m table[t][m] q[m]) for the outputs t of one line, as integers in units of
-// 2^(eL + eR[t] - EXP)
-template <int NQ, typename F>
-__device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, const fx_half* __restrict__ tab,
-                                        F&& emit) {
-  using L = FxLayout<NQ>;
-  constexpr int N = NQ - 1, H = L::H;
-  int64_t f[NQ];
-#pragma unroll
-  for (int m = 0; m < NQ; ++m) f[m] = fx_from_double<L::FS + 1>(q[m], eL);
-  fx_half x[NQ];
-  if constexpr (L::EO) {
-#pragma unroll
-    for (int m = 0; m < H; ++m) {
-      x[2 * m] = fx_split(f[m] + f[N - m]);
-      x[2 * m + 1] = fx_split(f[m] - f[N - m]);
-    }
-#pragma unroll
-    for (int t = 0; t < H; ++t) {
-      const int4* row = reinterpret_cast<const int4*>(tab + t * L::COLS);
-      fx_half dp[H], dm[H];
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        const int4 v = row[m];
-        dp[m] = {v.x, v.y};
-        dm[m] = {v.z, v.w};
-      }
-      fx_acc A(x[0], dp[0]), B(x[1], dm[0]);
-#pragma unroll
-      for (int m = 1; m < H; ++m) {
-        A.cross(x[2 * m], dp[m]);
-        B.cross(x[2 * m + 1], dm[m]);
-      }
-      A.fold();
-      B.fold();
-#pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A.high(x[2 * m], dp[m]);
-        B.high(x[2 * m + 1], dm[m]);
-      }
-      emit(t, A.v + B.v + 1);   // both were rounded down
-      emit(N - t, B.v - A.v);
-    }
-  } else {
-#pragma unroll
-    for (int m = 0; m < NQ; ++m) x[m] = fx_split(f[m]);
-#pragma unroll
-    for (int t = 0; t < NQ; ++t) {
-      fx_acc A(0x40000000ll);   // rounds to nearest
-      fx_half d[NQ];
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) {
-        d[m] = tab[t * L::COLS + m];
-        A.cross(x[m], d[m]);
-      }
-      A.fold();
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) A.high(x[m], d[m]);
-      emit(t, A.v);
-    }
-  }
-}
-
-// a line of zeros (as the masked lines of Dirichlet faces are): no magnitude bit is set
-template <int NQ>
-__device__ __forceinline__ bool fx_zero(const double (&v)[NQ], const unsigned key) {
-  int lo = 0;
-#pragma unroll
-  for (int m = 0; m < NQ; ++m) lo |= __double2loint(v[m]);
-  return key == 0 && lo == 0;
-}
-
-// row of the table that output t of a line uses
-template <int NQ>
-__device__ __forceinline__ constexpr int fx_row(int t) {
-  return FxLayout<NQ>::EO && t >= NQ / 2 ? NQ - 1 - t : t;
-}
-
 // MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
 // UNIT: lambda == 1 without a lambda field, the mass term is wJ q
 template <int NQ, int INMODE, int OUTMODE, bool MASS, bool UNIT>
@@ -559,20 +413,14 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
                  const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
                  double* __restrict__ out) {
   using L = FxLayout<NQ>;
-  constexpr int NP = L::NP, NL = L::NL, P = L::P, PL = L::PL, EPB = L::EPB, NT = L::NT;
+  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB;
   constexpr int TAB = L::ROWS * L::COLS;
   extern __shared__ __align__(16) unsigned char fx_smem[];
   __shared__ __align__(16) fx_half s_tab[2][TAB];   // D, D^T
   __shared__ int s_e[2][L::ROWS];                   // biased exponents of their rows
   __shared__ int s_x[EPB][3][NL];                   // exponents of the transposed lines, -1: FP64 values
   const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
-  double* S = reinterpret_cast<double*>(fx_smem) + el * (3 * PL * NQ);
-  const int a = l % NQ, b = l / NQ;
-  // line l of each copy, and node (a, b, 0) in each; node (a, b, k) is k PL, k PL, k further
-  double* const line = S + b * PL + a * P;
-  double* const nr = S + b * P + a;
-  double* const ns = S + PL * NQ + a * P + b;
-  double* const nt = S + 2 * PL * NQ + b * PL + a * P;
+  const FxElement<NQ> E(reinterpret_cast<double*>(fx_smem) + el * FxElement<NQ>::DOUBLES, l);
 
   int64_t e = (int64_t)blockIdx.x * EPB + el;
   const bool active = e < Nelements;
@@ -583,7 +431,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
     prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(double));
     if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(double));
   }
-  int plain = 0;
+  bool plain;
   {
     double v[NQ];
     if constexpr (INMODE == IN_GATHER) {
@@ -596,53 +444,12 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
 #pragma unroll
       for (int k = 0; k < NQ; ++k) v[k] = active ? q[nodeBase + k * NL] : 0.0;
     }
-    // tables of D and D^T while the gather is in flight; entries beyond 2^63 leave every
-    // line to FP64
-    for (int w = tid; w < 2 * TAB; w += NT) {
-      const int tr = w / TAB, t = (w % TAB) / L::COLS, c = w % L::COLS;
-      unsigned key = 0;
+    plain = fx_tables<NQ>(Dg, tid, s_tab, s_e);   // while the gather is in flight
 #pragma unroll
-      for (int m = 0; m < NQ; ++m) key = max(key, fx_key(Dg[tr ? m * NQ + t : t * NQ + m]));
-      const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
-      s_tab[tr][t * L::COLS + c] = fx_split(fx_from_double<L::DS + 1>(fx_table_entry<NQ>(Dg, tr, t, c), eR));
-      if (c == 0) s_e[tr][t] = eR;
-      plain |= eR > 1086;
-    }
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) nr[k * PL] = ns[k * PL] = nt[k] = v[k];
+    for (int k = 0; k < NQ; ++k) E.r(E.a, E.b, k) = E.s(E.a, E.b, k) = E.t(E.a, E.b, k) = v[k];
   }
   plain = __syncthreads_or(plain);
-
-  // D q along r, s, t
-#pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
-    double* const o = line + d * PL * NQ;
-    double v[NQ];
-    unsigned key = 0;
-#pragma unroll
-    for (int m = 0; m < NQ; ++m) {
-      v[m] = o[m];
-      key = max(key, fx_key(v[m]));
-    }
-    const int eL = (int)(key >> 20);
-    asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
-    if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ>(v, eL, s_tab[0], [&](int t, int64_t r) {
-        o[t] = fx_to_double(r, fx_base(eL + s_e[0][fx_row<NQ>(t)] - (L::EXP - 1086)));
-      });
-    } else if (fx_zero<NQ>(v, key)) {
-#pragma unroll
-      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
-    } else {
-#pragma unroll 1
-      for (int t = 0; t < NQ; ++t) {
-        double r = 0;
-#pragma unroll
-        for (int m = 0; m < NQ; ++m) r += Dg[t * NQ + m] * v[m];
-        o[t] = r;
-      }
-    }
-  }
+  fx_forward<NQ>(E, s_tab[0], s_e[0], plain, Dg);
   ax_fx_sync<NQ, EPB>(el);
 
   // G . grad q
@@ -655,48 +462,16 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
         G00 = gp[0 * NP + k * NL]; G01 = gp[1 * NP + k * NL]; G02 = gp[2 * NP + k * NL];
         G11 = gp[3 * NP + k * NL]; G12 = gp[4 * NP + k * NL]; G22 = gp[5 * NP + k * NL];
       }
-      const double qr = nr[k * PL], qs = ns[k * PL], qt = nt[k];
-      nr[k * PL] = G00 * qr + G01 * qs + G02 * qt;
-      ns[k * PL] = G01 * qr + G11 * qs + G12 * qt;
-      nt[k] = G02 * qr + G12 * qs + G22 * qt;
+      double &ur = E.r(E.a, E.b, k), &us = E.s(E.a, E.b, k), &ut = E.t(E.a, E.b, k);
+      const double qr = ur, qs = us, qt = ut;
+      ur = G00 * qr + G01 * qs + G02 * qt;
+      us = G01 * qr + G11 * qs + G12 * qt;
+      ut = G02 * qr + G12 * qs + G22 * qt;
     }
   }
   ax_fx_sync<NQ, EPB>(el);
 
-  // D^T along r, s, t, left as integers
-  bool fp = false;   // a line of this thread kept FP64 values
-#pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
-    double* const o = line + d * PL * NQ;
-    double v[NQ];
-    unsigned key = 0;
-#pragma unroll
-    for (int m = 0; m < NQ; ++m) {
-      v[m] = o[m];
-      key = max(key, fx_key(v[m]));
-    }
-    const int eL = (int)(key >> 20);
-    int x = eL;
-    asm volatile("" ::: "memory");
-    if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ>(v, eL, s_tab[1], [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
-    } else if (fx_zero<NQ>(v, key)) {
-      x = 128;
-#pragma unroll
-      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
-    } else {
-      x = -1;
-      fp = true;
-#pragma unroll 1
-      for (int t = 0; t < NQ; ++t) {
-        double r = 0;
-#pragma unroll
-        for (int m = 0; m < NQ; ++m) r += Dg[m * NQ + t] * v[m];
-        o[t] = r;
-      }
-    }
-    s_x[el][d][l] = x;
-  }
+  bool fp = fx_transposed<NQ>(E, s_tab[1], plain, Dg, s_x[el]);
   int32_t id[NQ];   // in flight over the barrier
   if constexpr (OUTMODE == OUT_ASSEMBLE || (MASS && INMODE == IN_GATHER)) {
 #pragma unroll
@@ -707,23 +482,10 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
   if (!active) return;
   const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
   const double* wp = wJ + e * wJStride + l;
-  const int er = s_e[1][fx_row<NQ>(a)], es = s_e[1][fx_row<NQ>(b)];
+  const int er = s_e[1][fx_row<NQ>(E.a)], es = s_e[1][fx_row<NQ>(E.b)];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    const int lr = s_x[el][0][b + NQ * k], ls = s_x[el][1][a + NQ * k], lt = s_x[el][2][l];
-    const int xr = lr + er, xs = ls + es, xt = lt + s_e[1][fx_row<NQ>(k)];
-    const double vr = nr[k * PL], vs = ns[k * PL], vt = nt[k];
-    double r;
-    if (!fp || (lr | ls | lt) >= 0) {
-      const int X = max(xr, max(xs, xt));
-      const int64_t sum = fx_shr(__double_as_longlong(vr), X - xr) + fx_shr(__double_as_longlong(vs), X - xs) +
-                          fx_shr(__double_as_longlong(vt), X - xt);
-      r = fx_to_double(sum, fx_base(X - (L::EXP - 1086)));
-    } else {
-      r = (lr < 0 ? vr : fx_to_double(__double_as_longlong(vr), fx_base(xr - (L::EXP - 1086)))) +
-          (ls < 0 ? vs : fx_to_double(__double_as_longlong(vs), fx_base(xs - (L::EXP - 1086)))) +
-          (lt < 0 ? vt : fx_to_double(__double_as_longlong(vt), fx_base(xt - (L::EXP - 1086))));
-    }
+    double r = fx_node_sum<NQ>(E, k, s_x[el], s_e[1], er, es, fp);
     if constexpr (MASS) {
       double v = 0.0;
       if constexpr (INMODE == IN_GATHER) v = id[k] >= 0 ? q[id[k]] : 0.0;
@@ -1334,7 +1096,7 @@ static int fx_config(KernelConfig* cfg, size_t* smem) {
   using L = FxLayout<NQ>;
   static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in, occupancy
   auto kern = ax_hex_fx_kernel<NQ, INMODE, OUTMODE, MASS, UNIT>;
-  const size_t bytes = sizeof(double) * 3 * L::PL * NQ * L::EPB;
+  const size_t bytes = sizeof(double) * FxElement<NQ>::DOUBLES * L::EPB;
   *smem = bytes;
   return perDevice.get(
       [&](int, KernelConfig& c) {

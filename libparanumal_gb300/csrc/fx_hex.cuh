@@ -1,0 +1,297 @@
+// Building blocks of the FP64 hexahedral operators with block fixed-point contractions
+// (fx64.cuh): the layout of an element in shared memory, the tables of D and D^T, and the
+// derivatives of a whole element along its three directions. Used by the C0 operator
+// (ax_hex.cu) and the interior-penalty operator (ipdg_hex.cu).
+//
+// One thread holds one line at a time: thread l of an element takes line l of the r, then
+// of the s, then of the t direction. Line maxima, even/odd sums and all integers of a line are
+// then the thread's own registers. The element is kept in three copies, each with the lines of
+// one direction contiguous, so one piece of code with immediate offsets serves all three, in
+// place.
+//
+// Nq = 4, 8: the GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
+// with e_m = q_m + q_{N-m}, o_m = q_m - q_{N-m} (m < H = Nq/2), outputs t and N-t are A + B
+// and B - A, A = sum Dp[t][m] e_m, B = sum Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m])/2.
+#pragma once
+
+#include "fx64.cuh"
+
+namespace lpg {
+
+// L2 prefetch of `bytes` (a multiple of 16) from global memory; skipped unless the address
+// is 16-byte aligned, as the bulk prefetch requires
+__device__ __forceinline__ void prefetch_l2_bulk(const void* gmem, unsigned bytes) {
+  if (((uintptr_t)gmem & 15u) == 0 && (bytes & 15u) == 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(gmem), "r"(bytes) : "memory");
+}
+// Barrier over the threads of one element where they are whole warps, else over the CTA;
+// returns whether `any` was set by one of them. The barrier numbers are immediates: a number
+// in a register reserves all 16 of a CTA's barriers, and an SM's 64 then hold only 4 CTAs.
+template <int NQ, int EPB>
+__device__ __forceinline__ bool ax_fx_sync(const int el, const bool any = false) {
+  if constexpr ((NQ * NQ) % 32 == 0 && EPB == 2) {
+    int r;
+#define LPG_FX_BARRIER(id)                                                                              \
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %2, 0;\nbarrier.cta.red.or.pred q, " #id ", %1, p;\n" \
+               "selp.s32 %0, 1, 0, q;\n}\n"                                                              \
+               : "=r"(r)                                                                                \
+               : "n"(NQ * NQ), "r"((int)any)                                                            \
+               : "memory")
+    if (el == 0) LPG_FX_BARRIER(1);
+    else LPG_FX_BARRIER(2);
+#undef LPG_FX_BARRIER
+    return r != 0;
+  } else {
+    return __syncthreads_or(any);
+  }
+}
+
+template <int NQ>
+struct FxLayout {
+  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ, H = NQ / 2;
+  static constexpr bool EO = (NQ == 4 || NQ == 8);
+  static constexpr int P = NQ | 1, PL = P * NQ;      // odd row pitch: conflict-free lines
+  static constexpr int ROWS = EO ? H : NQ;           // rows of a table
+  static constexpr int COLS = EO ? 2 * H : NQ;       // (Dp, Dm) interleaved, or D
+  // Bits S (fx64.cuh) of a line value (FS) and a table entry (DS): as many as keep the halves
+  // in 32 bits and, for any D, the sum of the middle quarters, COLS (EO: H per sum) products
+  // of each kind, and the sum of three transposed lines below 2^63. The mirror sums double a
+  // line value and a table entry (2 Dp).
+  static constexpr int FS = NQ <= 3 ? 8 : 7;
+  static constexpr int DS = NQ == 2 || NQ == 4 ? 8 : NQ == 9 ? 6 : 7;
+  static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
+  static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
+  static constexpr int NT = NL * EPB;
+  // resident CTAs per SM to compile for (registers): measured best of 5, 6, 7, 8
+  static constexpr int MINB = NQ == 9 ? 5 : 7;
+};
+
+// D (trans = false) or D^T in the layout's table: entry c of row t (2 Dp, 2 Dm)
+template <int NQ>
+__device__ __forceinline__ double fx_table_entry(const double* __restrict__ Dg, bool trans, int t, int c) {
+  using L = FxLayout<NQ>;
+  const int rs = trans ? 1 : NQ, cs = trans ? NQ : 1;
+  if constexpr (L::EO) {
+    const int m = c >> 1;
+    const double d0 = Dg[t * rs + m * cs], d1 = Dg[t * rs + (NQ - 1 - m) * cs];
+    return (c & 1) ? d0 - d1 : d0 + d1;
+  } else {
+    return Dg[t * rs + c * cs];
+  }
+}
+
+// emit(t, sum_m table[t][m] q[m]) for the outputs t of one line, as integers in units of
+// 2^(eL + eR[t] - EXP)
+template <int NQ, typename F>
+__device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, const fx_half* __restrict__ tab,
+                                        F&& emit) {
+  using L = FxLayout<NQ>;
+  constexpr int N = NQ - 1, H = L::H;
+  int64_t f[NQ];
+#pragma unroll
+  for (int m = 0; m < NQ; ++m) f[m] = fx_from_double<L::FS + 1>(q[m], eL);
+  fx_half x[NQ];
+  if constexpr (L::EO) {
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      x[2 * m] = fx_split(f[m] + f[N - m]);
+      x[2 * m + 1] = fx_split(f[m] - f[N - m]);
+    }
+#pragma unroll
+    for (int t = 0; t < H; ++t) {
+      const int4* row = reinterpret_cast<const int4*>(tab + t * L::COLS);
+      fx_half dp[H], dm[H];
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        const int4 v = row[m];
+        dp[m] = {v.x, v.y};
+        dm[m] = {v.z, v.w};
+      }
+      fx_acc A(x[0], dp[0]), B(x[1], dm[0]);
+#pragma unroll
+      for (int m = 1; m < H; ++m) {
+        A.cross(x[2 * m], dp[m]);
+        B.cross(x[2 * m + 1], dm[m]);
+      }
+      A.fold();
+      B.fold();
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        A.high(x[2 * m], dp[m]);
+        B.high(x[2 * m + 1], dm[m]);
+      }
+      emit(t, A.v + B.v + 1);   // both were rounded down
+      emit(N - t, B.v - A.v);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) x[m] = fx_split(f[m]);
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) {
+      fx_acc A(0x40000000ll);   // rounds to nearest
+      fx_half d[NQ];
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) {
+        d[m] = tab[t * L::COLS + m];
+        A.cross(x[m], d[m]);
+      }
+      A.fold();
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) A.high(x[m], d[m]);
+      emit(t, A.v);
+    }
+  }
+}
+
+// a line of zeros (as the masked lines of Dirichlet faces are): no magnitude bit is set
+template <int NQ>
+__device__ __forceinline__ bool fx_zero(const double (&v)[NQ], const unsigned key) {
+  int lo = 0;
+#pragma unroll
+  for (int m = 0; m < NQ; ++m) lo |= __double2loint(v[m]);
+  return key == 0 && lo == 0;
+}
+
+// row of the table that output t of a line uses
+template <int NQ>
+__device__ __forceinline__ constexpr int fx_row(int t) {
+  return FxLayout<NQ>::EO && t >= NQ / 2 ? NQ - 1 - t : t;
+}
+
+// one element's three copies in shared memory, seen by thread l = a + NQ b
+template <int NQ>
+struct FxElement {
+  using L = FxLayout<NQ>;
+  static constexpr int DOUBLES = 3 * L::PL * NQ;   // of an element
+  double* S;
+  int l, a, b;
+  __device__ __forceinline__ FxElement(double* base, int l_) : S(base), l(l_), a(l_ % NQ), b(l_ / NQ) {}
+  // line l of direction d
+  __device__ __forceinline__ double* line(int d) const { return S + d * L::PL * NQ + b * L::PL + a * L::P; }
+  // node (i, j, k) in the copies of direction r, s, t
+  __device__ __forceinline__ double& r(int i, int j, int k) const { return S[k * L::PL + j * L::P + i]; }
+  __device__ __forceinline__ double& s(int i, int j, int k) const { return S[L::PL * NQ + k * L::PL + i * L::P + j]; }
+  __device__ __forceinline__ double& t(int i, int j, int k) const { return S[2 * L::PL * NQ + j * L::PL + i * L::P + k]; }
+};
+
+// tables of D and D^T with the exponents of their rows, by the NT threads of a CTA; true where
+// an entry beyond 2^63 leaves every line to FP64
+template <int NQ>
+__device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid,
+                                          fx_half (&tab)[2][FxLayout<NQ>::ROWS * FxLayout<NQ>::COLS],
+                                          int (&ex)[2][FxLayout<NQ>::ROWS]) {
+  using L = FxLayout<NQ>;
+  constexpr int TAB = L::ROWS * L::COLS;
+  bool plain = false;
+  for (int w = tid; w < 2 * TAB; w += L::NT) {
+    const int tr = w / TAB, t = (w % TAB) / L::COLS, c = w % L::COLS;
+    unsigned key = 0;
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) key = max(key, fx_key(Dg[tr ? m * NQ + t : t * NQ + m]));
+    const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
+    tab[tr][t * L::COLS + c] = fx_split(fx_from_double<L::DS + 1>(fx_table_entry<NQ>(Dg, tr, t, c), eR));
+    if (c == 0) ex[tr][t] = eR;
+    plain |= eR > 1086;
+  }
+  return plain;
+}
+
+// the copies of q become D_r q, D_s q, D_t q
+template <int NQ>
+__device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half* tab, const int* ex, const bool plain,
+                                           const double* __restrict__ Dg) {
+  using L = FxLayout<NQ>;
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    double* const o = E.line(d);
+    double v[NQ];
+    unsigned key = 0;
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) {
+      v[m] = o[m];
+      key = max(key, fx_key(v[m]));
+    }
+    const int eL = (int)(key >> 20);
+    asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
+    if (fx_ordinary(eL) && !plain) {
+      fx_line<NQ>(v, eL, tab, [&](int t, int64_t r) {
+        o[t] = fx_to_double(r, fx_base(eL + ex[fx_row<NQ>(t)] - (L::EXP - 1086)));
+      });
+    } else if (fx_zero<NQ>(v, key)) {
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
+    } else {
+#pragma unroll 1
+      for (int t = 0; t < NQ; ++t) {
+        double r = 0;
+#pragma unroll
+        for (int m = 0; m < NQ; ++m) r += Dg[t * NQ + m] * v[m];
+        o[t] = r;
+      }
+    }
+  }
+}
+
+// the copies (u_r, u_s, u_t) become D_r^T u_r, D_s^T u_s, D_t^T u_t as integers, with the
+// exponents of the lines in x, -1 for a line kept as FP64 values; true if this thread kept one
+template <int NQ>
+__device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_half* tab, const bool plain,
+                                              const double* __restrict__ Dg, int (&x)[3][FxLayout<NQ>::NL]) {
+  bool fp = false;
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    double* const o = E.line(d);
+    double v[NQ];
+    unsigned key = 0;
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) {
+      v[m] = o[m];
+      key = max(key, fx_key(v[m]));
+    }
+    const int eL = (int)(key >> 20);
+    int xl = eL;
+    asm volatile("" ::: "memory");
+    if (fx_ordinary(eL) && !plain) {
+      fx_line<NQ>(v, eL, tab, [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
+    } else if (fx_zero<NQ>(v, key)) {
+      xl = 128;
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) o[t] = 0.0;
+    } else {
+      xl = -1;
+      fp = true;
+#pragma unroll 1
+      for (int t = 0; t < NQ; ++t) {
+        double r = 0;
+#pragma unroll
+        for (int m = 0; m < NQ; ++m) r += Dg[m * NQ + t] * v[m];
+        o[t] = r;
+      }
+    }
+    x[d][E.l] = xl;
+  }
+  return fp;
+}
+
+// sum of the three transposed parts at node (a, b, k); er, es: exponents of the rows a and b
+// of D^T; fp: some line of the element was kept in FP64
+template <int NQ>
+__device__ __forceinline__ double fx_node_sum(const FxElement<NQ>& E, const int k, const int (&x)[3][FxLayout<NQ>::NL],
+                                              const int* ex, const int er, const int es, const bool fp) {
+  using L = FxLayout<NQ>;
+  constexpr int OFF = L::EXP - 1086;
+  const int lr = x[0][E.b + NQ * k], ls = x[1][E.a + NQ * k], lt = x[2][E.l];
+  const int xr = lr + er, xs = ls + es, xt = lt + ex[fx_row<NQ>(k)];
+  const double vr = E.r(E.a, E.b, k), vs = E.s(E.a, E.b, k), vt = E.t(E.a, E.b, k);
+  if (!fp || (lr | ls | lt) >= 0) {
+    const int X = max(xr, max(xs, xt));
+    const int64_t sum = fx_shr(__double_as_longlong(vr), X - xr) + fx_shr(__double_as_longlong(vs), X - xs) +
+                        fx_shr(__double_as_longlong(vt), X - xt);
+    return fx_to_double(sum, fx_base(X - OFF));
+  }
+  return (lr < 0 ? vr : fx_to_double(__double_as_longlong(vr), fx_base(xr - OFF))) +
+         (ls < 0 ? vs : fx_to_double(__double_as_longlong(vs), fx_base(xs - OFF))) +
+         (lt < 0 ? vt : fx_to_double(__double_as_longlong(vt), fx_base(xt - OFF)));
+}
+
+}  // namespace lpg

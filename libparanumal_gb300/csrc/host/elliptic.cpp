@@ -409,11 +409,10 @@ int Elliptic::setup_ipdg(const MeshConfig& c, int N, const std::vector<double>* 
   EToE_h = hm->EToE;
   std::vector<int32_t> iota(Nlocal);
   for (int64_t n = 0; n < Nlocal; ++n) iota[n] = (int32_t)n;
-  DevBuf<int32_t> mapP;
   DevBuf<double> hfac;
   if ((rc = g2l.alloc(Nlocal)) || (rc = owner.alloc(Nlocal)) || (rc = weightG.alloc(Nlocal)) ||
-      (rc = vgeo.alloc(E * 10 * Np)) || (rc = sgeo.alloc(E * 5 * 6 * Nfp)) || (rc = g4.alloc(4 * Nlocal)) ||
-      (rc = vmapP.alloc(E * 6 * Nfp)) || (rc = mapP.alloc(E * 6 * Nfp)) || (rc = EToB.alloc(E * 6)) ||
+      (rc = vgeo.alloc(E * 10 * Np)) || (rc = sgeo.alloc(E * 5 * 6 * Nfp)) || (rc = fcoef.alloc(E * 5 * 6 * Nfp)) ||
+      (rc = trace.alloc(2 * E * 6 * Nfp)) || (rc = vmapP.alloc(E * 6 * Nfp)) || (rc = mapP.alloc(E * 6 * Nfp)) || (rc = EToB.alloc(E * 6)) ||
       (rc = hfac.alloc(E * 6 * Nfp)))
     return rc;
   if ((rc = g2l.upload(iota.data(), Nlocal, s)) || (rc = owner.upload(iota.data(), Nlocal, s)) ||
@@ -423,7 +422,7 @@ int Elliptic::setup_ipdg(const MeshConfig& c, int N, const std::vector<double>* 
   tau = 2.0 * (N + 1) * (N + 3);
   IpdgArgs a = ipdg_args();
   a.hfac = hfac.p;
-  if ((rc = ipdg_geometry(a, mapP.p, s))) return rc;
+  if ((rc = ipdg_geometry(a, s))) return rc;
   if ((rc = finish_setup(lamE, s))) return rc;   // synchronises before the host vectors go
   return LPG_OK;
 }
@@ -434,11 +433,11 @@ IpdgArgs Elliptic::ipdg_args() const {
   a.E = mesh.E;
   a.EX = mesh.EX.p; a.EY = mesh.EY.p; a.EZ = mesh.EZ.p;
   a.D = mesh.D_d.p; a.r1d = mesh.r1d_d.p; a.w1d = mesh.w1d_d.p;
-  a.vgeo = vgeo.p; a.sgeo = sgeo.p;
-  a.vmapP = vmapP.p; a.EToB = EToB.p;
+  a.geo = mesh.geo.p; a.vgeo = vgeo.p; a.sgeo = sgeo.p; a.fcoef = fcoef.p;
+  a.mapP = mapP.p; a.EToB = EToB.p;
   a.lambda = lambda; a.tau = tau;
   a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
-  a.g4 = reinterpret_cast<double4_32a*>(g4.p);
+  a.trace = reinterpret_cast<double2*>(trace.p);
   return a;
 }
 

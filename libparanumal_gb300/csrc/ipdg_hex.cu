@@ -9,15 +9,18 @@
 //
 // Layout (per element, structure of arrays): vgeo [e][10][Np] = rx ry rz sx sy sz tx ty tz JW;
 // sgeo [e][5][6 Nfp] = nx ny nz WsJ hinv for the face nodes of faces 0..5 (local index order);
-// gradients [E Np] double4_32a = (qx, qy, qz, q). The FP32 preconditioner levels run the same
-// gradient and operator kernels on FP32 copies of vgeo and sgeo with float4 gradients.
+// fcoef [e][5][6 Nfp] = n . grad r, n . grad s, n . grad t, WsJ / 2, tau hinv of the FP64
+// operator. The FP32 preconditioner levels run a gradient and an operator kernel on FP32
+// copies of vgeo and sgeo with float4 gradients.
 //
-// Kernels run one CTA per element with one thread per node. A node owns its accumulators:
+// Those kernels run one CTA per element with one thread per node. A node owns its accumulators:
 // the face terms of every face it lies on are added by that node's thread, in the face
 // order 0, 5, 1, 3, 2, 4, so no two threads write the same value.
+#include <algorithm>
 #include <type_traits>
 
 #include "df64.cuh"
+#include "fx_hex.cuh"
 #include "lpg_common.cuh"
 #include "lpg_internal.hpp"
 
@@ -160,9 +163,30 @@ __global__ void ipdg_hinv_kernel(const int64_t nFaceNodes, const int nfpAll, con
   }
 }
 
+// coefficients of the FP64 operator's face terms (n . grad of the reference coordinates,
+// WsJ / 2, tau hinv), so that it needs neither the nine volume factors nor the physical
+// gradient
+template <int NQ>
+__global__ void __launch_bounds__(256)
+ipdg_face_coef_kernel(const int64_t E, const double* __restrict__ vgeo, const double* __restrict__ sgeo,
+                      const double tau, double* __restrict__ fcoef) {
+  constexpr int NP = NQ * NQ * NQ, NFP = NQ * NQ, NS = 6 * NFP;
+  for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < E * NS; id += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t e = id / NS;
+    const int c = (int)(id % NS);
+    const double* vg = vgeo + e * kVgeo * NP + face_node<NQ>(c / NFP, c % NFP);
+    const double* sg = sgeo + e * kSgeo * NS + c;
+    double* fc = fcoef + e * 5 * NS + c;
+    const double nx = sg[0], ny = sg[NS], nz = sg[2 * NS];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) fc[d * NS] = nx * vg[3 * d * NP] + ny * vg[(3 * d + 1) * NP] + nz * vg[(3 * d + 2) * NP];
+    fc[3 * NS] = 0.5 * sg[3 * NS];
+    fc[4 * NS] = tau * sg[4 * NS];
+  }
+}
+
 // ---------------------------------------------------------------- gradient
-// T = double (the operator) or float (the FP32 preconditioner levels); V4 the matching
-// 4-vector (double4_32a, float4)
+// The FP32 preconditioner levels (T = float, V4 = float4)
 template <int NQ, typename T, typename V4>
 __global__ void __launch_bounds__(NQ * NQ * NQ)
 ipdg_gradient_kernel(const T* __restrict__ vgeo, const T* __restrict__ Dg, const T* __restrict__ q,
@@ -191,70 +215,6 @@ ipdg_gradient_kernel(const T* __restrict__ vgeo, const T* __restrict__ Dg, const
   g4[e * NP + n] = o;
 }
 
-// FP64 gradient with the even-odd split of D (Nq even; D[N-a][N-m] = -D[a][m] on GLL
-// points). Along each direction node i and its mirror N-i form a pair: with e_m = q_m +
-// q_{N-m}, o_m = q_m - q_{N-m} (m < Nq/2) and Dp, Dm the even and odd halves of D, the
-// lower node of the pair dots row min(i, N-i) of Dp with e, the upper one that row of Dm
-// with o, and the partial sums A, B are exchanged through shared memory: d(i) = A + B,
-// d(N-i) = B - A. Per node and direction: 1 + Nq/2 + 1 FP64 instructions instead of Nq.
-// Every selection between the two halves is an index, so warps do not diverge.
-template <int NQ>
-__global__ void __launch_bounds__(NQ * NQ * NQ)
-ipdg_gradient_eo_kernel(const double* __restrict__ vgeo, const double* __restrict__ Dg,
-                        const double* __restrict__ q, double4_32a* __restrict__ g4) {
-  constexpr int NP = NQ * NQ * NQ, NFP = NQ * NQ, H = NQ / 2, N = NQ - 1;
-  static_assert(NQ % 2 == 0, "even-odd gradient: Nq even");
-  __shared__ double s_q[NP];
-  __shared__ double s_eo[3][NP];       // e (lower half of each line) / o (upper half) per direction
-  __shared__ double s_x[3][NP];        // partial sums for the pair exchange
-  __shared__ double s_DpDm[2 * H * H]; // rows of Dp, then rows of Dm
-  const int64_t e = blockIdx.x;
-  const int n = threadIdx.x;
-  const int i = n % NQ, j = (n / NQ) % NQ, k = n / NFP;
-  if (n < H * H) {
-    const int a = n / H, m = n % H;
-    const double d0 = Dg[a * NQ + m], d1 = Dg[a * NQ + N - m];
-    s_DpDm[n] = 0.5 * (d0 + d1);
-    s_DpDm[H * H + n] = 0.5 * (d0 - d1);
-  }
-  const double qn = q[e * NP + n];
-  s_q[n] = qn;
-  __syncthreads();
-  // mirror nodes along r, s, t and the sign that forms e (lower half) or o (upper half)
-  const int pi = n + (N - 2 * i), pj = n + (N - 2 * j) * NQ, pk = n + (N - 2 * k) * NFP;
-  const double si = i < H ? 1.0 : -1.0, sj = j < H ? 1.0 : -1.0, sk = k < H ? 1.0 : -1.0;
-  s_eo[0][n] = fma(si, qn, s_q[pi]);   // i < H: e_i;  i >= H: o_{N-i} = q_{N-i} - q_i
-  s_eo[1][n] = fma(sj, qn, s_q[pj]);
-  s_eo[2][n] = fma(sk, qn, s_q[pk]);
-  __syncthreads();
-  const double* ci = s_DpDm + (i < H ? i * H : H * H + (N - i) * H);
-  const double* cj = s_DpDm + (j < H ? j * H : H * H + (N - j) * H);
-  const double* ck = s_DpDm + (k < H ? k * H : H * H + (N - k) * H);
-  double ar = 0, as = 0, at = 0;
-#pragma unroll
-  for (int m = 0; m < H; ++m) {
-    // e_m sits at line position m, o_m at position N - m
-    const int mi = i < H ? m : N - m, mj = j < H ? m : N - m, mk = k < H ? m : N - m;
-    ar = fma(ci[m], s_eo[0][mi + j * NQ + k * NFP], ar);
-    as = fma(cj[m], s_eo[1][i + mj * NQ + k * NFP], as);
-    at = fma(ck[m], s_eo[2][i + j * NQ + mk * NFP], at);
-  }
-  s_x[0][n] = ar;
-  s_x[1][n] = as;
-  s_x[2][n] = at;
-  __syncthreads();
-  const double qr = fma(si, s_x[0][pi], ar);   // lower: A + B, upper: B - A
-  const double qs = fma(sj, s_x[1][pj], as);
-  const double qt = fma(sk, s_x[2][pk], at);
-  const double* vg = vgeo + e * kVgeo * NP + n;
-  double4_32a o;
-  o.x = vg[0 * NP] * qr + vg[3 * NP] * qs + vg[6 * NP] * qt;
-  o.y = vg[1 * NP] * qr + vg[4 * NP] * qs + vg[7 * NP] * qt;
-  o.z = vg[2 * NP] * qr + vg[5 * NP] * qs + vg[8 * NP] * qt;
-  o.w = qn;
-  g4[e * NP + n] = o;
-}
-
 // ---------------------------------------------------------------- weak divergence (shared by Ax and rhs)
 // out_n = acc_n + sum_p D[p][i] ur(p,j,k) + D[p][j] us(i,p,k) + D[p][k] ut(i,j,p), with (ur, us, ut)
 // = (grad r, grad s, grad t) . (gx, gy, gz)
@@ -278,7 +238,7 @@ __device__ __forceinline__ T weak_divergence(const T* vg, T gx, T gy, T gz, T ac
   return v;
 }
 
-// ---------------------------------------------------------------- operator
+// ---------------------------------------------------------------- FP32 operator
 // The face terms run in three phases, one per opposite-face pair (0,5), (1,3), (2,4): the
 // 2 Nfp face slots of a pair sit on consecutive threads (whole warps), no node lies on both
 // faces of a pair, and the node accumulators live in shared memory, so every node receives
@@ -356,6 +316,164 @@ ipdg_ax_kernel(const T* __restrict__ vgeo, const T* __restrict__ sgeo, const int
   const V4 acc = s_acc[n];
   T* s_w = reinterpret_cast<T*>(s_M);   // the traces are no longer read: 3 Np values of scratch
   Aq[e * NP + n] = weak_divergence<NQ, T>(vg, acc.x, acc.y, acc.z, acc.w, s_w, s_w + NP, s_w + 2 * NP, s_D);
+}
+
+// ---------------------------------------------------------------- FP64 operator
+// Two kernels with the contractions in block fixed point (fx_hex.cuh), both on the reference
+// derivatives (D_r q, D_s q, D_t q):
+//   traces: (n . grad q, q) at every face node of an element, with its own outward normal;
+//   operator: the volume term G . grad q of the C0 operator, the face terms added to the three
+//   rows at the face nodes, the transposed derivatives, and the value terms.
+// A face node needs of its neighbour the value and the normal derivative alone: the two
+// outward normals of a conforming face are opposite, so n . grad q_P is minus the neighbour's
+// own. With f = n . grad q_M + n . grad q_P + tau hinv (q_P - q_M) and g = WsJ / 2 (q_P - q_M)
+// a face node adds (n . grad r, n . grad s, n . grad t) g to the rows and -WsJ / 2 f to the
+// value.
+//
+// Bounded by the FP64 pipe: 9 FP64 operations a node for the metric product, 9 a face node
+// (0.75 face nodes a node at N = 7) and 3 for its trace, 2 or 3 for the sum; against 84 a node
+// of the kernels replaced, which formed physical gradients from the nine volume factors.
+template <int NQ>
+__global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB)
+ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, const double* __restrict__ Dg,
+                     const double* __restrict__ q, double2* __restrict__ trace) {
+  using L = FxLayout<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
+  extern __shared__ __align__(16) unsigned char fx_smem[];
+  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::COLS];
+  __shared__ int s_e[2][L::ROWS];
+  const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
+  const FxElement<NQ> S(reinterpret_cast<double*>(fx_smem) + el * FxElement<NQ>::DOUBLES, l);
+  const int64_t e = (int64_t)blockIdx.x * EPB + el;
+  const bool active = e < Nelements;
+  const double* qe = q + e * NP;
+  bool plain;
+  {
+    double v[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
+    plain = fx_tables<NQ>(Dg, tid, s_tab, s_e);
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) S.r(S.a, S.b, k) = S.s(S.a, S.b, k) = S.t(S.a, S.b, k) = v[k];
+  }
+  plain = __syncthreads_or(plain);
+  fx_forward<NQ>(S, s_tab[0], s_e[0], plain, Dg);
+  ax_fx_sync<NQ, EPB>(el);
+  if (!active) return;
+  const double* fc = fcoef + e * 5 * NS + l;
+  double2* tr = trace + e * NS + l;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int i = f == 2 ? N : f == 4 ? 0 : S.a;
+    const int j = f == 1 ? 0 : f == 3 ? N : (f == 2 || f == 4) ? S.a : S.b;
+    const int k = f == 0 ? 0 : f == 5 ? N : S.b;
+    const double* c = fc + f * NL;
+    tr[f * NL] = make_double2(c[0] * S.r(i, j, k) + c[NS] * S.s(i, j, k) + c[2 * NS] * S.t(i, j, k),
+                              qe[i + NQ * j + NL * k]);
+  }
+}
+
+// MASS = false: lambda == 0 and no lambda field
+template <int NQ, bool MASS>
+__global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB > 6 ? 6 : FxLayout<NQ>::MINB)
+ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const double* __restrict__ fcoef,
+                  const int32_t* __restrict__ mapP, const int* __restrict__ EToB, const double* __restrict__ Dg,
+                  const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
+                  const double2* __restrict__ trace, double* __restrict__ Aq) {
+  using L = FxLayout<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
+  extern __shared__ __align__(16) unsigned char fx_smem[];
+  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::COLS];
+  __shared__ int s_e[2][L::ROWS];
+  __shared__ int s_x[EPB][3][NL];
+  __shared__ double s_val[EPB][4 * NL + 1];   // value terms of faces 1, 3, 2, 4, and a zero
+  const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
+  const FxElement<NQ> S(reinterpret_cast<double*>(fx_smem) + el * FxElement<NQ>::DOUBLES, l);
+  const int a = S.a, b = S.b;
+  const bool active = (int64_t)blockIdx.x * EPB + el < Nelements;
+  const int64_t e = active ? (int64_t)blockIdx.x * EPB + el : 0;
+  const double* qe = q + e * NP;
+  const double* gp = geo + e * 7 * NP + l;
+  const double* fc = fcoef + e * 5 * NS + l;
+  const double2* tr = trace + e * NS + l;
+  if (active && l == 0) {
+    prefetch_l2_bulk(geo + e * 7 * NP, (MASS ? 7 : 6) * NP * sizeof(double));
+    prefetch_l2_bulk(fcoef + e * 5 * NS, 5 * NS * sizeof(double));
+    prefetch_l2_bulk(mapP + e * NS, NS * sizeof(int32_t));
+  }
+  bool plain;
+  {
+    double v[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
+    plain = fx_tables<NQ>(Dg, tid, s_tab, s_e);
+    if (l == 0) s_val[el][4 * NL] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) S.r(a, b, k) = S.s(a, b, k) = S.t(a, b, k) = v[k];
+  }
+  plain = __syncthreads_or(plain);
+  fx_forward<NQ>(S, s_tab[0], s_e[0], plain, Dg);
+  ax_fx_sync<NQ, EPB>(el);
+
+  int32_t mP[6];   // in flight over the metric product
+#pragma unroll
+  for (int f = 0; f < 6; ++f) mP[f] = __ldg(mapP + e * NS + f * NL + l);
+#pragma unroll 4
+  for (int k = 0; k < NQ; ++k) {
+    const double G00 = gp[0 * NP + k * NL], G01 = gp[1 * NP + k * NL], G02 = gp[2 * NP + k * NL];
+    const double G11 = gp[3 * NP + k * NL], G12 = gp[4 * NP + k * NL], G22 = gp[5 * NP + k * NL];
+    double &ur = S.r(a, b, k), &us = S.s(a, b, k), &ut = S.t(a, b, k);
+    const double qr = ur, qs = us, qt = ut;
+    ur = G00 * qr + G01 * qs + G02 * qt;
+    us = G01 * qr + G11 * qs + G12 * qt;
+    ut = G02 * qr + G12 * qs + G22 * qt;
+  }
+  // face node l of face f at node (i, j, k): rows in shared memory, value term returned
+  auto face = [&](const int f, const int i, const int j, const int k) -> double {
+    const double* c = fc + f * NL;
+    const double c0 = c[0], c1 = c[NS], c2 = c[2 * NS], hw = c[3 * NS], th = c[4 * NS];
+    const double2 M = tr[f * NL];
+    double2 P = trace[mP[f]];
+    const int bc = EToB[e * 6 + f];
+    P.x = -P.x;
+    // homogeneous boundary state B (Dirichlet: q = 0, grad kept; Neumann: q kept, grad = 0),
+    // mirror state 2B - M
+    if (bc > 0) P = bc == 1 ? make_double2(M.x, -M.y) : make_double2(-M.x, M.y);
+    const double dq = P.y - M.y, g = hw * dq;
+    double &ur = S.r(i, j, k), &us = S.s(i, j, k), &ut = S.t(i, j, k);
+    ur = fma(c0, g, ur);
+    us = fma(c1, g, us);
+    ut = fma(c2, g, ut);
+    return -hw * fma(th, dq, M.x + P.x);
+  };
+  // opposite faces share no node; the t faces' nodes are this thread's own
+  const double v0 = face(0, a, b, 0), v5 = face(5, a, b, N);
+  ax_fx_sync<NQ, EPB>(el);
+  s_val[el][l] = face(1, a, 0, b);
+  s_val[el][NL + l] = face(3, a, N, b);
+  ax_fx_sync<NQ, EPB>(el);
+  s_val[el][2 * NL + l] = face(2, N, a, b);
+  s_val[el][3 * NL + l] = face(4, 0, a, b);
+  ax_fx_sync<NQ, EPB>(el);
+  bool fp = fx_transposed<NQ>(S, s_tab[1], plain, Dg, s_x[el]);
+  fp = ax_fx_sync<NQ, EPB>(el, fp);
+
+  if (!active) return;
+  const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
+  const int er = s_e[1][fx_row<NQ>(a)], es = s_e[1][fx_row<NQ>(b)];
+  // value terms of this column's nodes on the s faces (entries a + Nq k) and r faces (b + Nq k)
+  const double* zero = &s_val[el][4 * NL];
+  const double* ps = b == 0 ? &s_val[el][a] : b == N ? &s_val[el][NL + a] : zero;
+  const double* pr = a == N ? &s_val[el][2 * NL + b] : a == 0 ? &s_val[el][3 * NL + b] : zero;
+  const int ks = (b == 0 || b == N) ? NQ : 0, kr = (a == 0 || a == N) ? NQ : 0;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    double r = fx_node_sum<NQ>(S, k, s_x[el], s_e[1], er, es, fp) + (ps[ks * k] + pr[kr * k]);
+    if (k == 0) r += v0;
+    if (k == N) r += v5;
+    if constexpr (MASS) r = fma(gp[6 * NP + k * NL] * lam, qe[l + k * NL], r);
+    Aq[e * NP + l + k * NL] = r;
+  }
 }
 
 // ---------------------------------------------------------------- double-word operator
@@ -623,31 +741,50 @@ ipdg_diag_kernel(const double* __restrict__ vgeo, const double* __restrict__ sge
   diag[e * NP + n] = A;
 }
 
-template <int NQ, typename T, typename V4>
-int launch_operator(int64_t E, const T* vgeo, const T* sgeo, const int32_t* vmapP, const int* EToB, const T* D,
-                    T lambda, const T* lambdaE, T tau, const T* q, V4* g4, T* out, cudaStream_t s) {
+template <int NQ>
+int launch_operator_f32(const IpdgArgsF32& a, cudaStream_t s) {
   constexpr int NP = NQ * NQ * NQ;
-  if (E <= 0) return LPG_OK;
-  if constexpr (std::is_same<T, double>::value && NQ % 2 == 0) {
-    ipdg_gradient_eo_kernel<NQ><<<(unsigned)E, NP, 0, s>>>(vgeo, D, q, g4);
-    LPG_LAUNCH_CHECK("ipdg_gradient_eo_kernel");
-  } else {
-    ipdg_gradient_kernel<NQ, T, V4><<<(unsigned)E, NP, 0, s>>>(vgeo, D, q, g4);
-    LPG_LAUNCH_CHECK("ipdg_gradient_kernel");
-  }
-  constexpr size_t smem = AxSmem<NQ, T, V4>::bytes;
+  if (a.E <= 0) return LPG_OK;
+  ipdg_gradient_kernel<NQ, float, float4><<<(unsigned)a.E, NP, 0, s>>>(a.vgeo, a.D, a.q, a.g4);
+  LPG_LAUNCH_CHECK("ipdg_gradient_kernel");
+  constexpr size_t smem = AxSmem<NQ, float, float4>::bytes;
   static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in
   KernelConfig cfg;
   const int rc = perDevice.get(
       [&](int, KernelConfig&) {
-        LPG_CUDA_TRY(cudaFuncSetAttribute(ipdg_ax_kernel<NQ, T, V4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+        LPG_CUDA_TRY(cudaFuncSetAttribute(ipdg_ax_kernel<NQ, float, float4>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         return (int)LPG_OK;
       },
       &cfg);
   if (rc) return rc;
-  ipdg_ax_kernel<NQ, T, V4><<<(unsigned)E, NP, smem, s>>>(vgeo, sgeo, vmapP, EToB, D, lambda, lambdaE, tau, g4, out);
+  ipdg_ax_kernel<NQ, float, float4><<<(unsigned)a.E, NP, smem, s>>>(a.vgeo, a.sgeo, a.vmapP, a.EToB, a.D, a.lambda,
+                                                                    a.lambdaE, a.tau, a.g4, a.out);
   LPG_LAUNCH_CHECK("ipdg_ax_kernel");
+  return LPG_OK;
+}
+
+template <int NQ, bool MASS>
+int launch_operator_fx(const IpdgArgs& a, cudaStream_t s) {
+  using L = FxLayout<NQ>;
+  constexpr int smem = (int)sizeof(double) * FxElement<NQ>::DOUBLES * L::EPB;
+  static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in
+  KernelConfig cfg;
+  const int rc = perDevice.get(
+      [&](int, KernelConfig&) {
+        LPG_CUDA_TRY(cudaFuncSetAttribute(ipdg_fx_trace_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        LPG_CUDA_TRY(
+            cudaFuncSetAttribute(ipdg_fx_ax_kernel<NQ, MASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        return (int)LPG_OK;
+      },
+      &cfg);
+  if (rc) return rc;
+  const unsigned blocks = (unsigned)((a.E + L::EPB - 1) / L::EPB);
+  ipdg_fx_trace_kernel<NQ><<<blocks, L::NT, smem, s>>>(a.E, a.fcoef, a.D, a.q, a.trace);
+  LPG_LAUNCH_CHECK("ipdg_fx_trace_kernel");
+  ipdg_fx_ax_kernel<NQ, MASS><<<blocks, L::NT, smem, s>>>(a.E, a.geo, a.fcoef, a.mapP, a.EToB, a.D, a.lambda, a.lambdaE,
+                                                          a.q, a.trace, a.out);
+  LPG_LAUNCH_CHECK("ipdg_fx_ax_kernel");
   return LPG_OK;
 }
 
@@ -662,11 +799,15 @@ int launch_all(int which, const IpdgArgs& a, cudaStream_t s) {
       LPG_LAUNCH_CHECK("ipdg_geometry_kernel");
       return LPG_OK;
     case 1:
-      return launch_operator<NQ, double, double4_32a>(a.E, a.vgeo, a.sgeo, a.vmapP, a.EToB, a.D, a.lambda, a.lambdaE,
-                                                      a.tau, a.q, a.g4, a.out, s);
+      return (a.lambdaE || a.lambda != 0.0) ? launch_operator_fx<NQ, true>(a, s) : launch_operator_fx<NQ, false>(a, s);
     case 2:
       ipdg_rhs_bc_kernel<NQ><<<E, NP, 0, s>>>(a.EX, a.EY, a.EZ, a.r1d, a.vgeo, a.sgeo, a.EToB, a.D, a.tau, a.out);
       LPG_LAUNCH_CHECK("ipdg_rhs_bc_kernel");
+      return LPG_OK;
+    case 3:
+      ipdg_face_coef_kernel<NQ><<<(unsigned)std::min<int64_t>((a.E * 6 * NQ * NQ + 255) / 256, 152 * 16), 256, 0, s>>>(
+          a.E, a.vgeo, a.sgeo, a.tau, a.fcoef);
+      LPG_LAUNCH_CHECK("ipdg_face_coef_kernel");
       return LPG_OK;
     default:
       ipdg_diag_kernel<NQ><<<E, NP, 0, s>>>(a.vgeo, a.sgeo, a.EToB, a.D, a.lambda, a.lambdaE, a.tau, a.out);
@@ -691,16 +832,16 @@ int dispatch(int which, const IpdgArgs& a, cudaStream_t s) {
 
 }  // namespace
 
-int ipdg_geometry(const IpdgArgs& a, const int32_t* mapP, cudaStream_t s) {
+int ipdg_geometry(const IpdgArgs& a, cudaStream_t s) {
   int rc = dispatch(0, a, s);
   if (rc) return rc;
   const int nfpAll = 6 * (a.N + 1) * (a.N + 1);
   const int64_t nf = a.E * nfpAll;
   if (nf <= 0) return LPG_OK;
   const int64_t blocks = std::min<int64_t>((nf + 255) / 256, 152 * 16);
-  ipdg_hinv_kernel<<<(unsigned)blocks, 256, 0, s>>>(nf, nfpAll, a.hfac, mapP, a.sgeo);
+  ipdg_hinv_kernel<<<(unsigned)blocks, 256, 0, s>>>(nf, nfpAll, a.hfac, a.mapP, a.sgeo);
   LPG_LAUNCH_CHECK("ipdg_hinv_kernel");
-  return LPG_OK;
+  return dispatch(3, a, s);
 }
 int ipdg_operator(const IpdgArgs& a, cudaStream_t s) { return dispatch(1, a, s); }
 int ipdg_operator_dw(const IpdgArgsDW& a, cudaStream_t s) {
@@ -742,8 +883,7 @@ int ipdg_operator_dw(const IpdgArgsDW& a, cudaStream_t s) {
 int ipdg_operator_f32(const IpdgArgsF32& a, cudaStream_t s) {
   auto go = [&](auto nq) {
     constexpr int NQ = decltype(nq)::value;
-    return launch_operator<NQ, float, float4>(a.E, a.vgeo, a.sgeo, a.vmapP, a.EToB, a.D, a.lambda, a.lambdaE, a.tau,
-                                              a.q, a.g4, a.out, s);
+    return launch_operator_f32<NQ>(a, s);
   };
   switch (a.N) {
     case 1: return go(std::integral_constant<int, 2>{});
@@ -758,6 +898,6 @@ int ipdg_operator_f32(const IpdgArgsF32& a, cudaStream_t s) {
   }
 }
 int ipdg_rhs_bc(const IpdgArgs& a, cudaStream_t s) { return dispatch(2, a, s); }
-int ipdg_diagonal(const IpdgArgs& a, cudaStream_t s) { return dispatch(3, a, s); }
+int ipdg_diagonal(const IpdgArgs& a, cudaStream_t s) { return dispatch(4, a, s); }
 
 }  // namespace lpg

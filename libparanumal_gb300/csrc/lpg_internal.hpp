@@ -201,18 +201,20 @@ int nb_directions(int64_t N, double beta, const double* u, const double* w, doub
 // ---------------------------------------------------------------- IPDG
 // Interior-penalty DG operator pieces (DISCRETIZATION = IPDG); unknowns are the E*Np
 // local nodes. vgeo [e][10][Np] (rx..tz, JW), sgeo [e][5][6 Nfp] (nx, ny, nz, WsJ, hinv),
-// vmapP [e][6][Nfp] (neighbour volume node), EToB [e][6], g4 [E*Np] gradient scratch.
+// fcoef [e][5][6 Nfp] (ipdg_hex.cu), mapP [e][6][Nfp] (paired face node), EToB [e][6], geo
+// [e][7][Np] (G00..G22, wJ), trace [E 6 Nfp] scratch.
 struct IpdgArgs {
   int N = 0;
   int64_t E = 0;
   const double *EX = nullptr, *EY = nullptr, *EZ = nullptr, *D = nullptr, *r1d = nullptr, *w1d = nullptr;
-  double *vgeo = nullptr, *sgeo = nullptr, *hfac = nullptr;
-  const int32_t* vmapP = nullptr;
+  const double* geo = nullptr;
+  double *vgeo = nullptr, *sgeo = nullptr, *fcoef = nullptr, *hfac = nullptr;
+  const int32_t* mapP = nullptr;
   const int* EToB = nullptr;
   double lambda = 0, tau = 0;
   const double* lambdaE = nullptr;
   const double* q = nullptr;
-  double4_32a* g4 = nullptr;
+  double2* trace = nullptr;
   double* out = nullptr;
 };
 // the operator on FP32 copies of vgeo, sgeo, D and lambdaE (preconditioner levels)
@@ -245,9 +247,9 @@ struct IpdgArgsDW {
   double* out = nullptr;
 };
 int ipdg_operator_dw(const IpdgArgsDW& a, cudaStream_t s);
-// vgeo, sgeo (hfac = scratch [E][6 Nfp]); mapP = paired face node of each face node
-int ipdg_geometry(const IpdgArgs& a, const int32_t* mapP, cudaStream_t s);
-int ipdg_operator(const IpdgArgs& a, cudaStream_t s);   // out = A q (q, g4 scratch)
+// vgeo, sgeo, fcoef (hfac = scratch [E][6 Nfp])
+int ipdg_geometry(const IpdgArgs& a, cudaStream_t s);
+int ipdg_operator(const IpdgArgs& a, cudaStream_t s);   // out = A q (trace scratch)
 int ipdg_rhs_bc(const IpdgArgs& a, cudaStream_t s);     // out -= boundary data terms
 int ipdg_diagonal(const IpdgArgs& a, cudaStream_t s);   // out = diag(A)
 
