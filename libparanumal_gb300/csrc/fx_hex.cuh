@@ -9,9 +9,11 @@
 // one direction contiguous, so one piece of code with immediate offsets serves all three, in
 // place.
 //
-// Nq = 4, 8: the GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
+// The GLL mirror symmetry D[N-i][N-m] = -D[i][m] (and D^T) halves the products:
 // with e_m = q_m + q_{N-m}, o_m = q_m - q_{N-m} (m < H = Nq/2), outputs t and N-t are A + B
 // and B - A, A = sum Dp[t][m] e_m, B = sum Dm[t][m] o_m, Dp/Dm[t][m] = (D[t][m] +- D[t][N-m])/2.
+// It is used for a D that satisfies it exactly, as this library's does, and for Nq = 4, 8
+// always; other matrices at other Nq are contracted row by row.
 #pragma once
 
 #include "fx64.cuh"
@@ -46,19 +48,20 @@ __device__ __forceinline__ bool ax_fx_sync(const int el, const bool any = false)
   }
 }
 
-template <int NQ>
+// EO: contract through the mirror symmetry (the caller vouches for D; Nq = 4 and 8 always do)
+template <int NQ, bool EO_ = true>
 struct FxLayout {
-  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ, H = NQ / 2;
-  static constexpr bool EO = (NQ == 4 || NQ == 8);
+  static constexpr bool EO = EO_ || NQ == 4 || NQ == 8;
+  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ, H = NQ / 2, MID = NQ % 2;
   static constexpr int P = NQ | 1, PL = P * NQ;      // odd row pitch: conflict-free lines
-  static constexpr int ROWS = EO ? H : NQ;           // rows of a table
-  static constexpr int COLS = EO ? 2 * H : NQ;       // (Dp, Dm) interleaved, or D
+  static constexpr int ROWS = EO ? H + MID : NQ;     // rows of a table
+  static constexpr int RS = (NQ + 1) & ~1;           // their length, 16-byte aligned
   // Bits S (fx64.cuh) of a line value (FS) and a table entry (DS): as many as keep the halves
-  // in 32 bits and, for any D, the sum of the middle quarters, COLS (EO: H per sum) products
-  // of each kind, and the sum of three transposed lines below 2^63. The mirror sums double a
-  // line value and a table entry (2 Dp).
-  static constexpr int FS = NQ <= 3 ? 8 : 7;
-  static constexpr int DS = NQ == 2 || NQ == 4 ? 8 : NQ == 9 ? 6 : 7;
+  // in 32 bits and, for any D, the sum of the middle quarters, Nq products of each kind (EO:
+  // half as many per sum, of doubled line values e, o and doubled entries 2 Dp, 2 Dm), and the
+  // sum of three transposed lines below 2^63.
+  static constexpr int FS = !EO && NQ <= 3 ? 8 : 7;
+  static constexpr int DS = EO ? (NQ <= 4 ? 8 : 7) : NQ == 2 ? 8 : NQ == 9 ? 6 : 7;
   static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
   static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
   static constexpr int NT = NL * EPB;
@@ -66,26 +69,30 @@ struct FxLayout {
   static constexpr int MINB = NQ == 9 ? 5 : 7;
 };
 
-// D (trans = false) or D^T in the layout's table: entry c of row t (2 Dp, 2 Dm)
-template <int NQ>
-__device__ __forceinline__ double fx_table_entry(const double* __restrict__ Dg, bool trans, int t, int c) {
-  using L = FxLayout<NQ>;
+// Table of D (trans = false) or D^T: row t holds 2 Dp[t][m], 2 Dm[t][m] (m < H) alternating,
+// then twice the middle entry for odd Nq; without EO the row itself. eR: exponent of the row.
+// The sums are formed in integers: rounded to FP64 they would perturb D (N = 6, smooth field:
+// error 1e-14 instead of 6e-16).
+template <int NQ, bool EO>
+__device__ __forceinline__ fx_half fx_table_entry(const double* __restrict__ Dg, bool trans, int t, int c, int eR) {
+  using L = FxLayout<NQ, EO>;
   const int rs = trans ? 1 : NQ, cs = trans ? NQ : 1;
   if constexpr (L::EO) {
-    const int m = c >> 1;
-    const double d0 = Dg[t * rs + m * cs], d1 = Dg[t * rs + (NQ - 1 - m) * cs];
-    return (c & 1) ? d0 - d1 : d0 + d1;
+    const int m = c >> 1;   // the middle entry: m = H, its own mirror
+    const int64_t d0 = fx_from_double<L::DS + 1>(Dg[t * rs + m * cs], eR);
+    const int64_t d1 = fx_from_double<L::DS + 1>(Dg[t * rs + (NQ - 1 - m) * cs], eR);
+    return fx_split((c & 1) ? d0 - d1 : d0 + d1);
   } else {
-    return Dg[t * rs + c * cs];
+    return fx_split(fx_from_double<L::DS + 1>(Dg[t * rs + c * cs], eR));
   }
 }
 
 // emit(t, sum_m table[t][m] q[m]) for the outputs t of one line, as integers in units of
 // 2^(eL + eR[t] - EXP)
-template <int NQ, typename F>
+template <int NQ, bool EO, typename F>
 __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, const fx_half* __restrict__ tab,
                                         F&& emit) {
-  using L = FxLayout<NQ>;
+  using L = FxLayout<NQ, EO>;
   constexpr int N = NQ - 1, H = L::H;
   int64_t f[NQ];
 #pragma unroll
@@ -97,31 +104,44 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
       x[2 * m] = fx_split(f[m] + f[N - m]);
       x[2 * m + 1] = fx_split(f[m] - f[N - m]);
     }
+    if constexpr (L::MID) x[2 * H] = fx_split(f[H]);
 #pragma unroll
     for (int t = 0; t < H; ++t) {
-      const int4* row = reinterpret_cast<const int4*>(tab + t * L::COLS);
-      fx_half dp[H], dm[H];
+      const int4* row = reinterpret_cast<const int4*>(tab + t * L::RS);
+      fx_half dp[H + 1], dm[H];
 #pragma unroll
       for (int m = 0; m < H; ++m) {
         const int4 v = row[m];
         dp[m] = {v.x, v.y};
         dm[m] = {v.z, v.w};
       }
+      if constexpr (L::MID) dp[H] = tab[t * L::RS + 2 * H];
       fx_acc A(x[0], dp[0]), B(x[1], dm[0]);
 #pragma unroll
-      for (int m = 1; m < H; ++m) {
-        A.cross(x[2 * m], dp[m]);
-        B.cross(x[2 * m + 1], dm[m]);
-      }
+      for (int m = 1; m < H + L::MID; ++m) A.cross(x[2 * m], dp[m]);
+#pragma unroll
+      for (int m = 1; m < H; ++m) B.cross(x[2 * m + 1], dm[m]);
       A.fold();
       B.fold();
 #pragma unroll
-      for (int m = 0; m < H; ++m) {
-        A.high(x[2 * m], dp[m]);
-        B.high(x[2 * m + 1], dm[m]);
-      }
+      for (int m = 0; m < H + L::MID; ++m) A.high(x[2 * m], dp[m]);
+#pragma unroll
+      for (int m = 0; m < H; ++m) B.high(x[2 * m + 1], dm[m]);
       emit(t, A.v + B.v + 1);   // both were rounded down
       emit(N - t, B.v - A.v);
+    }
+    if constexpr (L::MID) {   // the middle output: its row is odd
+      fx_acc B(0x40000000ll);
+      fx_half dm[H];
+#pragma unroll
+      for (int m = 0; m < H; ++m) {
+        dm[m] = tab[H * L::RS + 2 * m + 1];
+        B.cross(x[2 * m + 1], dm[m]);
+      }
+      B.fold();
+#pragma unroll
+      for (int m = 0; m < H; ++m) B.high(x[2 * m + 1], dm[m]);
+      emit(H, B.v);
     }
   } else {
 #pragma unroll
@@ -132,7 +152,7 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
       fx_half d[NQ];
 #pragma unroll
       for (int m = 0; m < NQ; ++m) {
-        d[m] = tab[t * L::COLS + m];
+        d[m] = tab[t * L::RS + m];
         A.cross(x[m], d[m]);
       }
       A.fold();
@@ -153,15 +173,15 @@ __device__ __forceinline__ bool fx_zero(const double (&v)[NQ], const unsigned ke
 }
 
 // row of the table that output t of a line uses
-template <int NQ>
+template <int NQ, bool EO>
 __device__ __forceinline__ constexpr int fx_row(int t) {
-  return FxLayout<NQ>::EO && t >= NQ / 2 ? NQ - 1 - t : t;
+  return FxLayout<NQ, EO>::EO && t > NQ - 1 - t ? NQ - 1 - t : t;
 }
 
 // one element's three copies in shared memory, seen by thread l = a + NQ b
 template <int NQ>
 struct FxElement {
-  using L = FxLayout<NQ>;
+  using L = FxLayout<NQ>;   // EO does not matter here
   static constexpr int DOUBLES = 3 * L::PL * NQ;   // of an element
   double* S;
   int l, a, b;
@@ -176,20 +196,20 @@ struct FxElement {
 
 // tables of D and D^T with the exponents of their rows, by the NT threads of a CTA; true where
 // an entry beyond 2^63 leaves every line to FP64
-template <int NQ>
+template <int NQ, bool EO>
 __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid,
-                                          fx_half (&tab)[2][FxLayout<NQ>::ROWS * FxLayout<NQ>::COLS],
-                                          int (&ex)[2][FxLayout<NQ>::ROWS]) {
-  using L = FxLayout<NQ>;
-  constexpr int TAB = L::ROWS * L::COLS;
+                                          fx_half (&tab)[2][FxLayout<NQ, EO>::ROWS * FxLayout<NQ, EO>::RS],
+                                          int (&ex)[2][FxLayout<NQ, EO>::ROWS]) {
+  using L = FxLayout<NQ, EO>;
+  constexpr int TAB = L::ROWS * NQ;
   bool plain = false;
   for (int w = tid; w < 2 * TAB; w += L::NT) {
-    const int tr = w / TAB, t = (w % TAB) / L::COLS, c = w % L::COLS;
+    const int tr = w / TAB, t = (w % TAB) / NQ, c = w % NQ;
     unsigned key = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) key = max(key, fx_key(Dg[tr ? m * NQ + t : t * NQ + m]));
     const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
-    tab[tr][t * L::COLS + c] = fx_split(fx_from_double<L::DS + 1>(fx_table_entry<NQ>(Dg, tr, t, c), eR));
+    tab[tr][t * L::RS + c] = fx_table_entry<NQ, EO>(Dg, tr, t, c, eR);
     if (c == 0) ex[tr][t] = eR;
     plain |= eR > 1086;
   }
@@ -197,10 +217,10 @@ __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const i
 }
 
 // the copies of q become D_r q, D_s q, D_t q
-template <int NQ>
+template <int NQ, bool EO>
 __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half* tab, const int* ex, const bool plain,
                                            const double* __restrict__ Dg) {
-  using L = FxLayout<NQ>;
+  using L = FxLayout<NQ, EO>;
 #pragma unroll 1
   for (int d = 0; d < 3; ++d) {
     double* const o = E.line(d);
@@ -214,8 +234,8 @@ __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half
     const int eL = (int)(key >> 20);
     asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
     if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ>(v, eL, tab, [&](int t, int64_t r) {
-        o[t] = fx_to_double(r, fx_base(eL + ex[fx_row<NQ>(t)] - (L::EXP - 1086)));
+      fx_line<NQ, EO>(v, eL, tab, [&](int t, int64_t r) {
+        o[t] = fx_to_double(r, fx_base(eL + ex[fx_row<NQ, EO>(t)] - (L::EXP - 1086)));
       });
     } else if (fx_zero<NQ>(v, key)) {
 #pragma unroll
@@ -234,7 +254,7 @@ __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half
 
 // the copies (u_r, u_s, u_t) become D_r^T u_r, D_s^T u_s, D_t^T u_t as integers, with the
 // exponents of the lines in x, -1 for a line kept as FP64 values; true if this thread kept one
-template <int NQ>
+template <int NQ, bool EO>
 __device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_half* tab, const bool plain,
                                               const double* __restrict__ Dg, int (&x)[3][FxLayout<NQ>::NL]) {
   bool fp = false;
@@ -252,7 +272,7 @@ __device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_h
     int xl = eL;
     asm volatile("" ::: "memory");
     if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ>(v, eL, tab, [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
+      fx_line<NQ, EO>(v, eL, tab, [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
     } else if (fx_zero<NQ>(v, key)) {
       xl = 128;
 #pragma unroll
@@ -275,13 +295,13 @@ __device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_h
 
 // sum of the three transposed parts at node (a, b, k); er, es: exponents of the rows a and b
 // of D^T; fp: some line of the element was kept in FP64
-template <int NQ>
+template <int NQ, bool EO>
 __device__ __forceinline__ double fx_node_sum(const FxElement<NQ>& E, const int k, const int (&x)[3][FxLayout<NQ>::NL],
                                               const int* ex, const int er, const int es, const bool fp) {
-  using L = FxLayout<NQ>;
+  using L = FxLayout<NQ, EO>;
   constexpr int OFF = L::EXP - 1086;
   const int lr = x[0][E.b + NQ * k], ls = x[1][E.a + NQ * k], lt = x[2][E.l];
-  const int xr = lr + er, xs = ls + es, xt = lt + ex[fx_row<NQ>(k)];
+  const int xr = lr + er, xs = ls + es, xt = lt + ex[fx_row<NQ, EO>(k)];
   const double vr = E.r(E.a, E.b, k), vs = E.s(E.a, E.b, k), vt = E.t(E.a, E.b, k);
   if (!fp || (lr | ls | lt) >= 0) {
     const int X = max(xr, max(xs, xt));

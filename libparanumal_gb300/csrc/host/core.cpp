@@ -223,6 +223,13 @@ void gll_derivative(int N, const std::vector<double>& x, std::vector<double>& D)
     }
     D[i * Nq + i] = diag;
   }
+  // the points are symmetric about 0, so D[N-i][N-j] = -D[i][j]: made exact, the FP64
+  // operators contract through it
+  for (int i = 0; i < Nq * Nq; ++i) {
+    const int mirror = Nq * Nq - 1 - i;
+    if (i < mirror) D[mirror] = -D[i];
+    else if (i == mirror) D[i] = 0.0;
+  }
 }
 
 void gll_interpolation(int Nc, int Nf, std::vector<double>& P) {

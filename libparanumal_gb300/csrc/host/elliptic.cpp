@@ -513,7 +513,7 @@ int Elliptic::OperatorDW(const double* q, double* Aq, cudaStream_t s) {
   const int64_t Np = mesh.Np;
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geoDW.p; a.geoStride = 7 * Np; a.wJ = mesh.geoDW.p + 6 * Np; a.wJStride = 7 * Np;
-  a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
+  a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
   a.q = q; a.out = Aq; a.Nglobal = Nglobal;
   return ax_hex_dw(a, s);
 }
@@ -532,7 +532,7 @@ int Elliptic::Operator(const double* q, double* Aq, cudaStream_t s) {
   const int64_t Np = mesh.Np;
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geo.p; a.geoStride = 7 * Np; a.wJ = mesh.geo.p + 6 * Np; a.wJStride = 7 * Np;
-  a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
+  a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
   a.q = q; a.out = Aq; a.Nglobal = Nglobal;
   return ax_hex<double, double>(a, AxMode::Assemble, s);
 }
@@ -696,14 +696,14 @@ int Elliptic::OperatorHost(const double* qHost, double* AqHost, cudaStream_t s) 
       AxArgs<double, float2> a;
       a.N = mesh.N; a.Nelements = a1 - a0; a.g2l = g2l.p + a0 * Np;
       a.ggeo = mesh.geoDW.p + a0 * 7 * Np; a.geoStride = 7 * Np; a.wJ = a.ggeo + 6 * Np; a.wJStride = 7 * Np;
-      a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
+      a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
       a.q = pipe->q.p; a.out = pipe->Aq.p; a.Nglobal = 0;   // accumulate: the pipeline zeroed Aq
       return ax_hex_dw(a, s);
     }
     AxArgs<double, double> a;
     a.N = mesh.N; a.Nelements = a1 - a0; a.g2l = g2l.p + a0 * Np;
     a.ggeo = mesh.geo.p + a0 * 7 * Np; a.geoStride = 7 * Np; a.wJ = a.ggeo + 6 * Np; a.wJStride = 7 * Np;
-    a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
+    a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
     a.q = pipe->q.p; a.out = pipe->Aq.p; a.Nglobal = Nglobal;
     return ax_hex<double, double>(a, AxMode::AccumulateAssembled, s);
   };
@@ -782,7 +782,7 @@ int Elliptic::BuildRhs(double* r, cudaStream_t s) {
     const int64_t Np = mesh.Np;
     a.N = mesh.N; a.Nelements = mesh.E; a.g2l = g2l.p;
     a.ggeo = mesh.geo.p; a.geoStride = 7 * Np; a.wJ = mesh.geo.p + 6 * Np; a.wJStride = 7 * Np;
-    a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
+    a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
     a.q = gL.p; a.out = rL.p;
     if ((rc = ax_hex<double, double>(a, AxMode::LocalInSubtract, s))) return rc;
   }

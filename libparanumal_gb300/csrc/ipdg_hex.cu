@@ -340,7 +340,7 @@ ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, 
   using L = FxLayout<NQ>;
   constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
   extern __shared__ __align__(16) unsigned char fx_smem[];
-  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::COLS];
+  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::RS];
   __shared__ int s_e[2][L::ROWS];
   const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
   const FxElement<NQ> S(reinterpret_cast<double*>(fx_smem) + el * FxElement<NQ>::DOUBLES, l);
@@ -352,12 +352,12 @@ ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, 
     double v[NQ];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
-    plain = fx_tables<NQ>(Dg, tid, s_tab, s_e);
+    plain = fx_tables<NQ, true>(Dg, tid, s_tab, s_e);
 #pragma unroll
     for (int k = 0; k < NQ; ++k) S.r(S.a, S.b, k) = S.s(S.a, S.b, k) = S.t(S.a, S.b, k) = v[k];
   }
   plain = __syncthreads_or(plain);
-  fx_forward<NQ>(S, s_tab[0], s_e[0], plain, Dg);
+  fx_forward<NQ, true>(S, s_tab[0], s_e[0], plain, Dg);
   ax_fx_sync<NQ, EPB>(el);
   if (!active) return;
   const double* fc = fcoef + e * 5 * NS + l;
@@ -383,7 +383,7 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
   using L = FxLayout<NQ>;
   constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
   extern __shared__ __align__(16) unsigned char fx_smem[];
-  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::COLS];
+  __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::RS];
   __shared__ int s_e[2][L::ROWS];
   __shared__ int s_x[EPB][3][NL];
   __shared__ double s_val[EPB][4 * NL + 1];   // value terms of faces 1, 3, 2, 4, and a zero
@@ -406,13 +406,13 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
     double v[NQ];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
-    plain = fx_tables<NQ>(Dg, tid, s_tab, s_e);
+    plain = fx_tables<NQ, true>(Dg, tid, s_tab, s_e);
     if (l == 0) s_val[el][4 * NL] = 0.0;
 #pragma unroll
     for (int k = 0; k < NQ; ++k) S.r(a, b, k) = S.s(a, b, k) = S.t(a, b, k) = v[k];
   }
   plain = __syncthreads_or(plain);
-  fx_forward<NQ>(S, s_tab[0], s_e[0], plain, Dg);
+  fx_forward<NQ, true>(S, s_tab[0], s_e[0], plain, Dg);
   ax_fx_sync<NQ, EPB>(el);
 
   int32_t mP[6];   // in flight over the metric product
@@ -455,12 +455,12 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
   s_val[el][2 * NL + l] = face(2, N, a, b);
   s_val[el][3 * NL + l] = face(4, 0, a, b);
   ax_fx_sync<NQ, EPB>(el);
-  bool fp = fx_transposed<NQ>(S, s_tab[1], plain, Dg, s_x[el]);
+  bool fp = fx_transposed<NQ, true>(S, s_tab[1], plain, Dg, s_x[el]);
   fp = ax_fx_sync<NQ, EPB>(el, fp);
 
   if (!active) return;
   const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
-  const int er = s_e[1][fx_row<NQ>(a)], es = s_e[1][fx_row<NQ>(b)];
+  const int er = s_e[1][fx_row<NQ, true>(a)], es = s_e[1][fx_row<NQ, true>(b)];
   // value terms of this column's nodes on the s faces (entries a + Nq k) and r faces (b + Nq k)
   const double* zero = &s_val[el][4 * NL];
   const double* ps = b == 0 ? &s_val[el][a] : b == N ? &s_val[el][NL + a] : zero;
@@ -468,7 +468,7 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
   const int ks = (b == 0 || b == N) ? NQ : 0, kr = (a == 0 || a == N) ? NQ : 0;
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    double r = fx_node_sum<NQ>(S, k, s_x[el], s_e[1], er, es, fp) + (ps[ks * k] + pr[kr * k]);
+    double r = fx_node_sum<NQ, true>(S, k, s_x[el], s_e[1], er, es, fp) + (ps[ks * k] + pr[kr * k]);
     if (k == 0) r += v0;
     if (k == N) r += v5;
     if constexpr (MASS) r = fma(gp[6 * NP + k * NL] * lam, qe[l + k * NL], r);

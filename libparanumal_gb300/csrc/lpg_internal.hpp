@@ -22,6 +22,7 @@ struct AxArgs {
   const G* wJ = nullptr;
   int64_t wJStride = 0;
   const T* D = nullptr;
+  bool mirrored = false;   // D[N-i][N-m] == -D[i][m] exactly (this library's D)
   T lambda = 0;
   const T* lambdaE = nullptr;
   const T* q = nullptr;
