@@ -65,8 +65,8 @@ struct FxLayout {
   static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
   static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
   static constexpr int NT = NL * EPB;
-  // resident CTAs per SM to compile for (registers): measured best of 5, 6, 7, 8
-  static constexpr int MINB = NQ == 9 ? 5 : 7;
+  // resident CTAs per SM to compile for (registers): measured best of 5 to 10
+  static constexpr int MINB = NQ == 9 ? 5 : NQ <= 4 ? 10 : 7;
 };
 
 // Table of D (trans = false) or D^T: row t holds 2 Dp[t][m], 2 Dm[t][m] (m < H) alternating,
