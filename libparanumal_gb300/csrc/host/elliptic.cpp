@@ -505,7 +505,7 @@ int Elliptic::OperatorIpdgDW(const double* q, double* Aq, cudaStream_t s) {
   return ipdg_operator_dw(a, s);
 }
 
-int Elliptic::OperatorDW(const double* q, double* Aq, cudaStream_t s) {
+int Elliptic::OperatorDW(const double* q, double* Aq, cudaStream_t s, bool zeroed) {
   if (ipdg) return OperatorIpdgDW(q, Aq, s);
   int rc;
   if ((rc = mesh.make_dw(s))) return rc;
@@ -514,11 +514,11 @@ int Elliptic::OperatorDW(const double* q, double* Aq, cudaStream_t s) {
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geoDW.p; a.geoStride = 7 * Np; a.wJ = mesh.geoDW.p + 6 * Np; a.wJStride = 7 * Np;
   a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
-  a.q = q; a.out = Aq; a.Nglobal = Nglobal;
+  a.q = q; a.out = Aq; a.Nglobal = zeroed ? 0 : Nglobal;
   return ax_hex_dw(a, s);
 }
 
-int Elliptic::Operator(const double* q, double* Aq, cudaStream_t s) {
+int Elliptic::Operator(const double* q, double* Aq, cudaStream_t s, bool zeroed) {
   ++nOps;
   if (ipdg && opDW) return OperatorIpdgDW(q, Aq, s);
   if (ipdg) {
@@ -527,14 +527,14 @@ int Elliptic::Operator(const double* q, double* Aq, cudaStream_t s) {
     a.out = Aq;
     return ipdg_operator(a, s);
   }
-  if (opDW) return OperatorDW(q, Aq, s);
+  if (opDW) return OperatorDW(q, Aq, s, zeroed);
   AxArgs<double, double> a;
   const int64_t Np = mesh.Np;
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geo.p; a.geoStride = 7 * Np; a.wJ = mesh.geo.p + 6 * Np; a.wJStride = 7 * Np;
   a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
   a.q = q; a.out = Aq; a.Nglobal = Nglobal;
-  return ax_hex<double, double>(a, AxMode::Assemble, s);
+  return ax_hex<double, double>(a, zeroed ? AxMode::AccumulateAssembled : AxMode::Assemble, s);
 }
 
 int Elliptic::OperatorF32(const float* q, float* Aq, Prec prec, cudaStream_t s, float accumulate) {

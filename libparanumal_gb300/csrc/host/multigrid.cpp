@@ -1121,6 +1121,7 @@ class JacobiPrecon : public Precon {
   Elliptic* el;
   DevBuf<double> invDiag;
   explicit JacobiPrecon(Elliptic* e) : el(e) {}
+  const double* diagonal_scaling() const override { return el->allNeumann ? nullptr : invDiag.p; }
   int apply(const double* r, double* z, cudaStream_t s) override {
     int rc = amxpy<double>(el->Nglobal, 1.0, invDiag.p, r, 0.0, z, s);
     if (rc) return rc;

@@ -201,8 +201,9 @@ struct Elliptic {
   // OPERATOR PRECISION: FP64 (default) or DF64 (double-FP32 words on the FP32 pipe,
   // FP64-accurate) for every FP64 operator application of this object
   bool opDW = false;
-  int Operator(const double* q, double* Aq, cudaStream_t s);
-  int OperatorDW(const double* q, double* Aq, cudaStream_t s);
+  // zeroed: Aq is already 0 (a C0 operator then assembles into it without clearing it)
+  int Operator(const double* q, double* Aq, cudaStream_t s, bool zeroed = false);
+  int OperatorDW(const double* q, double* Aq, cudaStream_t s, bool zeroed = false);
   // accumulate = 0: Aq = A q; otherwise Aq += accumulate * A q (C0 only)
   // accumulate != 0: Aq += accumulate * A q (C0 only)
   int OperatorF32(const float* q, float* Aq, Prec prec, cudaStream_t s, float accumulate = 0.f);
@@ -232,6 +233,9 @@ struct Precon {
     *z32 = nullptr;
     return apply(r, z, s);
   }
+  // 1/diag where apply() is z = invDiag .* r and nothing else, so that a Krylov loop can form z
+  // in a pass of its own; otherwise nullptr
+  virtual const double* diagonal_scaling() const { return nullptr; }
   virtual int levels_p() const { return 0; }
   virtual int levels_amg() const { return 0; }
   virtual int64_t coarse_n() const { return 0; }
@@ -279,6 +283,7 @@ struct PCGResult {
 };
 struct PCGWork {
   DevBuf<double> p, z, Ax, Ap;
+  DevBuf<PcgScalars> sc;
   int ensure(int64_t n);
 };
 int pcg_solve(Platform* plat, Elliptic* el, Precon* pc, PCGWork& w, bool flexible, bool stopRhs,

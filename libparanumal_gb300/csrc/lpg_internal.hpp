@@ -132,10 +132,24 @@ int dot2(int64_t N, const T* x, const T* y, const T* z, double* out2, double* pa
 template <typename T> int update2(int64_t N, T a, const T* p, const T* q, T* x, T* r, cudaStream_t s);
 // update2 with a = sc[0] / sc[1] from device memory (0 when sc[1] <= 0 or not finite)
 template <typename T> int update2_dev(int64_t N, const double* sc, const T* p, const T* q, T* x, T* r, cudaStream_t s);
-// FPCG with an FP32 preconditioner output z: out2 = (r.z, z.Ap) in FP64, and p = z + beta p
-int dot2_mixed(int64_t N, const float* z, const double* r, const double* Ap, double* out2, double* partials,
-               cudaStream_t s);
-int direction_mixed(int64_t N, const float* z, double beta, double* p, cudaStream_t s);
+// (flexible) PCG iterations on device scalars (vec_ops.cu): z in FP64 or FP32, partials holds
+// kReducePartials doubles, done counts finished blocks (0 between kernels)
+struct PcgScalars {
+  double rz, beta, pAp, alpha, rr;
+  unsigned done;
+};
+// r.z (and z.Ap), then beta; with invDiag (FP64 z) z = invDiag .* r first
+template <typename TZ>
+int pcg_dots(int64_t N, const double* invDiag, const double* r, TZ* z, const double* Ap, bool flexible, bool first,
+             double* partials, PcgScalars* sc, cudaStream_t s);
+// p = z + beta p (beta = 0 ignores p); Ap = 0 if zeroAp
+template <typename TZ>
+int pcg_direction(int64_t N, const PcgScalars* sc, const TZ* z, double* p, double* Ap, bool zeroAp, cudaStream_t s);
+// p.Ap, alpha = r.z / p.Ap
+int pcg_curvature(int64_t N, const double* p, const double* Ap, double* partials, PcgScalars* sc, cudaStream_t s);
+// x += alpha p, r -= alpha Ap, r.r; nothing where p.Ap is not positive and finite
+int pcg_step(int64_t N, const double* p, const double* Ap, double* x, double* r, double* partials, PcgScalars* sc,
+             cudaStream_t s);
 // halo exchange halves: buf[i] = v[idx[i]]; v[idx[i]] += buf[i]
 int halo_pack(int64_t n, const int32_t* idx, const double* v, double* buf, cudaStream_t s);
 int halo_unpack_add(int64_t n, const int32_t* idx, const double* buf, double* v, cudaStream_t s);

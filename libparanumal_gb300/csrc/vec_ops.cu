@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "df64.cuh"
 #include "lpg_common.cuh"
 #include "lpg_internal.hpp"
 
@@ -360,17 +361,52 @@ int dot2(int64_t N, const T* x, const T* y, const T* z, double* out2, double* pa
 template int dot2<double>(int64_t, const double*, const double*, const double*, double*, double*, cudaStream_t);
 template int dot2<float>(int64_t, const float*, const float*, const float*, double*, double*, cudaStream_t);
 
-// FPCG with an FP32 preconditioner output z: out[0] = r.z, out[1] = z.Ap with z widened
-// exactly to FP64 and FP64 products; and p = z + beta p. z is read as FP32 and never
-// stored as FP64.
+// ---------------------------------------------------------------- PCG passes
+// One iteration of (flexible) PCG without a host round trip between its steps: alpha, beta and
+// the inner products stay in device memory (PcgScalars) and the host reads them once an
+// iteration. Each reduction is one kernel: the block that finishes last adds the partial sums
+// in block order, so the result does not depend on which block that is.
+__device__ __forceinline__ bool last_block(unsigned* done) {
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();   // this block's partial sums before its count
+    s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (s_last) *done = 0;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+__device__ __forceinline__ double sum_partials(const double* partials) {
+  double v = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v += __ldcg(partials + i);
+  return block_sum(v);   // thread 0
+}
+// exact widening of z; from FP32 by integers, as the FP64 pipe (2 lanes a clock and SM, and
+// needed for the products) also does the conversions
+__device__ __forceinline__ double pcg_widen(double z) { return z; }
+__device__ __forceinline__ double pcg_widen(float z) { return (fabsf(z) < 1.17549435e-38f) ? (double)z : dw_float_to_double(z); }
+
+// r.z and, if flexible, z.Ap; then beta = -alpha z.Ap / (r.z before) or r.z / (r.z before),
+// 0 in the first iteration. JACOBI: z = invDiag .* r is formed (and stored) here.
+template <typename TZ, bool JACOBI>
 __global__ void __launch_bounds__(kRedThreads)
-dot2_mixed_stage1(const int64_t N, const float* __restrict__ z, const double* __restrict__ r,
-                  const double* __restrict__ Ap, double* __restrict__ partials) {
+pcg_dots_kernel(const int64_t N, const double* __restrict__ invDiag, const double* __restrict__ r, TZ* __restrict__ z,
+                const double* __restrict__ Ap, const int flexible, const int first, double* __restrict__ partials,
+                PcgScalars* __restrict__ sc) {
   double a = 0, b = 0;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
-    const double zn = (double)z[n];
-    a += r[n] * zn;
-    b += zn * Ap[n];
+    const double rn = r[n];
+    double zn;
+    if constexpr (JACOBI) {
+      zn = invDiag[n] * rn;
+      z[n] = zn;
+    } else {
+      zn = pcg_widen(z[n]);
+    }
+    a += rn * zn;
+    if (flexible) b += zn * Ap[n];
   }
   a = block_sum(a);
   b = block_sum(b);
@@ -378,25 +414,101 @@ dot2_mixed_stage1(const int64_t N, const float* __restrict__ z, const double* __
     partials[blockIdx.x] = a;
     partials[gridDim.x + blockIdx.x] = b;
   }
+  if (!last_block(&sc->done)) return;
+  a = sum_partials(partials);
+  b = sum_partials(partials + gridDim.x);
+  if (threadIdx.x == 0) {
+    sc->beta = first ? 0.0 : flexible ? -sc->alpha * b / sc->rz : a / sc->rz;
+    sc->rz = a;
+  }
 }
-int dot2_mixed(int64_t N, const float* z, const double* r, const double* Ap, double* out2, double* partials,
-               cudaStream_t s) {
+template <typename TZ>
+int pcg_dots(int64_t N, const double* invDiag, const double* r, TZ* z, const double* Ap, bool flexible, bool first,
+             double* partials, PcgScalars* sc, cudaStream_t s) {
   const int nb = std::min(red_blocks(N), kReducePartials / 2);
-  dot2_mixed_stage1<<<nb, kRedThreads, 0, s>>>(N, z, r, Ap, partials);
-  LPG_LAUNCH_CHECK("dot2_mixed_stage1");
-  dot2_stage2<<<1, kRedThreads, 0, s>>>(nb, partials, out2);
-  LPG_LAUNCH_CHECK("dot2_stage2");
+  if constexpr (std::is_same<TZ, double>::value) {
+    if (invDiag) {
+      pcg_dots_kernel<TZ, true><<<nb, kRedThreads, 0, s>>>(N, invDiag, r, z, Ap, flexible, first, partials, sc);
+      LPG_LAUNCH_CHECK("pcg_dots_kernel");
+      return LPG_OK;
+    }
+  }
+  pcg_dots_kernel<TZ, false><<<nb, kRedThreads, 0, s>>>(N, nullptr, r, z, Ap, flexible, first, partials, sc);
+  LPG_LAUNCH_CHECK("pcg_dots_kernel");
   return LPG_OK;
 }
-__global__ void direction_mixed_kernel(const int64_t N, const float* __restrict__ z, const double beta,
-                                       double* __restrict__ p) {
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x)
-    p[n] = (double)z[n] + beta * p[n];
+template int pcg_dots<double>(int64_t, const double*, const double*, double*, const double*, bool, bool, double*,
+                              PcgScalars*, cudaStream_t);
+template int pcg_dots<float>(int64_t, const double*, const double*, float*, const double*, bool, bool, double*,
+                             PcgScalars*, cudaStream_t);
+
+// p = z + beta p, and Ap = 0 for the operator to assemble into (zeroAp)
+template <typename TZ>
+__global__ void __launch_bounds__(256)
+pcg_direction_kernel(const int64_t N, const PcgScalars* __restrict__ sc, const TZ* __restrict__ z,
+                     double* __restrict__ p, double* __restrict__ Ap, const int zeroAp) {
+  const double beta = sc->beta;
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
+    p[n] = pcg_widen(z[n]) + (beta != 0.0 ? beta * p[n] : 0.0);
+    if (zeroAp) Ap[n] = 0.0;
+  }
 }
-int direction_mixed(int64_t N, const float* z, double beta, double* p, cudaStream_t s) {
+template <typename TZ>
+int pcg_direction(int64_t N, const PcgScalars* sc, const TZ* z, double* p, double* Ap, bool zeroAp, cudaStream_t s) {
   if (N <= 0) return LPG_OK;
-  direction_mixed_kernel<<<grid_for(N, 256, kStreamCap), 256, 0, s>>>(N, z, beta, p);
-  LPG_LAUNCH_CHECK("direction_mixed_kernel");
+  pcg_direction_kernel<TZ><<<grid_for(N, 256, kStreamCap), 256, 0, s>>>(N, sc, z, p, Ap, zeroAp ? 1 : 0);
+  LPG_LAUNCH_CHECK("pcg_direction_kernel");
+  return LPG_OK;
+}
+template int pcg_direction<double>(int64_t, const PcgScalars*, const double*, double*, double*, bool, cudaStream_t);
+template int pcg_direction<float>(int64_t, const PcgScalars*, const float*, double*, double*, bool, cudaStream_t);
+
+// p.Ap and alpha = r.z / p.Ap
+__global__ void __launch_bounds__(kRedThreads)
+pcg_curvature_kernel(const int64_t N, const double* __restrict__ p, const double* __restrict__ Ap,
+                     double* __restrict__ partials, PcgScalars* __restrict__ sc) {
+  double a = 0;
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x)
+    a += p[n] * Ap[n];
+  a = block_sum(a);
+  if (threadIdx.x == 0) partials[blockIdx.x] = a;
+  if (!last_block(&sc->done)) return;
+  a = sum_partials(partials);
+  if (threadIdx.x == 0) {
+    sc->pAp = a;
+    sc->alpha = sc->rz / a;
+  }
+}
+int pcg_curvature(int64_t N, const double* p, const double* Ap, double* partials, PcgScalars* sc, cudaStream_t s) {
+  pcg_curvature_kernel<<<red_blocks(N), kRedThreads, 0, s>>>(N, p, Ap, partials, sc);
+  LPG_LAUNCH_CHECK("pcg_curvature_kernel");
+  return LPG_OK;
+}
+
+// x += alpha p; r -= alpha Ap; r.r -- unless p.Ap is not positive and finite (a breakdown,
+// which leaves x and r)
+__global__ void __launch_bounds__(kRedThreads)
+pcg_step_kernel(const int64_t N, const double* __restrict__ p, const double* __restrict__ Ap, double* __restrict__ x,
+                double* __restrict__ r, double* __restrict__ partials, PcgScalars* __restrict__ sc) {
+  if (!(sc->pAp > 0.0) || !isfinite(sc->pAp)) return;
+  const double alpha = sc->alpha;
+  double acc = 0;
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
+    x[n] += alpha * p[n];
+    const double rn = r[n] - alpha * Ap[n];
+    r[n] = rn;
+    acc += rn * rn;
+  }
+  acc = block_sum(acc);
+  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+  if (!last_block(&sc->done)) return;
+  acc = sum_partials(partials);
+  if (threadIdx.x == 0) sc->rr = acc;
+}
+int pcg_step(int64_t N, const double* p, const double* Ap, double* x, double* r, double* partials, PcgScalars* sc,
+             cudaStream_t s) {
+  pcg_step_kernel<<<red_blocks(N), kRedThreads, 0, s>>>(N, p, Ap, x, r, partials, sc);
+  LPG_LAUNCH_CHECK("pcg_step_kernel");
   return LPG_OK;
 }
 
