@@ -137,7 +137,6 @@ void DevBuf<T>::release() {
   n = 0;
 }
 template struct DevBuf<double>;
-template struct DevBuf<PcgScalars>;
 template struct DevBuf<float>;
 template struct DevBuf<int32_t>;
 template struct DevBuf<int64_t>;

@@ -74,7 +74,7 @@ double hessenberg_spectral_radius(int k, const std::vector<double>& Hcolmajor);
 struct Platform {
   cudaStream_t stream = nullptr;
   DevBuf<double> partials;   // reduction partial sums
-  DevBuf<double> scalars;    // device scalars for reductions
+  DevBuf<double> scalars;    // device scalars for reductions; the last 8 are PCG's (PcgScalars)
   double* hostScalars = nullptr;  // pinned mirror
   int init();
   ~Platform();
@@ -283,7 +283,8 @@ struct PCGResult {
 };
 struct PCGWork {
   DevBuf<double> p, z, Ax, Ap;
-  DevBuf<PcgScalars> sc;
+  cudaEvent_t read[2] = {nullptr, nullptr};   // an iteration's scalars have reached the host
+  ~PCGWork();
   int ensure(int64_t n);
 };
 int pcg_solve(Platform* plat, Elliptic* el, Precon* pc, PCGWork& w, bool flexible, bool stopRhs,

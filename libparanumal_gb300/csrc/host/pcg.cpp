@@ -2,7 +2,7 @@
 // (libs/linearSolver/linearSolverPCG.cpp:67-171). Vector updates, reductions, alpha and beta
 // are formed on the device; the host reads p.Ap and r.r once an iteration to decide on
 // convergence (the reference's host reads every inner product: with four reads an iteration
-// 8^3, N = 5, Jacobi took 23.1 ms a solve, with one 10.3 ms).
+// 8^3, N = 5, Jacobi took 23.1 ms a solve, with one 10.3 ms, queued ahead 8.0 ms).
 #include "objects.hpp"
 
 #include <algorithm>
@@ -10,14 +10,17 @@
 
 namespace lpg {
 
+PCGWork::~PCGWork() {
+  for (cudaEvent_t ev : read)
+    if (ev) cudaEventDestroy(ev);
+}
+
 int PCGWork::ensure(int64_t n) {
   if (p.n == n) return LPG_OK;
   int rc;
-  if ((rc = p.alloc(n)) || (rc = z.alloc(n)) || (rc = Ax.alloc(n)) || (rc = Ap.alloc(n)) || (rc = sc.alloc(1)))
-    return rc;
+  if ((rc = p.alloc(n)) || (rc = z.alloc(n)) || (rc = Ax.alloc(n)) || (rc = Ap.alloc(n))) return rc;
   LPG_CUDA_TRY(cudaMemset(p.p, 0, sizeof(double) * n));
   LPG_CUDA_TRY(cudaMemset(Ap.p, 0, sizeof(double) * n));
-  LPG_CUDA_TRY(cudaMemset(sc.p, 0, sizeof(PcgScalars)));
   return LPG_OK;
 }
 
@@ -47,31 +50,62 @@ int pcg_solve(Platform* plat, Elliptic* el, Precon* pc, PCGWork& w, bool flexibl
     res.rdotr = rdotr0;
     return LPG_OK;
   }
-  PcgScalars* sc = w.sc.p;
-  PcgScalars* got = reinterpret_cast<PcgScalars*>(plat->hostScalars);   // page-locked
+  static_assert(sizeof(PcgScalars) <= 8 * sizeof(double), "the second half of Platform::scalars");
+  PcgScalars* sc = reinterpret_cast<PcgScalars*>(plat->scalars.p + 8);
+  for (cudaEvent_t& ev : w.read)
+    if (!ev) LPG_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  LPG_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(PcgScalars), s));
+  PcgScalars* got = reinterpret_cast<PcgScalars*>(plat->hostScalars);   // page-locked, two iterations
   const double* invDiag = pc->diagonal_scaling();
   const bool zeroAp = !el->ipdg;
-  for (iter = 0; iter < maxit; ++iter) {
-    if ((iter == 0 && rdotr0 == 0.0) || (iter > 0 && rdotr0 <= TOL)) break;
+  // one iteration, and the copy of its scalars to got[k & 1]
+  auto enqueue = [&](int k) -> int {
+    int rc;
     const float* z32 = nullptr;   // an FP32 preconditioner's output, widened exactly where it is read
-    const bool first = iter == 0;
-    if (!invDiag && (rc = pc->apply_mixed(r, w.z.p, &z32, s))) return rc;
-    if (z32)
-      rc = pcg_dots<float>(N, nullptr, r, const_cast<float*>(z32), w.Ap.p, flexible, first, plat->partials.p, sc, s);
-    else
-      rc = pcg_dots<double>(N, invDiag, r, w.z.p, w.Ap.p, flexible, first, plat->partials.p, sc, s);
-    if (rc) return rc;
-    if (z32) rc = pcg_direction<float>(N, sc, z32, w.p.p, w.Ap.p, zeroAp, s);
-    else rc = pcg_direction<double>(N, sc, w.z.p, w.p.p, w.Ap.p, zeroAp, s);
+    if (invDiag) {   // later iterations' inner products come with the step before them
+      if (k == 0) rc = pcg_dots<double>(N, invDiag, r, nullptr, w.Ap.p, flexible, true, plat->partials.p, sc, s);
+      else rc = LPG_OK;
+      if (!rc) rc = pcg_direction<double>(N, sc, invDiag, r, w.p.p, w.Ap.p, zeroAp, s);
+    } else {
+      if ((rc = pc->apply_mixed(r, w.z.p, &z32, s))) return rc;
+      if (z32) {
+        if ((rc = pcg_dots<float>(N, nullptr, r, z32, w.Ap.p, flexible, k == 0, plat->partials.p, sc, s))) return rc;
+        rc = pcg_direction<float>(N, sc, nullptr, z32, w.p.p, w.Ap.p, zeroAp, s);
+      } else {
+        if ((rc = pcg_dots<double>(N, nullptr, r, w.z.p, w.Ap.p, flexible, k == 0, plat->partials.p, sc, s))) return rc;
+        rc = pcg_direction<double>(N, sc, nullptr, w.z.p, w.p.p, w.Ap.p, zeroAp, s);
+      }
+    }
     if (rc) return rc;
     if ((rc = el->Operator(w.p.p, w.Ap.p, s, zeroAp))) return rc;
     if ((rc = pcg_curvature(N, w.p.p, w.Ap.p, plat->partials.p, sc, s))) return rc;
-    if ((rc = pcg_step(N, w.p.p, w.Ap.p, x, r, plat->partials.p, sc, s))) return rc;
-    LPG_CUDA_TRY(cudaMemcpyAsync(got, sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s));
-    LPG_CUDA_TRY(cudaStreamSynchronize(s));
-    if (!(got->pAp > 0.0) || !std::isfinite(got->pAp)) { res.breakdown = true; break; }
-    rdotr0 = got->rr;
-    if (!std::isfinite(rdotr0)) { res.breakdown = true; ++iter; break; }
+    if ((rc = pcg_step(N, invDiag, w.p.p, w.Ap.p, x, r, TOL, flexible, plat->partials.p, sc, s))) return rc;
+    LPG_CUDA_TRY(cudaMemcpyAsync(got + (k & 1), sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s));
+    LPG_CUDA_TRY(cudaEventRecord(w.read[k & 1], s));
+    return LPG_OK;
+  };
+  // With diagonal scaling the host queues iteration k + 1 before it waits for iteration k, so
+  // the GPU does not idle over the read; the one queued past the end does nothing but an
+  // operator application on work vectors. A preconditioner with an apply() of its own is too
+  // much work to run once in vain.
+  const int ahead = invDiag ? 1 : 0;
+  int queued = 0;
+  iter = 0;
+  if (rdotr0 != 0.0 && maxit > 0) {
+    for (;;) {
+      while (queued < maxit && queued <= iter + ahead)
+        if ((rc = enqueue(queued++))) return rc;
+      LPG_CUDA_TRY(cudaEventSynchronize(w.read[iter & 1]));
+      const PcgScalars& it = got[iter & 1];
+      if (it.stop == 2) { res.breakdown = true; break; }
+      rdotr0 = it.rr;
+      ++iter;
+      if (it.stop) { res.breakdown = it.stop == 3; break; }
+      if (iter == maxit) break;
+    }
+    if (ahead) LPG_CUDA_TRY(cudaStreamSynchronize(s));
+    // what was queued past the end is no application of the solve
+    el->nOps -= queued - (res.breakdown && iter < queued && got[iter & 1].stop == 2 ? iter + 1 : iter);
   }
   res.iters = iter;
   res.rdotr = rdotr0;

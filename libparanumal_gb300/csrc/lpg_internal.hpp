@@ -137,19 +137,22 @@ template <typename T> int update2_dev(int64_t N, const double* sc, const T* p, c
 struct PcgScalars {
   double rz, beta, pAp, alpha, rr;
   unsigned done;
+  int stop;   // 0 running, 1 converged, 2 p.Ap not positive and finite, 3 r.r not finite
 };
-// r.z (and z.Ap), then beta; with invDiag (FP64 z) z = invDiag .* r first
+// r.z (and z.Ap), then beta; with invDiag (FP64) z = invDiag .* r and the argument z is not read
 template <typename TZ>
-int pcg_dots(int64_t N, const double* invDiag, const double* r, TZ* z, const double* Ap, bool flexible, bool first,
-             double* partials, PcgScalars* sc, cudaStream_t s);
-// p = z + beta p (beta = 0 ignores p); Ap = 0 if zeroAp
+int pcg_dots(int64_t N, const double* invDiag, const double* r, const TZ* z, const double* Ap, bool flexible,
+             bool first, double* partials, PcgScalars* sc, cudaStream_t s);
+// p = z + beta p (beta = 0 ignores p); Ap = 0 if zeroAp; with invDiag (FP64) z is r to be scaled
 template <typename TZ>
-int pcg_direction(int64_t N, const PcgScalars* sc, const TZ* z, double* p, double* Ap, bool zeroAp, cudaStream_t s);
+int pcg_direction(int64_t N, const PcgScalars* sc, const double* invDiag, const TZ* z, double* p, double* Ap,
+                  bool zeroAp, cudaStream_t s);
 // p.Ap, alpha = r.z / p.Ap
 int pcg_curvature(int64_t N, const double* p, const double* Ap, double* partials, PcgScalars* sc, cudaStream_t s);
-// x += alpha p, r -= alpha Ap, r.r; nothing where p.Ap is not positive and finite
-int pcg_step(int64_t N, const double* p, const double* Ap, double* x, double* r, double* partials, PcgScalars* sc,
-             cudaStream_t s);
+// x += alpha p, r -= alpha Ap, r.r; stops at r.r <= tol; with invDiag pcg_dots of the next
+// iteration in the same pass
+int pcg_step(int64_t N, const double* invDiag, const double* p, const double* Ap, double* x, double* r, double tol,
+             bool flexible, double* partials, PcgScalars* sc, cudaStream_t s);
 // halo exchange halves: buf[i] = v[idx[i]]; v[idx[i]] += buf[i]
 int halo_pack(int64_t n, const int32_t* idx, const double* v, double* buf, cudaStream_t s);
 int halo_unpack_add(int64_t n, const int32_t* idx, const double* buf, double* v, cudaStream_t s);

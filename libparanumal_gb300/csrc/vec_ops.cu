@@ -264,7 +264,9 @@ reduce_stage2(const int nparts, const double* __restrict__ partials, double* __r
 }
 
 static inline int red_blocks(int64_t N) {
-  int64_t b = (N + kRedThreads * 4 - 1) / (kRedThreads * 4);
+  // one entry a thread until the partial sums run out: a thread's entries are read one after
+  // the other (59,319 entries at four a thread: the PCG update took 10 us against 8)
+  int64_t b = (N + kRedThreads - 1) / kRedThreads;
   if (b > kReducePartials) b = kReducePartials;
   if (b < 1) b = 1;
   return (int)b;
@@ -389,22 +391,22 @@ __device__ __forceinline__ double pcg_widen(double z) { return z; }
 __device__ __forceinline__ double pcg_widen(float z) { return (fabsf(z) < 1.17549435e-38f) ? (double)z : dw_float_to_double(z); }
 
 // r.z and, if flexible, z.Ap; then beta = -alpha z.Ap / (r.z before) or r.z / (r.z before),
-// 0 in the first iteration. JACOBI: z = invDiag .* r is formed (and stored) here.
+// 0 in the first iteration. With invDiag z = invDiag .* r, which is not stored.
+__device__ __forceinline__ void pcg_beta(PcgScalars* sc, double rz, double zAp, int flexible, int first) {
+  sc->beta = first ? 0.0 : flexible ? -sc->alpha * zAp / sc->rz : rz / sc->rz;
+  sc->rz = rz;
+}
 template <typename TZ, bool JACOBI>
 __global__ void __launch_bounds__(kRedThreads)
-pcg_dots_kernel(const int64_t N, const double* __restrict__ invDiag, const double* __restrict__ r, TZ* __restrict__ z,
-                const double* __restrict__ Ap, const int flexible, const int first, double* __restrict__ partials,
-                PcgScalars* __restrict__ sc) {
+pcg_dots_kernel(const int64_t N, const double* __restrict__ invDiag, const double* __restrict__ r,
+                const TZ* __restrict__ z, const double* __restrict__ Ap, const int flexible, const int first,
+                double* __restrict__ partials, PcgScalars* __restrict__ sc) {
   double a = 0, b = 0;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
     const double rn = r[n];
     double zn;
-    if constexpr (JACOBI) {
-      zn = invDiag[n] * rn;
-      z[n] = zn;
-    } else {
-      zn = pcg_widen(z[n]);
-    }
+    if constexpr (JACOBI) zn = invDiag[n] * rn;
+    else zn = pcg_widen(z[n]);
     a += rn * zn;
     if (flexible) b += zn * Ap[n];
   }
@@ -417,14 +419,11 @@ pcg_dots_kernel(const int64_t N, const double* __restrict__ invDiag, const doubl
   if (!last_block(&sc->done)) return;
   a = sum_partials(partials);
   b = sum_partials(partials + gridDim.x);
-  if (threadIdx.x == 0) {
-    sc->beta = first ? 0.0 : flexible ? -sc->alpha * b / sc->rz : a / sc->rz;
-    sc->rz = a;
-  }
+  if (threadIdx.x == 0) pcg_beta(sc, a, b, flexible, first);
 }
 template <typename TZ>
-int pcg_dots(int64_t N, const double* invDiag, const double* r, TZ* z, const double* Ap, bool flexible, bool first,
-             double* partials, PcgScalars* sc, cudaStream_t s) {
+int pcg_dots(int64_t N, const double* invDiag, const double* r, const TZ* z, const double* Ap, bool flexible,
+             bool first, double* partials, PcgScalars* sc, cudaStream_t s) {
   const int nb = std::min(red_blocks(N), kReducePartials / 2);
   if constexpr (std::is_same<TZ, double>::value) {
     if (invDiag) {
@@ -437,36 +436,52 @@ int pcg_dots(int64_t N, const double* invDiag, const double* r, TZ* z, const dou
   LPG_LAUNCH_CHECK("pcg_dots_kernel");
   return LPG_OK;
 }
-template int pcg_dots<double>(int64_t, const double*, const double*, double*, const double*, bool, bool, double*,
+template int pcg_dots<double>(int64_t, const double*, const double*, const double*, const double*, bool, bool, double*,
                               PcgScalars*, cudaStream_t);
-template int pcg_dots<float>(int64_t, const double*, const double*, float*, const double*, bool, bool, double*,
+template int pcg_dots<float>(int64_t, const double*, const double*, const float*, const double*, bool, bool, double*,
                              PcgScalars*, cudaStream_t);
 
-// p = z + beta p, and Ap = 0 for the operator to assemble into (zeroAp)
-template <typename TZ>
+// p = z + beta p, and Ap = 0 for the operator to assemble into (zeroAp); JACOBI: z = invDiag .* r
+template <typename TZ, bool JACOBI>
 __global__ void __launch_bounds__(256)
-pcg_direction_kernel(const int64_t N, const PcgScalars* __restrict__ sc, const TZ* __restrict__ z,
-                     double* __restrict__ p, double* __restrict__ Ap, const int zeroAp) {
+pcg_direction_kernel(const int64_t N, const PcgScalars* __restrict__ sc, const double* __restrict__ invDiag,
+                     const TZ* __restrict__ z, double* __restrict__ p, double* __restrict__ Ap, const int zeroAp) {
+  if (sc->stop) return;
   const double beta = sc->beta;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
-    p[n] = pcg_widen(z[n]) + (beta != 0.0 ? beta * p[n] : 0.0);
+    double zn;
+    if constexpr (JACOBI) zn = invDiag[n] * z[n];
+    else zn = pcg_widen(z[n]);
+    p[n] = zn + (beta != 0.0 ? beta * p[n] : 0.0);
     if (zeroAp) Ap[n] = 0.0;
   }
 }
 template <typename TZ>
-int pcg_direction(int64_t N, const PcgScalars* sc, const TZ* z, double* p, double* Ap, bool zeroAp, cudaStream_t s) {
+int pcg_direction(int64_t N, const PcgScalars* sc, const double* invDiag, const TZ* z, double* p, double* Ap,
+                  bool zeroAp, cudaStream_t s) {
   if (N <= 0) return LPG_OK;
-  pcg_direction_kernel<TZ><<<grid_for(N, 256, kStreamCap), 256, 0, s>>>(N, sc, z, p, Ap, zeroAp ? 1 : 0);
+  const unsigned grid = grid_for(N, 256, kStreamCap);
+  if constexpr (std::is_same<TZ, double>::value) {
+    if (invDiag) {
+      pcg_direction_kernel<TZ, true><<<grid, 256, 0, s>>>(N, sc, invDiag, z, p, Ap, zeroAp ? 1 : 0);
+      LPG_LAUNCH_CHECK("pcg_direction_kernel");
+      return LPG_OK;
+    }
+  }
+  pcg_direction_kernel<TZ, false><<<grid, 256, 0, s>>>(N, sc, nullptr, z, p, Ap, zeroAp ? 1 : 0);
   LPG_LAUNCH_CHECK("pcg_direction_kernel");
   return LPG_OK;
 }
-template int pcg_direction<double>(int64_t, const PcgScalars*, const double*, double*, double*, bool, cudaStream_t);
-template int pcg_direction<float>(int64_t, const PcgScalars*, const float*, double*, double*, bool, cudaStream_t);
+template int pcg_direction<double>(int64_t, const PcgScalars*, const double*, const double*, double*, double*, bool,
+                                   cudaStream_t);
+template int pcg_direction<float>(int64_t, const PcgScalars*, const double*, const float*, double*, double*, bool,
+                                  cudaStream_t);
 
 // p.Ap and alpha = r.z / p.Ap
 __global__ void __launch_bounds__(kRedThreads)
 pcg_curvature_kernel(const int64_t N, const double* __restrict__ p, const double* __restrict__ Ap,
                      double* __restrict__ partials, PcgScalars* __restrict__ sc) {
+  if (sc->stop) return;
   double a = 0;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x)
     a += p[n] * Ap[n];
@@ -477,6 +492,7 @@ pcg_curvature_kernel(const int64_t N, const double* __restrict__ p, const double
   if (threadIdx.x == 0) {
     sc->pAp = a;
     sc->alpha = sc->rz / a;
+    if (!(a > 0.0) || !isfinite(a)) sc->stop = 2;
   }
 }
 int pcg_curvature(int64_t N, const double* p, const double* Ap, double* partials, PcgScalars* sc, cudaStream_t s) {
@@ -485,29 +501,59 @@ int pcg_curvature(int64_t N, const double* p, const double* Ap, double* partials
   return LPG_OK;
 }
 
-// x += alpha p; r -= alpha Ap; r.r -- unless p.Ap is not positive and finite (a breakdown,
-// which leaves x and r)
+// x += alpha p; r -= alpha Ap; r.r; stops at r.r <= tol or not finite. JACOBI: the next
+// iteration's inner products and beta (z = invDiag .* r) in the same pass, which has r and Ap
+// in registers.
+template <bool JACOBI>
 __global__ void __launch_bounds__(kRedThreads)
-pcg_step_kernel(const int64_t N, const double* __restrict__ p, const double* __restrict__ Ap, double* __restrict__ x,
-                double* __restrict__ r, double* __restrict__ partials, PcgScalars* __restrict__ sc) {
-  if (!(sc->pAp > 0.0) || !isfinite(sc->pAp)) return;
+pcg_step_kernel(const int64_t N, const double* __restrict__ invDiag, const double* __restrict__ p,
+                const double* __restrict__ Ap, double* __restrict__ x, double* __restrict__ r, const double tol,
+                const int flexible, double* __restrict__ partials, PcgScalars* __restrict__ sc) {
+  if (sc->stop) return;
   const double alpha = sc->alpha;
-  double acc = 0;
+  double acc = 0, rz = 0, zAp = 0;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
+    const double An = Ap[n];
     x[n] += alpha * p[n];
-    const double rn = r[n] - alpha * Ap[n];
+    const double rn = r[n] - alpha * An;
     r[n] = rn;
     acc += rn * rn;
+    if constexpr (JACOBI) {
+      const double zn = invDiag[n] * rn;
+      rz += rn * zn;
+      if (flexible) zAp += zn * An;
+    }
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+  if constexpr (JACOBI) {
+    rz = block_sum(rz);
+    zAp = block_sum(zAp);
+    if (threadIdx.x == 0) {
+      partials[gridDim.x + blockIdx.x] = rz;
+      partials[2 * gridDim.x + blockIdx.x] = zAp;
+    }
+  }
   if (!last_block(&sc->done)) return;
   acc = sum_partials(partials);
-  if (threadIdx.x == 0) sc->rr = acc;
+  if constexpr (JACOBI) {
+    rz = sum_partials(partials + gridDim.x);
+    zAp = sum_partials(partials + 2 * gridDim.x);
+  }
+  if (threadIdx.x == 0) {
+    sc->rr = acc;
+    if (acc <= tol) sc->stop = 1;
+    else if (!isfinite(acc)) sc->stop = 3;
+    if constexpr (JACOBI) pcg_beta(sc, rz, zAp, flexible, 0);
+  }
 }
-int pcg_step(int64_t N, const double* p, const double* Ap, double* x, double* r, double* partials, PcgScalars* sc,
-             cudaStream_t s) {
-  pcg_step_kernel<<<red_blocks(N), kRedThreads, 0, s>>>(N, p, Ap, x, r, partials, sc);
+int pcg_step(int64_t N, const double* invDiag, const double* p, const double* Ap, double* x, double* r, double tol,
+             bool flexible, double* partials, PcgScalars* sc, cudaStream_t s) {
+  if (invDiag)
+    pcg_step_kernel<true><<<std::min(red_blocks(N), kReducePartials / 3), kRedThreads, 0, s>>>(
+        N, invDiag, p, Ap, x, r, tol, flexible, partials, sc);
+  else
+    pcg_step_kernel<false><<<red_blocks(N), kRedThreads, 0, s>>>(N, nullptr, p, Ap, x, r, tol, flexible, partials, sc);
   LPG_LAUNCH_CHECK("pcg_step_kernel");
   return LPG_OK;
 }
