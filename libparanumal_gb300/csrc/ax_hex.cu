@@ -30,19 +30,20 @@ constexpr int elems_per_block() {
   return (256 / (NQ * NQ)) > 0 ? (256 / (NQ * NQ)) : 1;
 }
 
-template <int NQ, typename T, typename G, int INMODE, int OUTMODE>
+// FP64 with direct contractions, one layer at a time: LPG_AX_FP64 = direct
+template <int NQ, int INMODE, int OUTMODE>
 __global__ void __launch_bounds__(NQ * NQ * elems_per_block<NQ>())
 ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
-              const int32_t* __restrict__ g2l, const G* __restrict__ ggeo, const int64_t geoStride,
-              const G* __restrict__ wJ, const int64_t wJStride, const T* __restrict__ Dg,
-              const T lambda, const T* __restrict__ lambdaE, const T* __restrict__ q,
-              T* __restrict__ out, const T outScale) {
+              const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
+              const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
+              const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
+              double* __restrict__ out) {
   constexpr int NP = NQ * NQ * NQ;
   constexpr int EPB = elems_per_block<NQ>();
-  __shared__ T s_D[NQ][NQ];
-  __shared__ T s_q[EPB][NQ][NQ];
-  __shared__ T s_Gqr[EPB][NQ][NQ];
-  __shared__ T s_Gqs[EPB][NQ][NQ];
+  __shared__ double s_D[NQ][NQ];
+  __shared__ double s_q[EPB][NQ][NQ];
+  __shared__ double s_Gqr[EPB][NQ][NQ];
+  __shared__ double s_Gqs[EPB][NQ][NQ];
 
   const int i = threadIdx.x, j = threadIdx.y, el = threadIdx.z;
   const int tid = i + NQ * (j + NQ * el);
@@ -53,7 +54,7 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
   if (active && elementList) e = elementList[e];
   if (!active) e = 0;
 
-  T r_q[NQ], r_Aq[NQ];
+  double r_q[NQ], r_Aq[NQ];
   int32_t r_id[NQ];
   const int64_t nodeBase = e * NP + j * NQ + i;
 #pragma unroll
@@ -62,41 +63,41 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
     if (INMODE == IN_GATHER) {
       const int32_t id = active ? __ldg(g2l + nodeBase + k * NQ * NQ) : -1;
       r_id[k] = id;
-      r_q[k] = (id >= 0) ? q[id] : T(0);
+      r_q[k] = (id >= 0) ? q[id] : 0.0;
     } else {
       r_id[k] = 0;
-      r_q[k] = active ? q[nodeBase + k * NQ * NQ] : T(0);
+      r_q[k] = active ? q[nodeBase + k * NQ * NQ] : 0.0;
     }
   }
   if (OUTMODE == OUT_ASSEMBLE && INMODE != IN_GATHER) {
 #pragma unroll
     for (int k = 0; k < NQ; ++k) r_id[k] = active ? __ldg(g2l + nodeBase + k * NQ * NQ) : -1;
   }
-  const T lam = (lambdaE && active) ? lambdaE[e] : lambda;
-  const G* gp = ggeo + e * geoStride + j * NQ + i;
-  const G* wp = wJ + e * wJStride + j * NQ + i;
+  const double lam = (lambdaE && active) ? lambdaE[e] : lambda;
+  const double* gp = ggeo + e * geoStride + j * NQ + i;
+  const double* wp = wJ + e * wJStride + j * NQ + i;
   __syncthreads();
 
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    T G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0, GwJ = 0;
+    double G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0, GwJ = 0;
     if (active) {
       const int off = k * NQ * NQ;
-      G00 = load_geo<T, G>(gp + 0 * NP + off);
-      G01 = load_geo<T, G>(gp + 1 * NP + off);
-      G02 = load_geo<T, G>(gp + 2 * NP + off);
-      G11 = load_geo<T, G>(gp + 3 * NP + off);
-      G12 = load_geo<T, G>(gp + 4 * NP + off);
-      G22 = load_geo<T, G>(gp + 5 * NP + off);
-      GwJ = load_geo<T, G>(wp + off);
+      G00 = __ldg(gp + 0 * NP + off);
+      G01 = __ldg(gp + 1 * NP + off);
+      G02 = __ldg(gp + 2 * NP + off);
+      G11 = __ldg(gp + 3 * NP + off);
+      G12 = __ldg(gp + 4 * NP + off);
+      G22 = __ldg(gp + 5 * NP + off);
+      GwJ = __ldg(wp + off);
     }
     s_q[el][j][i] = r_q[k];
-    T qt = 0;
+    double qt = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) qt += s_D[k][m] * r_q[m];
     __syncthreads();
 
-    T qr = 0, qs = 0;
+    double qr = 0, qs = 0;
 #pragma unroll
     for (int m = 0; m < NQ; ++m) {
       qr += s_D[i][m] * s_q[el][j][m];
@@ -104,8 +105,8 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
     }
     s_Gqs[el][j][i] = (G01 * qr + G11 * qs + G12 * qt);
     s_Gqr[el][j][i] = (G00 * qr + G01 * qs + G02 * qt);
-    const T Gqt = (G02 * qr + G12 * qs + G22 * qt);
-    T Auk = GwJ * lam * r_q[k];
+    const double Gqt = (G02 * qr + G12 * qs + G22 * qt);
+    double Auk = GwJ * lam * r_q[k];
     __syncthreads();
 
 #pragma unroll
@@ -122,17 +123,135 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
     if (OUTMODE == OUT_ASSEMBLE) {
-      // FP32: the scaled assembly of the fused residual; FP64 always adds A q itself
-      if constexpr (std::is_same<T, float>::value) {
-        if (r_id[k] >= 0) atomicAdd(out + r_id[k], outScale * r_Aq[k]);
-      } else {
-        if (r_id[k] >= 0) atomicAdd(out + r_id[k], r_Aq[k]);
-      }
+      if (r_id[k] >= 0) atomicAdd(out + r_id[k], r_Aq[k]);
     } else if (OUTMODE == OUT_LOCAL) {
       out[nodeBase + k * NQ * NQ] = r_Aq[k];
     } else {
       out[nodeBase + k * NQ * NQ] -= r_Aq[k];
     }
+  }
+}
+
+// ---------------------------------------------------------------- FP32 line variant
+// FP32 vectors at the degrees whose element rows are not 16-byte multiples (odd Nq), which the
+// staged kernel cannot copy. One thread holds one line at a time: its t-pencil in registers,
+// its r- and s-line through two line-contiguous copies of the element in shared memory,
+// contracted in place. An element needs 4 barriers instead of 3 a layer, and the factors of
+// all its layers are loaded independently of them.
+template <int NQ>
+struct LineLayout {
+  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ;
+  // Odd row pitch, and the copies of a CTA's elements one after the other: line l of element
+  // el starts at P (l + NL el), without bank conflicts across the warps' element boundaries.
+  static constexpr int P = NQ | 1, PL = P * NQ, ES = P * NL;
+  static constexpr int EPB = 256 / NL, NT = NL * EPB;
+  static constexpr int RD = (NQ + 3) & ~3;        // row of D in shared memory, 16-byte multiple
+  static constexpr int MINB = NQ <= 3 ? 5 : 4;    // resident CTAs per SM to compile for, best of 2 to 5
+};
+
+// y = M x with the rows of M read from shared memory (16-byte aligned, RD entries)
+template <int NQ>
+__device__ __forceinline__ void line_product(const float* __restrict__ M, const float (&x)[NQ], float (&y)[NQ]) {
+  constexpr int RD = LineLayout<NQ>::RD;
+#pragma unroll
+  for (int t = 0; t < NQ; ++t) {
+    float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+    for (int m = 0; m < NQ; m += 4) {
+      const float4 c = *reinterpret_cast<const float4*>(M + t * RD + m);
+      r0 += c.x * x[m];
+      if (m + 1 < NQ) r1 += c.y * x[m + 1 < NQ ? m + 1 : 0];
+      if (m + 2 < NQ) r0 += c.z * x[m + 2 < NQ ? m + 2 : 0];
+      if (m + 3 < NQ) r1 += c.w * x[m + 3 < NQ ? m + 3 : 0];
+    }
+    y[t] = r0 + r1;
+  }
+}
+
+template <int NQ, typename G, bool MASS>
+__global__ void __launch_bounds__(LineLayout<NQ>::NT, LineLayout<NQ>::MINB)
+ax_hex_line_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
+                   const int32_t* __restrict__ g2l, const G* __restrict__ ggeo, const int64_t geoStride,
+                   const G* __restrict__ wJ, const int64_t wJStride, const float* __restrict__ Dg, const float lambda,
+                   const float* __restrict__ lambdaE, const float* __restrict__ q, float* __restrict__ out,
+                   const float outScale) {
+  using L = LineLayout<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, P = L::P, PL = L::PL, EPB = L::EPB;
+  constexpr int UD = NQ <= 6 ? 2 : 1;
+  __shared__ __align__(16) float s_D[2][NQ * L::RD];   // D, D^T
+  __shared__ float s_v[2][EPB * L::ES];
+  const int tid = threadIdx.x, el = tid / NL, l = tid % NL, a = l % NQ, b = l / NQ;
+  float* const line = &s_v[0][P * tid];                           // r-line l (s: EPB ES further)
+  float* const nr = &s_v[0][el * L::ES + b * P + a];              // node (a, b, k): k PL further
+  float* const ns = &s_v[1][el * L::ES + a * P + b];
+  int64_t e = (int64_t)blockIdx.x * EPB + el;
+  const bool active = e < Nelements;
+  if (active && elementList) e = elementList[e];
+  if (!active) e = 0;
+  const int64_t nodeBase = e * NP + l;
+  // one thread asks for the factors of the CTA's run of elements in L2 (whole 16-byte units
+  // inside the run: the rows are not aligned)
+  if (tid == 0 && !elementList && geoStride <= 7 * NP) {
+    const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
+    const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
+    const uintptr_t hi = (uintptr_t)(ggeo + (e + n) * geoStride) & ~(uintptr_t)15;
+    if (hi > lo) prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
+  }
+  int32_t id[NQ];
+  float v0[NQ], ut[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+  for (int t = tid; t < NL; t += L::NT) {
+    const float d = Dg[t];
+    s_D[0][t / NQ * L::RD + t % NQ] = d;
+    s_D[1][t % NQ * L::RD + t / NQ] = d;
+  }
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) v0[k] = id[k] >= 0 ? q[id[k]] : 0.f;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) nr[k * PL] = ns[k * PL] = v0[k];
+  __syncthreads();
+  auto lines = [&](const float* M) {
+#pragma unroll UD
+    for (int d = 0; d < 2; ++d) {
+      if constexpr (UD == 1) asm volatile("" ::: "memory");   // keeps D out of registers
+      float* const o = line + d * EPB * L::ES;
+      float x[NQ], y[NQ];
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) x[m] = o[m];
+      line_product<NQ>(M, x, y);
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) o[m] = y[m];
+    }
+    if constexpr (UD == 1) asm volatile("" ::: "memory");
+  };
+  lines(s_D[0]);
+  line_product<NQ>(s_D[0], v0, ut);
+  __syncthreads();
+  const G* gp = ggeo + e * geoStride + l;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    float g[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) g[c] = active ? load_geo<float, G>(gp + c * NP + k * NL) : 0.f;
+    const float qr = nr[k * PL], qs = ns[k * PL], qt = ut[k];
+    nr[k * PL] = g[0] * qr + g[1] * qs + g[2] * qt;
+    ns[k * PL] = g[1] * qr + g[3] * qs + g[4] * qt;
+    ut[k] = g[2] * qr + g[4] * qs + g[5] * qt;
+  }
+  __syncthreads();
+  lines(s_D[1]);
+  float At[NQ];
+  line_product<NQ>(s_D[1], ut, At);
+  __syncthreads();
+  if (!active) return;
+  const float lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.f;
+  const G* wp = wJ + e * wJStride + l;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    float r = At[k] + nr[k * PL] + ns[k * PL];
+    if constexpr (MASS) r += load_geo<float, G>(wp + k * NL) * lam * v0[k];
+    if (id[k] >= 0) atomicAdd(out + id[k], outScale * r);
   }
 }
 
@@ -1130,51 +1249,76 @@ static int launch_fx(const AxArgs<double, double>& a, cudaStream_t s) {
   return LPG_OK;
 }
 
-template <int NQ, typename T, typename G, int INMODE, int OUTMODE>
-static int launch_ax(const AxArgs<T, G>& a, cudaStream_t s) {
-  if constexpr (std::is_same<T, float>::value && INMODE == IN_GATHER && OUTMODE == OUT_ASSEMBLE) {
-    if (staged_ok<NQ, T, G>(a)) {
+template <int NQ, typename G>
+static int launch_line(const AxArgs<float, G>& a, cudaStream_t s) {
+  using L = LineLayout<NQ>;
+  const int64_t blocks = (a.Nelements + L::EPB - 1) / L::EPB;
+  if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
+  auto go = [&](auto kern) {
+    kern<<<(unsigned)blocks, L::NT, 0, s>>>(a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride,
+                                            a.D, a.lambda, a.lambdaE, a.q, a.out, a.outScale);
+  };
+  if (a.lambda == 0 && !a.lambdaE) go(ax_hex_line_kernel<NQ, G, false>);
+  else go(ax_hex_line_kernel<NQ, G, true>);
+  LPG_LAUNCH_CHECK("ax_hex_line_kernel");
+  return LPG_OK;
+}
+
+// FP32 vectors: the staged kernel at Nq = 8, and at Nq = 4 with FP32 geometry, on 16-byte
+// aligned rows; the line kernel elsewhere. Measured, staged against line, FP32 geometry:
+// 40^3, N = 7 251 against 300 us; 60^3, N = 3 109 against 112; 40^3, N = 5 148 against 141;
+// 100^3, N = 1 222 against 68; BF16 geometry: 60^3, N = 3 107 against 101; 40^3, N = 5 123
+// against 119. The one-layer-at-a-time kernel that served the odd Nq before the line kernel:
+// 48^3, N = 4 151 against 120 us; 30^3, N = 6 130 against 99; 24^3, N = 8 195 against 113;
+// 80^3, N = 2 125 against 118.
+template <int NQ, int INMODE, int OUTMODE, typename G>
+static int launch_ax(const AxArgs<float, G>& a, cudaStream_t s) {
+  if constexpr (INMODE == IN_GATHER && OUTMODE == OUT_ASSEMBLE) {
+    if (a.Nelements <= 0) return LPG_OK;
+    constexpr bool F32 = std::is_same<G, float>::value;
+    if constexpr (NQ == 8 || (NQ == 4 && F32)) {
       // LPG_AX_STAGED = off | EPBxSTAGES (2x2, 2x3, 4x2, 4x3) | 2x2pf: tuning override
       const int v = staged_variant();
-      if (v == 0) { /* fall through to the unstaged kernel */ }
-      else if (v == 22) return launch_staged<NQ, T, G, 2, 2>(a, s);
-      else if (v == 23) return launch_staged<NQ, T, G, 2, 3>(a, s);
-      else if (v == 43) return launch_staged<NQ, T, G, 4, 3>(a, s);
-      else if (v == 42) return launch_staged<NQ, T, G, 4, 2>(a, s);
-      else if (v == 122) return launch_staged<NQ, T, G, 2, 2, true>(a, s);
-      // measured best at N=7: FP32 geometry with the next group's q gathered half-way
-      // through the current group (0.997 vs 1.112 ms at 64^3); BF16 geometry without it
-      // (lambda = 0 without a lambda field: the instantiation without the mass term and wJ copy)
-      const bool noMass = (a.lambda == 0 && !a.lambdaE);
-      if constexpr (std::is_same<G, float>::value)
-        return noMass ? launch_staged<NQ, T, G, 2, 2, true, false>(a, s) : launch_staged<NQ, T, G, 2, 2, true>(a, s);
-      else
-        return noMass ? launch_staged<NQ, T, G, 2, 2, false, false>(a, s) : launch_staged<NQ, T, G, 2, 2>(a, s);
+      if (v != 0 && staged_ok<NQ, float, G>(a)) {
+        if (v == 22) return launch_staged<NQ, float, G, 2, 2>(a, s);
+        if (v == 23) return launch_staged<NQ, float, G, 2, 3>(a, s);
+        if (v == 43) return launch_staged<NQ, float, G, 4, 3>(a, s);
+        if (v == 42) return launch_staged<NQ, float, G, 4, 2>(a, s);
+        if (v == 122) return launch_staged<NQ, float, G, 2, 2, true>(a, s);
+        // measured best at N=7: FP32 geometry with the next group's q gathered half-way
+        // through the current group (0.997 vs 1.112 ms at 64^3); BF16 geometry without it
+        // (lambda = 0 without a lambda field: the instantiation without the mass term and wJ copy)
+        const bool noMass = (a.lambda == 0 && !a.lambdaE);
+        return noMass ? launch_staged<NQ, float, G, 2, 2, F32, false>(a, s) : launch_staged<NQ, float, G, 2, 2, F32>(a, s);
+      }
     }
+    return launch_line<NQ, G>(a, s);
+  } else {
+    return set_error(LPG_ERR_UNSUPPORTED, "ax: FP32 vectors are provided for the assembled operator only");
+  }
+}
+
+template <int NQ, int INMODE, int OUTMODE>
+static int launch_ax(const AxArgs<double, double>& a, cudaStream_t s) {
+  if (a.Nelements <= 0) return LPG_OK;
+  if (!fp64_direct_override()) {
+    auto go = [&](auto eo) {
+      constexpr bool EO = decltype(eo)::value;
+      if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, false, false>(a, s);
+      if (a.lambda == 1.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, true, true>(a, s);
+      return launch_fx<NQ, EO, INMODE, OUTMODE, true, false>(a, s);
+    };
+    // half the products where D is known to be mirrored (28^3, N = 5: 133 against 156 us;
+    // 20^3, N = 8: 201 against 253 us)
+    if constexpr (NQ != 4 && NQ != 8 && OUTMODE == OUT_ASSEMBLE)
+      if (a.mirrored) return go(std::true_type{});
+    return go(std::integral_constant<bool, NQ == 4 || NQ == 8>{});
   }
   constexpr int EPB = elems_per_block<NQ>();
-  if (a.Nelements <= 0) return LPG_OK;
   const int64_t blocks = (a.Nelements + EPB - 1) / EPB;
   if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
-  dim3 block(NQ, NQ, EPB);
-  if constexpr (std::is_same<T, double>::value) {
-    if (!fp64_direct_override()) {
-      auto go = [&](auto eo) {
-        constexpr bool EO = decltype(eo)::value;
-        if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, false, false>(a, s);
-        if (a.lambda == 1.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, true, true>(a, s);
-        return launch_fx<NQ, EO, INMODE, OUTMODE, true, false>(a, s);
-      };
-      // half the products where D is known to be mirrored (28^3, N = 5: 133 against 156 us;
-      // 20^3, N = 8: 201 against 253 us)
-      if constexpr (NQ != 4 && NQ != 8 && OUTMODE == OUT_ASSEMBLE)
-        if (a.mirrored) return go(std::true_type{});
-      return go(std::integral_constant<bool, NQ == 4 || NQ == 8>{});
-    }
-  }
-  ax_hex_kernel<NQ, T, G, INMODE, OUTMODE><<<(unsigned)blocks, block, 0, s>>>(
-      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda,
-      a.lambdaE, a.q, a.out, a.outScale);
+  ax_hex_kernel<NQ, INMODE, OUTMODE><<<(unsigned)blocks, dim3(NQ, NQ, EPB), 0, s>>>(
+      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out);
   LPG_LAUNCH_CHECK("ax_hex_kernel");
   return LPG_OK;
 }
@@ -1182,14 +1326,14 @@ static int launch_ax(const AxArgs<T, G>& a, cudaStream_t s) {
 template <typename T, typename G, int INMODE, int OUTMODE>
 static int dispatch_ax(const AxArgs<T, G>& a, cudaStream_t s) {
   switch (a.N) {
-    case 1: return launch_ax<2, T, G, INMODE, OUTMODE>(a, s);
-    case 2: return launch_ax<3, T, G, INMODE, OUTMODE>(a, s);
-    case 3: return launch_ax<4, T, G, INMODE, OUTMODE>(a, s);
-    case 4: return launch_ax<5, T, G, INMODE, OUTMODE>(a, s);
-    case 5: return launch_ax<6, T, G, INMODE, OUTMODE>(a, s);
-    case 6: return launch_ax<7, T, G, INMODE, OUTMODE>(a, s);
-    case 7: return launch_ax<8, T, G, INMODE, OUTMODE>(a, s);
-    case 8: return launch_ax<9, T, G, INMODE, OUTMODE>(a, s);
+    case 1: return launch_ax<2, INMODE, OUTMODE>(a, s);
+    case 2: return launch_ax<3, INMODE, OUTMODE>(a, s);
+    case 3: return launch_ax<4, INMODE, OUTMODE>(a, s);
+    case 4: return launch_ax<5, INMODE, OUTMODE>(a, s);
+    case 5: return launch_ax<6, INMODE, OUTMODE>(a, s);
+    case 6: return launch_ax<7, INMODE, OUTMODE>(a, s);
+    case 7: return launch_ax<8, INMODE, OUTMODE>(a, s);
+    case 8: return launch_ax<9, INMODE, OUTMODE>(a, s);
     default: return set_error(LPG_ERR_UNSUPPORTED, "ax: polynomial degree must be 1..8");
   }
 }
@@ -1227,7 +1371,7 @@ static int wave_elements(bool dw, bool mass) {
     else
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_dw_kernel<NQ>, NQ * NQ * epb, 0);
   } else if (fp64_direct_override()) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_kernel<NQ, double, double, IN_GATHER, OUT_ASSEMBLE>,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ax_hex_kernel<NQ, IN_GATHER, OUT_ASSEMBLE>,
                                                       NQ * NQ * epb, 0);
   } else {
     KernelConfig cfg;
