@@ -37,7 +37,7 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
               const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
               const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
               const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
-              double* __restrict__ out) {
+              double* __restrict__ out, const double outScale) {
   constexpr int NP = NQ * NQ * NQ;
   constexpr int EPB = elems_per_block<NQ>();
   __shared__ double s_D[NQ][NQ];
@@ -123,7 +123,7 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
     if (OUTMODE == OUT_ASSEMBLE) {
-      if (r_id[k] >= 0) atomicAdd(out + r_id[k], r_Aq[k]);
+      if (r_id[k] >= 0) atomicAdd(out + r_id[k], outScale * r_Aq[k]);
     } else if (OUTMODE == OUT_LOCAL) {
       out[nodeBase + k * NQ * NQ] = r_Aq[k];
     } else {
@@ -524,20 +524,32 @@ ax_hex_staged_kernel(const int64_t Nelements, const int32_t* __restrict__ elemen
 // lines 1.37 against 1.37 ms.
 // MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
 // UNIT: lambda == 1 without a lambda field, the mass term is wJ q
-template <int NQ, bool EO, int INMODE, int OUTMODE, bool MASS, bool UNIT>
-__global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB)
+// W = 3: three threads a line position, each with one direction of the derivatives and a third
+// of the layers, for problems too small to fill the GPU otherwise
+template <int NQ, int W>
+struct FxThreads {
+  using L = FxLayout<NQ>;
+  static constexpr int EPB = W == 1 ? L::EPB : (L::NL * W >= 96 ? 1 : 96 / (L::NL * W));
+  static constexpr int NT = L::NL * W * EPB, MINB = W == 1 ? L::MINB : 1;
+};
+
+template <int NQ, bool EO, int W, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+__global__ void __launch_bounds__(FxThreads<NQ, W>::NT, FxThreads<NQ, W>::MINB)
 ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
                  const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
                  const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
                  const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
-                 double* __restrict__ out) {
+                 double* __restrict__ out, const int outSign) {
   using L = FxLayout<NQ, EO>;
-  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB;
+  constexpr int NP = L::NP, NL = L::NL, EPB = FxThreads<NQ, W>::EPB, KN = (NQ + W - 1) / W;
   extern __shared__ __align__(16) unsigned char fx_smem[];
   __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::RS];   // D, D^T
   __shared__ int s_e[2][L::ROWS];                   // biased exponents of their rows
   __shared__ int s_x[EPB][3][NL];                   // exponents of the transposed lines, -1: FP64 values
-  const int tid = threadIdx.x, el = tid / NL, l = tid % NL;
+  const int tid = threadIdx.x, el = tid / (NL * W), l = tid % NL, w = W == 1 ? 0 : tid / NL % W;
+  // this thread's layers w, w + W, ... (layer() is a constant for W = 1)
+  auto layer = [&](int i) { return W == 1 ? i : w + W * i; };
+  auto inside = [&](int i) { return W == 1 || NQ % W == 0 || w + W * i < NQ; };
   const FxElement<NQ> E(reinterpret_cast<double*>(fx_smem) + el * FxElement<NQ>::DOUBLES, l);
 
   int64_t e = (int64_t)blockIdx.x * EPB + el;
@@ -549,7 +561,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
   // else for the CTA's whole run of elements (one request per lane would be issued one by one:
   // 90^3, N = 1: 138 against 121 us)
   if constexpr (EPB <= 2) {
-    if (active && l == 0) {
+    if (active && l == 0 && w == 0) {
       prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(double));
       if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(double));
     }
@@ -560,30 +572,38 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
   }
   bool plain;
   {
-    double v[NQ];
+    double v[KN];
     if constexpr (INMODE == IN_GATHER) {
-      int32_t id[NQ];
+      int32_t id[KN];
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+      for (int i = 0; i < KN; ++i) id[i] = active && inside(i) ? __ldg(g2l + nodeBase + layer(i) * NL) : -1;
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) v[k] = id[k] >= 0 ? q[id[k]] : 0.0;
+      for (int i = 0; i < KN; ++i) v[i] = id[i] >= 0 ? q[id[i]] : 0.0;
     } else {
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) v[k] = active ? q[nodeBase + k * NL] : 0.0;
+      for (int i = 0; i < KN; ++i) v[i] = active && inside(i) ? q[nodeBase + layer(i) * NL] : 0.0;
     }
-    plain = fx_tables<NQ, EO>(Dg, tid, s_tab, s_e);   // while the gather is in flight
+    plain = fx_tables<NQ, EO>(Dg, tid, FxThreads<NQ, W>::NT, s_tab, s_e);   // while the gather is in flight
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) E.r(E.a, E.b, k) = E.s(E.a, E.b, k) = E.t(E.a, E.b, k) = v[k];
+    for (int i = 0; i < KN; ++i)
+      if (inside(i)) E.r(E.a, E.b, layer(i)) = E.s(E.a, E.b, layer(i)) = E.t(E.a, E.b, layer(i)) = v[i];
   }
   plain = __syncthreads_or(plain);
-  fx_forward<NQ, EO>(E, s_tab[0], s_e[0], plain, Dg);
-  ax_fx_sync<NQ, EPB>(el);
+  auto sync = [&](bool any) -> bool {
+    if constexpr (W == 1) return ax_fx_sync<NQ, EPB>(el, any);
+    else return __syncthreads_or(any);
+  };
+  const int d0 = W == 1 ? 0 : w, d1 = W == 1 ? 3 : w + 1;
+  fx_forward<NQ, EO>(E, s_tab[0], s_e[0], plain, Dg, d0, d1);
+  sync(false);
 
   // G . grad q
   {
     const double* gp = ggeo + e * geoStride + l;
 #pragma unroll 4
-    for (int k = 0; k < NQ; ++k) {
+    for (int i = 0; i < KN; ++i) {
+      if (!inside(i)) break;
+      const int k = layer(i);
       double G00 = 0, G01 = 0, G02 = 0, G11 = 0, G12 = 0, G22 = 0;
       if (active) {
         G00 = gp[0 * NP + k * NL]; G01 = gp[1 * NP + k * NL]; G02 = gp[2 * NP + k * NL];
@@ -596,31 +616,34 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
       ut = G02 * qr + G12 * qs + G22 * qt;
     }
   }
-  ax_fx_sync<NQ, EPB>(el);
+  sync(false);
 
-  bool fp = fx_transposed<NQ, EO>(E, s_tab[1], plain, Dg, s_x[el]);
-  int32_t id[NQ];   // in flight over the barrier
+  bool fp = fx_transposed<NQ, EO>(E, s_tab[1], plain, Dg, s_x[el], d0, d1);
+  int32_t id[KN];   // in flight over the barrier
   if constexpr (OUTMODE == OUT_ASSEMBLE || (MASS && INMODE == IN_GATHER)) {
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+    for (int i = 0; i < KN; ++i) id[i] = active && inside(i) ? __ldg(g2l + nodeBase + layer(i) * NL) : -1;
   }
-  fp = ax_fx_sync<NQ, EPB>(el, fp);
+  fp = sync(fp);
 
   if (!active) return;
   const double lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.0;
   const double* wp = wJ + e * wJStride + l;
   const int er = s_e[1][fx_row<NQ, EO>(E.a)], es = s_e[1][fx_row<NQ, EO>(E.b)];
 #pragma unroll
-  for (int k = 0; k < NQ; ++k) {
+  for (int i = 0; i < KN; ++i) {
+    if (!inside(i)) break;
+    const int k = layer(i);
     double r = fx_node_sum<NQ, EO>(E, k, s_x[el], s_e[1], er, es, fp);
     if constexpr (MASS) {
       double v = 0.0;
-      if constexpr (INMODE == IN_GATHER) v = id[k] >= 0 ? q[id[k]] : 0.0;
+      if constexpr (INMODE == IN_GATHER) v = id[i] >= 0 ? q[id[i]] : 0.0;
       else v = q[nodeBase + k * NL];
       r = fma(UNIT ? wp[k * NL] : wp[k * NL] * lam, v, r);
     }
     if constexpr (OUTMODE == OUT_ASSEMBLE) {
-      if (id[k] >= 0) atomicAdd(out + id[k], r);
+      // outSign: the sign bit for out -= A q
+      if (id[i] >= 0) atomicAdd(out + id[i], __hiloint2double(__double2hiint(r) ^ outSign, __double2loint(r)));
     } else if constexpr (OUTMODE == OUT_LOCAL) {
       out[nodeBase + k * NL] = r;
     } else {
@@ -1218,11 +1241,11 @@ static bool fp64_direct_override() {
   return direct;
 }
 
-template <int NQ, bool EO, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+template <int NQ, bool EO, int W, int INMODE, int OUTMODE, bool MASS, bool UNIT>
 static int fx_config(KernelConfig* cfg, size_t* smem) {
-  using L = FxLayout<NQ>;
+  using L = FxThreads<NQ, W>;
   static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in, occupancy
-  auto kern = ax_hex_fx_kernel<NQ, EO, INMODE, OUTMODE, MASS, UNIT>;
+  auto kern = ax_hex_fx_kernel<NQ, EO, W, INMODE, OUTMODE, MASS, UNIT>;
   const size_t bytes = sizeof(double) * FxElement<NQ>::DOUBLES * L::EPB;
   *smem = bytes;
   return perDevice.get(
@@ -1234,17 +1257,18 @@ static int fx_config(KernelConfig* cfg, size_t* smem) {
       cfg);
 }
 
-template <int NQ, bool EO, int INMODE, int OUTMODE, bool MASS, bool UNIT>
+template <int NQ, bool EO, int W, int INMODE, int OUTMODE, bool MASS, bool UNIT>
 static int launch_fx(const AxArgs<double, double>& a, cudaStream_t s) {
-  using L = FxLayout<NQ>;
+  using L = FxThreads<NQ, W>;
   KernelConfig cfg;
   size_t smem;
-  const int rc = fx_config<NQ, EO, INMODE, OUTMODE, MASS, UNIT>(&cfg, &smem);
+  const int rc = fx_config<NQ, EO, W, INMODE, OUTMODE, MASS, UNIT>(&cfg, &smem);
   if (rc) return rc;
   const int64_t blocks = (a.Nelements + L::EPB - 1) / L::EPB;
   if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
-  ax_hex_fx_kernel<NQ, EO, INMODE, OUTMODE, MASS, UNIT><<<(unsigned)blocks, L::NT, smem, s>>>(
-      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out);
+  ax_hex_fx_kernel<NQ, EO, W, INMODE, OUTMODE, MASS, UNIT><<<(unsigned)blocks, L::NT, smem, s>>>(
+      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out,
+      a.outScale < 0 ? (int)0x80000000 : 0);
   LPG_LAUNCH_CHECK("ax_hex_fx_kernel");
   return LPG_OK;
 }
@@ -1304,9 +1328,24 @@ static int launch_ax(const AxArgs<double, double>& a, cudaStream_t s) {
   if (!fp64_direct_override()) {
     auto go = [&](auto eo) {
       constexpr bool EO = decltype(eo)::value;
-      if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, false, false>(a, s);
-      if (a.lambda == 1.0 && !a.lambdaE) return launch_fx<NQ, EO, INMODE, OUTMODE, true, true>(a, s);
-      return launch_fx<NQ, EO, INMODE, OUTMODE, true, false>(a, s);
+      // Below 448 line positions an SM the GPU is not full and the time is that of one element:
+      // three threads a position, each with one direction. Measured, one against three threads:
+      // N = 7, 4^3 18.6 against 12.5 us, 10^3 29.1 against 25.0, 12^3 35.2 against 35.4, 16^3 73
+      // against 79; N = 5, 8^3 17.6 against 13.6, 16^3 35.2 against 35.0; N = 3, 14^3 16.9
+      // against 14.8, 20^3 23.0 against 24.9.
+      if constexpr (OUTMODE == OUT_ASSEMBLE && EO) {
+        KernelConfig cfg;
+        size_t smem;
+        const int rc = fx_config<NQ, EO, 1, INMODE, OUTMODE, true, false>(&cfg, &smem);
+        if (rc) return rc;
+        if (a.Nelements * (NQ * NQ) <= (int64_t)448 * cfg.numSMs) {
+          if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, EO, 3, INMODE, OUTMODE, false, false>(a, s);
+          return launch_fx<NQ, EO, 3, INMODE, OUTMODE, true, false>(a, s);
+        }
+      }
+      if (a.lambda == 0.0 && !a.lambdaE) return launch_fx<NQ, EO, 1, INMODE, OUTMODE, false, false>(a, s);
+      if (a.lambda == 1.0 && !a.lambdaE) return launch_fx<NQ, EO, 1, INMODE, OUTMODE, true, true>(a, s);
+      return launch_fx<NQ, EO, 1, INMODE, OUTMODE, true, false>(a, s);
     };
     // half the products where D is known to be mirrored (28^3, N = 5: 133 against 156 us;
     // 20^3, N = 8: 201 against 253 us)
@@ -1318,7 +1357,8 @@ static int launch_ax(const AxArgs<double, double>& a, cudaStream_t s) {
   const int64_t blocks = (a.Nelements + EPB - 1) / EPB;
   if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
   ax_hex_kernel<NQ, INMODE, OUTMODE><<<(unsigned)blocks, dim3(NQ, NQ, EPB), 0, s>>>(
-      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out);
+      a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out,
+      a.outScale);
   LPG_LAUNCH_CHECK("ax_hex_kernel");
   return LPG_OK;
 }
@@ -1340,8 +1380,8 @@ static int dispatch_ax(const AxArgs<T, G>& a, cudaStream_t s) {
 
 template <typename T, typename G>
 int ax_hex(const AxArgs<T, G>& a, AxMode mode, cudaStream_t s) {
-  if (!std::is_same<T, float>::value && a.outScale != T(1))
-    return set_error(LPG_ERR_UNSUPPORTED, "ax: a scaled assembly is provided for FP32 only");
+  if (std::is_same<T, double>::value && a.outScale != T(1) && a.outScale != T(-1))
+    return set_error(LPG_ERR_UNSUPPORTED, "ax: FP64 assembles A q or -A q");
   switch (mode) {
     case AxMode::Assemble: {
       if (a.Nglobal > 0) LPG_CUDA_TRY(cudaMemsetAsync(a.out, 0, sizeof(T) * a.Nglobal, s));
@@ -1376,8 +1416,8 @@ static int wave_elements(bool dw, bool mass) {
   } else {
     KernelConfig cfg;
     size_t smem;
-    const int rc = mass ? fx_config<NQ, true, IN_GATHER, OUT_ASSEMBLE, true, false>(&cfg, &smem)
-                        : fx_config<NQ, true, IN_GATHER, OUT_ASSEMBLE, false, false>(&cfg, &smem);
+    const int rc = mass ? fx_config<NQ, true, 1, IN_GATHER, OUT_ASSEMBLE, true, false>(&cfg, &smem)
+                        : fx_config<NQ, true, 1, IN_GATHER, OUT_ASSEMBLE, false, false>(&cfg, &smem);
     per = rc ? 0 : cfg.ctasPerSM;
     epb = FxLayout<NQ>::EPB;
   }

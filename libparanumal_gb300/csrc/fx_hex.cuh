@@ -194,16 +194,16 @@ struct FxElement {
   __device__ __forceinline__ double& t(int i, int j, int k) const { return S[2 * L::PL * NQ + j * L::PL + i * L::P + k]; }
 };
 
-// tables of D and D^T with the exponents of their rows, by the NT threads of a CTA; true where
+// tables of D and D^T with the exponents of their rows, by the threads of a CTA; true where
 // an entry beyond 2^63 leaves every line to FP64
 template <int NQ, bool EO>
-__device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid,
+__device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid, const int threads,
                                           fx_half (&tab)[2][FxLayout<NQ, EO>::ROWS * FxLayout<NQ, EO>::RS],
                                           int (&ex)[2][FxLayout<NQ, EO>::ROWS]) {
   using L = FxLayout<NQ, EO>;
   constexpr int TAB = L::ROWS * NQ;
   bool plain = false;
-  for (int w = tid; w < 2 * TAB; w += L::NT) {
+  for (int w = tid; w < 2 * TAB; w += threads) {
     const int tr = w / TAB, t = (w % TAB) / NQ, c = w % NQ;
     unsigned key = 0;
 #pragma unroll
@@ -216,13 +216,13 @@ __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const i
   return plain;
 }
 
-// the copies of q become D_r q, D_s q, D_t q
+// the copies of q become D_r q, D_s q, D_t q (directions d0 to d1 - 1 by this thread)
 template <int NQ, bool EO>
 __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half* tab, const int* ex, const bool plain,
-                                           const double* __restrict__ Dg) {
+                                           const double* __restrict__ Dg, const int d0 = 0, const int d1 = 3) {
   using L = FxLayout<NQ, EO>;
 #pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
+  for (int d = d0; d < d1; ++d) {
     double* const o = E.line(d);
     double v[NQ];
     unsigned key = 0;
@@ -256,10 +256,11 @@ __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half
 // exponents of the lines in x, -1 for a line kept as FP64 values; true if this thread kept one
 template <int NQ, bool EO>
 __device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_half* tab, const bool plain,
-                                              const double* __restrict__ Dg, int (&x)[3][FxLayout<NQ>::NL]) {
+                                              const double* __restrict__ Dg, int (&x)[3][FxLayout<NQ>::NL],
+                                              const int d0 = 0, const int d1 = 3) {
   bool fp = false;
 #pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
+  for (int d = d0; d < d1; ++d) {
     double* const o = E.line(d);
     double v[NQ];
     unsigned key = 0;
