@@ -528,13 +528,27 @@ int Elliptic::Operator(const double* q, double* Aq, cudaStream_t s, bool zeroed)
     return ipdg_operator(a, s);
   }
   if (opDW) return OperatorDW(q, Aq, s, zeroed);
+  AxArgs<double, double> a = ax_args();
+  a.q = q; a.out = Aq;
+  return ax_hex<double, double>(a, zeroed ? AxMode::AccumulateAssembled : AxMode::Assemble, s);
+}
+
+AxArgs<double, double> Elliptic::ax_args() const {
   AxArgs<double, double> a;
   const int64_t Np = mesh.Np;
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geo.p; a.geoStride = 7 * Np; a.wJ = mesh.geo.p + 6 * Np; a.wJStride = 7 * Np;
   a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
-  a.q = q; a.out = Aq; a.Nglobal = Nglobal;
-  return ax_hex<double, double>(a, zeroed ? AxMode::AccumulateAssembled : AxMode::Assemble, s);
+  a.Nglobal = Nglobal;
+  return a;
+}
+
+int Elliptic::OperatorSubtract(const double* q, double* u, cudaStream_t s) {
+  if (!can_subtract()) return set_error(LPG_ERR_UNSUPPORTED, "subtracting operator: C0 in native FP64 only");
+  ++nOps;
+  AxArgs<double, double> a = ax_args();
+  a.q = q; a.out = u; a.outScale = -1.0;
+  return ax_hex<double, double>(a, AxMode::AccumulateAssembled, s);
 }
 
 int Elliptic::OperatorF32(const float* q, float* Aq, Prec prec, cudaStream_t s, float accumulate) {

@@ -523,11 +523,15 @@ int MultiGrid::op<float>(Elliptic* el, const float* q, float* Aq, cudaStream_t s
   return el->OperatorF32(q, Aq, opt.prec, s);
 }
 
-// RES = RHS - A X. The C0 FP32 operator assembles straight into a copy of RHS with the
+// RES = RHS - A X. The C0 operators (but the double-word one) assemble straight into a copy of RHS with the
 // sign of the contributions flipped (one copy instead of a memset and an axpy pass).
 template <>
 int MultiGrid::residual<double>(Elliptic* el, const double* RHS, const double* X, double* RES, cudaStream_t s) {
   int rc;
+  if (el->can_subtract()) {
+    LPG_CUDA_TRY(cudaMemcpyAsync(RES, RHS, sizeof(double) * el->Nglobal, cudaMemcpyDeviceToDevice, s));
+    return el->OperatorSubtract(X, RES, s);
+  }
   if ((rc = el->Operator(X, RES, s))) return rc;
   return axpy<double>(el->Nglobal, 1.0, RHS, -1.0, RES, s);
 }
@@ -543,7 +547,7 @@ int MultiGrid::residual<float>(Elliptic* el, const float* RHS, const float* X, f
 }
 
 // ---------------------------------------------------------------- p-level smoothing
-// LPG_CHEB=unfused (a tuning override): the FP32 Chebyshev steps with a separate A d vector
+// LPG_CHEB=unfused (a tuning override): Chebyshev steps with a separate A d vector
 static bool cheb_unfused() {
   static const bool v = [] {
     const char* e = std::getenv("LPG_CHEB");
@@ -574,31 +578,28 @@ int MultiGrid::smooth(PLevel& L, const T* r, T* X, bool xIsZero, cudaStream_t s)
   // same recurrence as the reference's loop (x += d before each application of A, and
   // once at the end), with each x += d fused into the pass that produced d
   if (!xIsZero && (rc = op<T>(L.el, X, RES, s))) return rc;
-  // FP32 C0 levels: the smoother keeps the unscaled residual u = r - A x, which the
-  // operator updates in place (u -= A d, assembled straight into it): no A d vector and no
-  // memset of it, and each step pass reads 4 vectors and writes 2 instead of 5 and 3
-  const bool fused = std::is_same<T, float>::value && !L.el->ipdg && !cheb_unfused();
-  bool started = false;
-  if constexpr (std::is_same<T, float>::value) {
-    if (fused) {
-      if ((rc = cheb_start_u<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s)))
-        return rc;
-      started = true;
-    }
-  }
-  if (!started && (rc = cheb_start<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s)))
-    return rc;
+  // C0 levels (but with the double-word operator): the smoother keeps the unscaled residual
+  // u = r - A x, which the operator updates in place (u -= A d, assembled straight into it): no
+  // A d vector and no clearing of it, and each step pass reads 4 vectors and writes 2 instead
+  // of 5 and 3
+  bool fused = !L.el->ipdg && !cheb_unfused();
+  if constexpr (std::is_same<T, double>::value) fused = fused && L.el->can_subtract();
+  if (fused)
+    rc = cheb_start_u<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s);
+  else
+    rc = cheb_start<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s);
+  if (rc) return rc;
   for (int k = 0; k < opt.chebDegree; ++k) {
     rho_np1 = 1.0 / (2. * sigma - rho_n);
     const double rhoDivDelta = 2.0 * rho_np1 / delta;
     const bool last = (k == opt.chebDegree - 1);   // the last step's res and d are not read again
-    if constexpr (std::is_same<T, float>::value) {
-      if (fused) {
-        if ((rc = L.el->OperatorF32(d, RES, opt.prec, s, -1.f))) return rc;
-        if ((rc = cheb_step_u<T>(N, invDiag, RES, d, X, (T)(rho_np1 * rho_n), (T)rhoDivDelta, s, last))) return rc;
-        rho_n = rho_np1;
-        continue;
-      }
+    if (fused) {
+      if constexpr (std::is_same<T, float>::value) rc = L.el->OperatorF32(d, RES, opt.prec, s, -1.f);
+      else rc = L.el->OperatorSubtract(d, RES, s);
+      if (rc) return rc;
+      if ((rc = cheb_step_u<T>(N, invDiag, RES, d, X, (T)(rho_np1 * rho_n), (T)rhoDivDelta, s, last))) return rc;
+      rho_n = rho_np1;
+      continue;
     }
     if ((rc = op<T>(L.el, d, Ad, s))) return rc;
     if ((rc = cheb_step<T>(N, invDiag, Ad, RES, d, X, (T)(rho_np1 * rho_n), (T)rhoDivDelta, s, last))) return rc;

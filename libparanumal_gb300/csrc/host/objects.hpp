@@ -187,6 +187,7 @@ struct Elliptic {
   int BuildMatrixIpdg(std::vector<int64_t>& rowStarts, std::vector<int32_t>& cols, std::vector<double>& vals,
                       cudaStream_t s);
   IpdgArgs ipdg_args() const;
+  AxArgs<double, double> ax_args() const;
 
   int setup(Platform* p, const MeshConfig& c, int N, double lambda, const std::vector<double>* lamE,
             cudaStream_t s);
@@ -203,6 +204,9 @@ struct Elliptic {
   bool opDW = false;
   // zeroed: Aq is already 0 (a C0 operator then assembles into it without clearing it)
   int Operator(const double* q, double* Aq, cudaStream_t s, bool zeroed = false);
+  // u -= A q, assembled straight into u; for C0 operators in native FP64 (can_subtract())
+  bool can_subtract() const { return !ipdg && !opDW; }
+  int OperatorSubtract(const double* q, double* u, cudaStream_t s);
   int OperatorDW(const double* q, double* Aq, cudaStream_t s, bool zeroed = false);
   // accumulate = 0: Aq = A q; otherwise Aq += accumulate * A q (C0 only)
   // accumulate != 0: Aq += accumulate * A q (C0 only)

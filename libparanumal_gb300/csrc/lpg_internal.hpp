@@ -28,7 +28,7 @@ struct AxArgs {
   const T* q = nullptr;
   T* out = nullptr;
   int64_t Nglobal = 0;
-  // assembled modes: out += outScale * A q (FP32 kernels only; FP64 requires 1). With
+  // assembled modes: out += outScale * A q (FP64: 1 or -1). With
   // out preset to b and outScale = -1 an AccumulateAssembled launch leaves the residual
   // b - A q without a separate vector pass.
   T outScale = T(1);

@@ -771,6 +771,10 @@ int cheb_step_u(int64_t N, const T* invDiag, const T* u, T* d, T* x, T a, T b, c
   LPG_LAUNCH_CHECK("cheb_step_u_kernel");
   return LPG_OK;
 }
+template int cheb_start_u<double>(int64_t, const double*, const double*, const double*, double*, double*, double*, double,
+                                  bool, cudaStream_t);
+template int cheb_step_u<double>(int64_t, const double*, const double*, double*, double*, double, double, cudaStream_t,
+                                 bool);
 template int cheb_start_u<float>(int64_t, const float*, const float*, const float*, float*, float*, float*, float, bool,
                                  cudaStream_t);
 template int cheb_step_u<float>(int64_t, const float*, const float*, float*, float*, float, float, cudaStream_t, bool);
