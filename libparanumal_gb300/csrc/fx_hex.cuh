@@ -195,7 +195,7 @@ struct FxElement {
 };
 
 // tables of D and D^T with the exponents of their rows, by the threads of a CTA; true where
-// an entry beyond 2^63 leaves every line to FP64
+// a row whose largest entry lies outside [2^-63, 2^63] leaves every line to FP64
 template <int NQ, bool EO>
 __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid, const int threads,
                                           fx_half (&tab)[2][FxLayout<NQ, EO>::ROWS * FxLayout<NQ, EO>::RS],
@@ -211,7 +211,7 @@ __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const i
     const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
     tab[tr][t * L::RS + c] = fx_table_entry<NQ, EO>(Dg, tr, t, c, eR);
     if (c == 0) ex[tr][t] = eR;
-    plain |= eR > 1086;
+    plain |= eR > 1086 || (key >> 20) < 960;
   }
   return plain;
 }

@@ -104,3 +104,27 @@ def test_entry_point_forms(N, prec, form):
     copies = np.bincount(idx[idx >= 0], minlength=Ng).max()   # the assembly of random indices
     err = np.abs(out.cpu().numpy().astype(LD) - ref)
     assert np.all(err <= (2 * Nq + 8 + copies) * roundoff * mag)
+
+
+@pytest.mark.parametrize("N", [2, 3, 6, 7])
+@pytest.mark.parametrize("scale", [2.0 ** -90, 2.0 ** 90])
+def test_scaled_derivative(N, scale):
+    """A D outside the integers' range of rows is served by FP64 lines: same bound."""
+    rng = np.random.default_rng(N)
+    Nq, E = N + 1, 5
+    Np = Nq ** 3
+    D = rng.uniform(-2, 2, (Nq, Nq)) * scale
+    if N in (3, 7):
+        D = 0.5 * (D - D[::-1, ::-1])
+    geo, q = rng.uniform(-1, 1, (E, 7, Nq, Nq, Nq)), rng.uniform(-1, 1, E * Np)
+    dev = lambda x: torch.tensor(x, device="cuda").reshape(-1)
+    dG, out = dev(geo), torch.empty(E * Np, dtype=torch.float64, device="cuda")
+    lpg.ax_hex("f64", N, E, dev(np.arange(E * Np, dtype=np.int32)), dG, 7 * Np, dG[6 * Np:], 7 * Np, dev(D), 0.0,
+               dev(q), out, E * Np)
+    torch.cuda.synchronize()
+    LD = np.longdouble
+    G, W, u = geo[:, :6].astype(LD), geo[:, 6].astype(LD), q.astype(LD).reshape(-1, Nq, Nq, Nq)
+    ref = _apply(G, W, D.astype(LD), np.zeros(E, LD), u)
+    mag = _apply(np.abs(G), W, np.abs(D).astype(LD), np.zeros(E, LD), np.abs(u), top=True)
+    err = np.abs(out.cpu().numpy().astype(LD) - ref.reshape(-1))
+    assert np.all(err <= (2 * Nq + 8 + 1) * 2.0 ** -53 * mag.reshape(-1))
