@@ -125,8 +125,11 @@ struct DCSR {
       if ((rc = cols.alloc(A.nnz())) || (rc = cols.upload(A.cols.data(), A.nnz(), s))) return rc;
       if ((rc = vals.alloc(A.nnz())) || (rc = vals.upload(A.vals.data(), A.nnz(), s))) return rc;
     }
+    longRows = A.nnz() > 48 * A.n;   // csr_pass_kernel
     return LPG_OK;
   }
+  bool longRows = false;
+  CsrView view() const { return {n, rs.p, cols.p, vals.p, longRows}; }
 };
 
 // ================================================================ AMG setup (host)
@@ -760,19 +763,25 @@ int MultiGrid::smooth_a(ALevel& L, const double* b, double* x, bool xIsZero, cud
   const double invTheta = 1.0 / theta;
   const double sigma = theta / delta;
   double rho_n = 1. / sigma, rho_np1;
-  double* d = L.s1.p;
-  double* r = L.s2.p;
+  // d alternates between two vectors, and a start on x != 0 works on a copy of x (L.res, free
+  // while smoothing): other rows still read the old ones
+  double *d = L.s1.p, *dNext = L.s3.p, *r = L.s2.p, *xs = x;
+  const CsrView A = L.dA.view();
   if (xIsZero) {
     if ((rc = csr_cheb_start(N, invTheta, L.dDiagInv.p, b, r, d, x, s))) return rc;
   } else {
-    if ((rc = csr_cheb_residual(N, L.dA.rs.p, L.dA.cols.p, L.dA.vals.p, 0.0, 1.0, L.dDiagInv.p, b, x, r, s))) return rc;
-    if ((rc = csr_cheb_update(N, 0.0, invTheta, opt.amgChebDegree == 0, r, d, x, s))) return rc;
+    if ((rc = csr_cheb_restart(A, L.dDiagInv.p, invTheta, b, x, r, d, L.res.p, s))) return rc;
+    xs = L.res.p;
+    if (opt.amgChebDegree <= 0)
+      LPG_CUDA_TRY(cudaMemcpyAsync(x, xs, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
   }
   for (int k = 0; k < opt.amgChebDegree; ++k) {
-    if ((rc = csr_cheb_residual(N, L.dA.rs.p, L.dA.cols.p, L.dA.vals.p, 1.0, 0.0, L.dDiagInv.p, b, d, r, s))) return rc;
     rho_np1 = 1.0 / (2. * sigma - rho_n);
-    if ((rc = csr_cheb_update(N, rho_np1 * rho_n, 2.0 * rho_np1 / delta, k == opt.amgChebDegree - 1, r, d, x, s)))
+    const bool last = k == opt.amgChebDegree - 1;
+    if ((rc = csr_cheb_step(A, L.dDiagInv.p, rho_np1 * rho_n, 2.0 * rho_np1 / delta, d, r, last ? nullptr : dNext, xs,
+                            last ? x : xs, s)))
       return rc;
+    std::swap(d, dNext);
     rho_n = rho_np1;
   }
   return LPG_OK;
@@ -782,14 +791,12 @@ int MultiGrid::vcycle_a(int k, const double* RHS, double* X, cudaStream_t s) {
   if (k == (int)a.size() - 1) return gemv(coarseN, coarseInv.p, RHS, X, s);
   ALevel& L = *a[k];
   ALevel& C = *a[k + 1];
-  const int64_t N = L.A.n;
   int rc;
   if ((rc = smooth_a(L, RHS, X, true, s))) return rc;
-  if ((rc = csr_spmv(N, L.dA.rs.p, L.dA.cols.p, L.dA.vals.p, -1.0, X, 0.0, L.res.p, s))) return rc;
-  if ((rc = axpy<double>(N, 1.0, RHS, 1.0, L.res.p, s))) return rc;
-  if ((rc = csr_spmv(L.R.n, L.dR.rs.p, L.dR.cols.p, L.dR.vals.p, 1.0, L.res.p, 0.0, C.rhs.p, s))) return rc;
+  if ((rc = csr_residual(L.dA.view(), RHS, X, L.res.p, s))) return rc;
+  if ((rc = csr_product(L.dR.view(), L.res.p, C.rhs.p, s))) return rc;
   if ((rc = vcycle_a(k + 1, C.rhs.p, C.x.p, s))) return rc;
-  if ((rc = csr_spmv(N, L.dP.rs.p, L.dP.cols.p, L.dP.vals.p, 1.0, C.x.p, 1.0, X, s))) return rc;
+  if ((rc = csr_product_add(L.dP.view(), C.x.p, X, s))) return rc;
   return smooth_a(L, RHS, X, false, s);
 }
 
@@ -889,7 +896,7 @@ int MultiGrid::setup_amg(Elliptic* el, Rand48& rng) {
     ALevel& L = *a[k];
     const int64_t n = L.A.n;
     if ((rc = L.rhs.alloc(n)) || (rc = L.x.alloc(n)) || (rc = L.res.alloc(n)) || (rc = L.s1.alloc(n)) ||
-        (rc = L.s2.alloc(n)))
+        (rc = L.s2.alloc(n)) || (rc = L.s3.alloc(n)))
       return rc;
     if (k + 1 < a.size()) {
       if ((rc = L.dA.upload(L.A, s)) || (rc = L.dP.upload(L.P, s)) || (rc = L.dR.upload(L.R, s))) return rc;

@@ -289,6 +289,24 @@ int csr_cheb_residual(int64_t N, const int64_t* rowStarts, const int32_t* cols, 
                       const double* x, double* r, cudaStream_t s);
 int csr_cheb_update(int64_t N, double a, double b, int lastIt, const double* r, double* d,
                     double* x, cudaStream_t s);
+// passes of the level cycle (pmg_amg.cu); longRows: a warp a row
+struct CsrView {
+  int64_t n = 0;
+  const int64_t* rowStarts = nullptr;
+  const int32_t* cols = nullptr;
+  const double* vals = nullptr;
+  bool longRows = false;
+};
+int csr_product(const CsrView& A, const double* x, double* y, cudaStream_t s);        // y = A x
+int csr_product_add(const CsrView& A, const double* x, double* y, cudaStream_t s);    // y += A x
+int csr_residual(const CsrView& A, const double* b, const double* x, double* res, cudaStream_t s);   // res = b - A x
+// r = diagInv (b - A x), d = invTheta r, xOut = x + d (xOut is not x)
+int csr_cheb_restart(const CsrView& A, const double* diagInv, double invTheta, const double* b, const double* x,
+                     double* r, double* d, double* xOut, cudaStream_t s);
+// r -= diagInv (A d), dOut = a d + b r, xOut = x + dOut; dOut == nullptr: the last step, r and
+// dOut not stored (dOut is not d; xOut may be x)
+int csr_cheb_step(const CsrView& A, const double* diagInv, double a, double b, const double* d, double* r, double* dOut,
+                  const double* x, double* xOut, cudaStream_t s);
 // dense y = A x, A row-major n x n
 int gemv(int64_t n, const double* A, const double* x, double* y, cudaStream_t s);
 
