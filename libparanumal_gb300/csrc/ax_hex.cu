@@ -132,135 +132,6 @@ ax_hex_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
   }
 }
 
-// ---------------------------------------------------------------- FP32 line variant
-// FP32 vectors at the degrees whose element rows are not 16-byte multiples (odd Nq), which the
-// staged kernel cannot copy. One thread holds one line at a time: its t-pencil in registers,
-// its r- and s-line through two line-contiguous copies of the element in shared memory,
-// contracted in place. An element needs 4 barriers instead of 3 a layer, and the factors of
-// all its layers are loaded independently of them.
-template <int NQ>
-struct LineLayout {
-  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ;
-  // Odd row pitch, and the copies of a CTA's elements one after the other: line l of element
-  // el starts at P (l + NL el), without bank conflicts across the warps' element boundaries.
-  static constexpr int P = NQ | 1, PL = P * NQ, ES = P * NL;
-  static constexpr int EPB = 256 / NL, NT = NL * EPB;
-  static constexpr int RD = (NQ + 3) & ~3;        // row of D in shared memory, 16-byte multiple
-  static constexpr int MINB = NQ <= 3 ? 5 : 4;    // resident CTAs per SM to compile for, best of 2 to 5
-};
-
-// y = M x with the rows of M read from shared memory (16-byte aligned, RD entries)
-template <int NQ>
-__device__ __forceinline__ void line_product(const float* __restrict__ M, const float (&x)[NQ], float (&y)[NQ]) {
-  constexpr int RD = LineLayout<NQ>::RD;
-#pragma unroll
-  for (int t = 0; t < NQ; ++t) {
-    float r0 = 0.f, r1 = 0.f;
-#pragma unroll
-    for (int m = 0; m < NQ; m += 4) {
-      const float4 c = *reinterpret_cast<const float4*>(M + t * RD + m);
-      r0 += c.x * x[m];
-      if (m + 1 < NQ) r1 += c.y * x[m + 1 < NQ ? m + 1 : 0];
-      if (m + 2 < NQ) r0 += c.z * x[m + 2 < NQ ? m + 2 : 0];
-      if (m + 3 < NQ) r1 += c.w * x[m + 3 < NQ ? m + 3 : 0];
-    }
-    y[t] = r0 + r1;
-  }
-}
-
-template <int NQ, typename G, bool MASS>
-__global__ void __launch_bounds__(LineLayout<NQ>::NT, LineLayout<NQ>::MINB)
-ax_hex_line_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
-                   const int32_t* __restrict__ g2l, const G* __restrict__ ggeo, const int64_t geoStride,
-                   const G* __restrict__ wJ, const int64_t wJStride, const float* __restrict__ Dg, const float lambda,
-                   const float* __restrict__ lambdaE, const float* __restrict__ q, float* __restrict__ out,
-                   const float outScale) {
-  using L = LineLayout<NQ>;
-  constexpr int NP = L::NP, NL = L::NL, P = L::P, PL = L::PL, EPB = L::EPB;
-  constexpr int UD = NQ <= 6 ? 2 : 1;
-  __shared__ __align__(16) float s_D[2][NQ * L::RD];   // D, D^T
-  __shared__ float s_v[2][EPB * L::ES];
-  const int tid = threadIdx.x, el = tid / NL, l = tid % NL, a = l % NQ, b = l / NQ;
-  float* const line = &s_v[0][P * tid];                           // r-line l (s: EPB ES further)
-  float* const nr = &s_v[0][el * L::ES + b * P + a];              // node (a, b, k): k PL further
-  float* const ns = &s_v[1][el * L::ES + a * P + b];
-  int64_t e = (int64_t)blockIdx.x * EPB + el;
-  const bool active = e < Nelements;
-  if (active && elementList) e = elementList[e];
-  if (!active) e = 0;
-  const int64_t nodeBase = e * NP + l;
-  // one thread asks for the factors of the CTA's run of elements in L2 (whole 16-byte units
-  // inside the run: the rows are not aligned)
-  if (tid == 0 && !elementList && geoStride <= 7 * NP) {
-    const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
-    const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
-    const uintptr_t hi = (uintptr_t)(ggeo + (e + n) * geoStride) & ~(uintptr_t)15;
-    if (hi > lo) prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
-  }
-  int32_t id[NQ];
-  float v0[NQ], ut[NQ];
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
-  for (int t = tid; t < NL; t += L::NT) {
-    const float d = Dg[t];
-    s_D[0][t / NQ * L::RD + t % NQ] = d;
-    s_D[1][t % NQ * L::RD + t / NQ] = d;
-  }
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) v0[k] = id[k] >= 0 ? q[id[k]] : 0.f;
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) nr[k * PL] = ns[k * PL] = v0[k];
-  __syncthreads();
-  auto lines = [&](const float* M) {
-#pragma unroll UD
-    for (int d = 0; d < 2; ++d) {
-      if constexpr (UD == 1) asm volatile("" ::: "memory");   // keeps D out of registers
-      float* const o = line + d * EPB * L::ES;
-      float x[NQ], y[NQ];
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) x[m] = o[m];
-      line_product<NQ>(M, x, y);
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) o[m] = y[m];
-    }
-    if constexpr (UD == 1) asm volatile("" ::: "memory");
-  };
-  lines(s_D[0]);
-  line_product<NQ>(s_D[0], v0, ut);
-  __syncthreads();
-  const G* gp = ggeo + e * geoStride + l;
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    float g[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) g[c] = active ? load_geo<float, G>(gp + c * NP + k * NL) : 0.f;
-    const float qr = nr[k * PL], qs = ns[k * PL], qt = ut[k];
-    nr[k * PL] = g[0] * qr + g[1] * qs + g[2] * qt;
-    ns[k * PL] = g[1] * qr + g[3] * qs + g[4] * qt;
-    ut[k] = g[2] * qr + g[4] * qs + g[5] * qt;
-  }
-  __syncthreads();
-  lines(s_D[1]);
-  float At[NQ];
-  line_product<NQ>(s_D[1], ut, At);
-  __syncthreads();
-  if (!active) return;
-  const float lam = MASS ? (lambdaE ? lambdaE[e] : lambda) : 0.f;
-  const G* wp = wJ + e * wJStride + l;
-#pragma unroll
-  for (int k = 0; k < NQ; ++k) {
-    float r = At[k] + nr[k * PL] + ns[k * PL];
-    if constexpr (MASS) r += load_geo<float, G>(wp + k * NL) * lam * v0[k];
-    if (id[k] >= 0) atomicAdd(out + id[k], outScale * r);
-  }
-}
-
-// ---------------------------------------------------------------- staged variant
-// Persistent CTAs walk groups of EPB elements. Each element's geometric factors (7 x Np)
-// and GlobalToLocal block (Np int32) are copied into a STAGES-deep shared-memory ring
-// with 16-byte cp.async, STAGES-1 groups ahead of the one being computed, so DRAM traffic
-// overlaps the contractions. D's rows and columns needed by a thread live in registers;
-// the t-direction contractions of the whole pencil run once per element (64 FMA each way).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
@@ -268,6 +139,210 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+template <typename G> __device__ __forceinline__ float geo_to_float(G v);
+template <> __device__ __forceinline__ float geo_to_float<float>(float v) { return v; }
+template <> __device__ __forceinline__ float geo_to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+// ---------------------------------------------------------------- FP32 line kernel
+// FP32 vectors. One thread holds one line of an element in each direction: its t-line in
+// registers, its r- and s-line through two line-contiguous copies of the element in shared
+// memory, contracted in place; a row of D is read once for the three. Two passes (D, D^T) with
+// the metric product between them, 4 barriers an element. Many small CTAs: while some wait for
+// their loads, others compute. 48^3, N = 7 with FP32 factors moves 2.26 GB in 357 us, 0.93 of
+// the measured copy rate; with BF16 factors shared memory bounds it (80 % of its cycles).
+template <int NQ>
+struct LineLayout {
+  static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ;
+  static constexpr bool VEC = NQ % 4 == 0;   // lines of whole 16-byte units
+  // Line l of an element starts at P l. An odd pitch keeps the accesses to lines and to columns
+  // free of bank conflicts; at Nq = 8 the two 16-byte halves of a line trade places in every
+  // other group of four lines instead, and at Nq = 4 the elements of a warp lie 16 banks apart.
+  static constexpr int P = VEC ? NQ : NQ | 1;
+  static constexpr int ES = P * NL + (NQ == 4 ? 16 : 0);   // a copy of an element
+  // threads of a CTA (at most, at least one element) and resident CTAs per SM to compile for: the
+  // best of 64, 128 and 256 threads and of 3 to 18 CTAs. Larger against chosen, us: 100^3, N = 1
+  // 73.5 / 66.2; 80^3, N = 2 122.6 / 109.1; 48^3, N = 4 114.1 / 109.9; smaller against chosen:
+  // 40^3, N = 5 113.5 / 110.9; 30^3, N = 6 88.6 / 82.9; 24^3, N = 8 110.3 / 95.6
+  static constexpr int CTA = VEC || NQ <= 3 ? 64 : NQ == 5 ? 128 : 256, EPB = CTA / NL, NT = NL * EPB;
+  static constexpr int RD = (NQ + 3) & ~3;                 // row of D in shared memory, 16-byte multiple
+  // (Nq = 8, with the mass term and without a copy: 48^3 383 us at 16, 401 at 14)
+  static constexpr int minb(bool full) {
+    return NQ == 8 && full ? 16 : VEC ? 14 : NQ <= 3 ? 12 : NQ == 5 ? 10 : NQ == 9 ? 3 : 4;
+  }
+  __device__ __forceinline__ static constexpr int at(int l, int m) { return P * l + (NQ == 8 ? m ^ (l & 4) : m); }
+};
+
+// COPY: the factors are copied to shared memory by 16-byte cp.async while q is gathered and
+// differentiated, instead of asked for in L2 and read where they are used
+template <int NQ, typename G, bool MASS, bool COPY>
+__global__ void __launch_bounds__(LineLayout<NQ>::NT, LineLayout<NQ>::minb(MASS && !COPY))
+ax_hex_line_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
+                   const int32_t* __restrict__ g2l, const G* __restrict__ ggeo, const int64_t geoStride,
+                   const G* __restrict__ wJ, const int64_t wJStride, const float* __restrict__ Dg, const float lambda,
+                   const float* __restrict__ lambdaE, const float* __restrict__ q, float* __restrict__ out,
+                   const float outScale) {
+  using L = LineLayout<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, RD = L::RD, ROWS = MASS ? 7 : 6;
+  constexpr int ROW_BYTES = NP * (int)sizeof(G);
+  constexpr bool REREAD = NQ == 8 && !COPY;   // the dofs are read again: fewer registers, more CTAs
+  __shared__ __align__(16) float s_D[2][NQ * RD];   // D, D^T
+  __shared__ __align__(16) float s_v[2][EPB * L::ES];
+  __shared__ __align__(16) unsigned char s_g[COPY ? EPB * ROWS * ROW_BYTES : 16];
+  const int tid = threadIdx.x, el = tid / NL, l = tid % NL, a = l % NQ, b = l / NQ;
+  float* const vr = &s_v[0][el * L::ES];   // r-lines: line (k, b), entry a
+  float* const vs = &s_v[1][el * L::ES];   // s-lines: line (k, a), entry b
+  const G* const sg = reinterpret_cast<const G*>(s_g) + el * ROWS * NP + l;
+  int64_t e = (int64_t)blockIdx.x * EPB + el;
+  const bool active = e < Nelements;
+  if (active && elementList) e = elementList[e];
+  if (!active) e = 0;
+  const int64_t nodeBase = e * NP + l;
+  if constexpr (!COPY) {
+    if ((MASS || NQ < 4) && !elementList && geoStride <= 7 * NP) {
+      // one thread asks for the factors of the CTA's run of elements in L2 (whole 16-byte
+      // units inside the run: the rows need not be aligned)
+      if (tid == 0) {
+        const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
+        const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
+        const uintptr_t hi = (uintptr_t)(ggeo + (e + n) * geoStride) & ~(uintptr_t)15;
+        if (hi > lo) prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
+      }
+    } else if (NQ >= 4 && l == 0 && active) {
+      const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
+      const uintptr_t hi = (uintptr_t)(ggeo + e * geoStride + 6 * NP) & ~(uintptr_t)15;
+      prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
+      if constexpr (MASS) {
+        const uintptr_t lw = ((uintptr_t)(wJ + e * wJStride) + 15) & ~(uintptr_t)15;
+        const uintptr_t hw = (uintptr_t)(wJ + e * wJStride + NP) & ~(uintptr_t)15;
+        prefetch_l2_bulk((const void*)lw, (unsigned)(hw - lw));
+      }
+    }
+  }
+  int32_t id[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) id[k] = active ? __ldg(g2l + nodeBase + k * NL) : -1;
+  if constexpr (COPY) {
+    if (active) {
+      constexpr int C = ROW_BYTES / 16;
+      unsigned char* const dst = s_g + el * ROWS * ROW_BYTES;
+      const char* src = reinterpret_cast<const char*>(ggeo + e * geoStride);
+      for (int c = l; c < 6 * C; c += NL) cp_async16(dst + 16 * c, src + 16 * c);
+      if constexpr (MASS) {
+        src = reinterpret_cast<const char*>(wJ + e * wJStride);
+        for (int c = l; c < C; c += NL) cp_async16(dst + 16 * (6 * C + c), src + 16 * c);
+      }
+    }
+    cp_async_commit();
+  }
+  for (int t = tid; t < NL; t += L::NT) {
+    s_D[0][t / NQ * RD + t % NQ] = Dg[t];
+    s_D[1][t / NQ * RD + t % NQ] = Dg[t % NQ * NQ + t / NQ];
+  }
+  float v0[NQ], vt[NQ];
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) v0[k] = id[k] >= 0 ? q[id[k]] : 0.f;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    vr[L::at(k * NQ + b, a)] = vs[L::at(k * NQ + a, b)] = v0[k];
+    vt[k] = v0[k];
+  }
+  __syncthreads();
+  auto lines = [&](const float* M) {   // r-line l, s-line l and the column vt times M
+    float xr[NQ], xs[NQ], xt[NQ];
+    if constexpr (L::VEC) {
+#pragma unroll
+      for (int c = 0; c < NQ; c += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(vr + L::at(l, c));
+        const float4 w = *reinterpret_cast<const float4*>(vs + L::at(l, c));
+        xr[c] = u.x; xr[c + 1] = u.y; xr[c + 2] = u.z; xr[c + 3] = u.w;
+        xs[c] = w.x; xs[c + 1] = w.y; xs[c + 2] = w.z; xs[c + 3] = w.w;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) {
+        xr[m] = vr[L::at(l, m)];
+        xs[m] = vs[L::at(l, m)];
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < NQ; ++m) xt[m] = vt[m];
+    if constexpr (L::VEC) {
+      float y[NQ];
+#pragma unroll
+      for (int c = 0; c < NQ; c += 4) {
+        float yr[4], ys[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float r0 = 0.f, r1 = 0.f, s0 = 0.f, s1 = 0.f, t0 = 0.f, t1 = 0.f;
+#pragma unroll
+          for (int m = 0; m < NQ; m += 4) {
+            const float4 d = *reinterpret_cast<const float4*>(M + (c + u) * NQ + m);
+            r0 += d.x * xr[m]; r1 += d.y * xr[m + 1]; r0 += d.z * xr[m + 2]; r1 += d.w * xr[m + 3];
+            s0 += d.x * xs[m]; s1 += d.y * xs[m + 1]; s0 += d.z * xs[m + 2]; s1 += d.w * xs[m + 3];
+            t0 += d.x * xt[m]; t1 += d.y * xt[m + 1]; t0 += d.z * xt[m + 2]; t1 += d.w * xt[m + 3];
+          }
+          yr[u] = r0 + r1; ys[u] = s0 + s1; y[c + u] = t0 + t1;
+        }
+        *reinterpret_cast<float4*>(vr + L::at(l, c)) = make_float4(yr[0], yr[1], yr[2], yr[3]);
+        *reinterpret_cast<float4*>(vs + L::at(l, c)) = make_float4(ys[0], ys[1], ys[2], ys[3]);
+      }
+#pragma unroll
+      for (int k = 0; k < NQ; ++k) vt[k] = y[k];
+      return;
+    }
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) {
+      float r[2] = {0.f, 0.f}, s[2] = {0.f, 0.f}, u[2] = {0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < NQ; c += 4) {
+        const float4 d4 = *reinterpret_cast<const float4*>(M + t * RD + c);
+        const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+        for (int m = c; m < NQ && m < c + 4; ++m) {
+          r[m & 1] += d[m - c] * xr[m];
+          s[m & 1] += d[m - c] * xs[m];
+          u[m & 1] += d[m - c] * xt[m];
+        }
+      }
+      vr[L::at(l, t)] = r[0] + r[1];
+      vs[L::at(l, t)] = s[0] + s[1];
+      vt[t] = u[0] + u[1];
+    }
+  };
+  lines(s_D[0]);
+  const float lam = MASS && active ? (lambdaE ? lambdaE[e] : lambda) : 0.f;
+  if constexpr (COPY) cp_async_wait<0>();
+  __syncthreads();
+  const G* const gp = ggeo + e * geoStride + l;
+  const G* const wp = wJ + e * wJStride + l;
+  if (active) {
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      float g[ROWS];
+#pragma unroll
+      for (int c = 0; c < ROWS; ++c)
+        g[c] = COPY ? geo_to_float(sg[c * NP + k * NL]) : load_geo<float, G>(c == 6 ? wp + k * NL : gp + c * NP + k * NL);
+      float &r = vr[L::at(k * NQ + b, a)], &s = vs[L::at(k * NQ + a, b)];
+      const float qr = r, qs = s, qt = vt[k];
+      r = g[0] * qr + g[1] * qs + g[2] * qt;
+      s = g[1] * qr + g[3] * qs + g[4] * qt;
+      vt[k] = g[2] * qr + g[4] * qs + g[5] * qt;
+      if constexpr (MASS) v0[k] *= g[6] * lam;
+    }
+  }
+  __syncthreads();
+  lines(s_D[1]);
+  __syncthreads();
+  if (!active) return;
+#pragma unroll
+  for (int k = 0; k < NQ; ++k) {
+    float r = vt[k] + vr[L::at(k * NQ + b, a)] + vs[L::at(k * NQ + a, b)];
+    if constexpr (MASS) r += v0[k];
+    const int32_t g = REREAD ? __ldg(g2l + nodeBase + k * NL) : id[k];
+    if (g >= 0) atomicAdd(out + g, outScale * r);
+  }
+}
 
 // Barrier over the NQ*NQ threads of one element (named barrier 1 + el) when that is a
 // whole number of warps, else over the CTA.
@@ -278,228 +353,6 @@ __device__ __forceinline__ void elem_sync(const int el) {
   } else {
     __syncthreads();
   }
-}
-
-template <typename G> __device__ __forceinline__ float geo_to_float(G v);
-template <> __device__ __forceinline__ float geo_to_float<float>(float v) { return v; }
-template <> __device__ __forceinline__ float geo_to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-template <int NQ, typename G>
-struct StagedLayout {
-  static constexpr int NP = NQ * NQ * NQ;
-  static constexpr int ROW_BYTES = NP * (int)sizeof(G);
-  static constexpr int GEO_BYTES = 7 * ROW_BYTES;
-  static constexpr int IDX_BYTES = NP * 4;
-  static constexpr int ELEM_BYTES = GEO_BYTES + IDX_BYTES;
-  static constexpr bool ok = (ROW_BYTES % 16 == 0) && (IDX_BYTES % 16 == 0);
-};
-
-// Dot product of NQ coefficients with a shared-memory row: 128-bit loads when the row is
-// 16-byte aligned and NQ is a multiple of 4.
-template <int NQ, bool VEC>
-__device__ __forceinline__ float row_dot(const float* __restrict__ row, const float* c) {
-  float acc = 0.f;
-  if constexpr (VEC) {
-    // two partial sums halve the dependent FMA chain
-    float acc1 = 0.f;
-#pragma unroll
-    for (int m = 0; m < NQ; m += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(row + m);
-      acc += c[m] * v.x;
-      acc1 += c[m + 1] * v.y;
-      acc += c[m + 2] * v.z;
-      acc1 += c[m + 3] * v.w;
-    }
-    acc += acc1;
-  } else {
-#pragma unroll
-    for (int m = 0; m < NQ; ++m) acc += c[m] * row[m];
-  }
-  return acc;
-}
-
-// MASS = false: lambda == 0 and no lambda field, the wJ row is neither copied nor used
-template <int NQ, typename T, typename G, int EPB, int STAGES, bool PF = false, bool MASS = true>
-__global__ void __launch_bounds__(NQ * NQ * EPB)
-ax_hex_staged_kernel(const int64_t Nelements, const int32_t* __restrict__ elementList,
-                     const int32_t* __restrict__ g2l, const G* __restrict__ ggeo, const int64_t geoStride,
-                     const G* __restrict__ wJ, const int64_t wJStride, const T* __restrict__ Dg, const T lambda,
-                     const T* __restrict__ lambdaE, const T* __restrict__ q, T* __restrict__ out,
-                     const T outScale) {
-  static_assert(std::is_same<T, float>::value, "staged kernel is FP32");
-  using L = StagedLayout<NQ, G>;
-  constexpr int NP = L::NP, NT = NQ * NQ * EPB;
-  constexpr int CHUNKS = L::ELEM_BYTES / 16;
-  constexpr int STAGE_BYTES = EPB * L::ELEM_BYTES;
-  constexpr bool VEC = (NQ % 4 == 0);
-  constexpr int RS = VEC ? NQ : NQ;          // row stride of s_q / s_Gqr
-  constexpr int TS = VEC ? NQ + 4 : NQ + 1;  // row stride of the transposed copies (bank-conflict padding)
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ __align__(16) float s_D[NQ][NQ];
-  // layer slabs, double-buffered by layer parity so one barrier per layer suffices
-  // between reading a slab and overwriting it two layers later
-  __shared__ __align__(16) float s_q[2][EPB][NQ][RS];     // s_q[j][i]   = q(i,j,k)
-  __shared__ __align__(16) float s_qT[2][EPB][NQ][TS];    // s_qT[i][j]  = q(i,j,k)
-  __shared__ __align__(16) float s_Gqr[2][EPB][NQ][RS];   // s_Gqr[j][i]
-  __shared__ __align__(16) float s_GqsT[2][EPB][NQ][TS];  // s_GqsT[i][j]
-
-  const int i = threadIdx.x, j = threadIdx.y, el = threadIdx.z;
-  const int tid = i + NQ * (j + NQ * el);
-  for (int t = tid; t < NQ * NQ; t += NT) s_D[t / NQ][t % NQ] = Dg[t];
-  const int64_t ngroups = (Nelements + EPB - 1) / EPB;
-
-  // copy of one element group: 7 geometric-factor rows and the index row per element,
-  // each a contiguous run of 16-byte chunks (compile-time trip counts)
-  constexpr int ROW_CHUNKS = L::ROW_BYTES / 16, IDX_CHUNKS = L::IDX_BYTES / 16;
-  auto issue = [&](const int64_t grp, const int stage) {
-    if (grp < ngroups) {
-      unsigned char* base = smem + stage * STAGE_BYTES;
-#pragma unroll
-      for (int le = 0; le < EPB; ++le) {
-        const int64_t ei = grp * EPB + le;
-        if (ei < Nelements) {
-          const int64_t e = elementList ? (int64_t)elementList[ei] : ei;
-          unsigned char* dst = base + le * L::ELEM_BYTES;
-#pragma unroll
-          for (int comp = 0; comp < (MASS ? 7 : 6); ++comp) {
-            const unsigned char* src =
-                (comp < 6) ? reinterpret_cast<const unsigned char*>(ggeo + e * geoStride + (int64_t)comp * NP)
-                           : reinterpret_cast<const unsigned char*>(wJ + e * wJStride);
-            for (int c = tid; c < ROW_CHUNKS; c += NT) cp_async16(dst + comp * L::ROW_BYTES + c * 16, src + c * 16);
-          }
-          const unsigned char* srci = reinterpret_cast<const unsigned char*>(g2l + e * NP);
-          for (int c = tid; c < IDX_CHUNKS; c += NT) cp_async16(dst + L::GEO_BYTES + c * 16, srci + c * 16);
-        }
-      }
-    }
-    cp_async_commit();
-  };
-
-#pragma unroll
-  for (int st = 0; st < STAGES - 1; ++st) issue(blockIdx.x + (int64_t)st * gridDim.x, st);
-  __syncthreads();
-  float Dr[NQ], Ds[NQ], DTi[NQ], DTj[NQ];
-#pragma unroll
-  for (int m = 0; m < NQ; ++m) {
-    Dr[m] = s_D[i][m];
-    Ds[m] = s_D[j][m];
-    DTi[m] = s_D[m][i];
-    DTj[m] = s_D[m][j];
-  }
-
-  const int node = j * NQ + i;
-  // PF: the gather of the next group's q through its staged index row is issued half-way
-  // through this group's layers (after a wait for that group's copy, which was issued at
-  // the start of this group), so its L2 latency overlaps the remaining layers
-  float n_q[PF ? NQ : 1];
-  int32_t n_id[PF ? NQ : 1];
-  auto gather_next = [&](const int64_t g, const int stage) {
-    if constexpr (PF) {
-      const int32_t* nidx = reinterpret_cast<const int32_t*>(smem + stage * STAGE_BYTES + el * L::ELEM_BYTES +
-                                                            L::GEO_BYTES);
-      const bool act = (g < ngroups) && (g * EPB + el < Nelements);
-#pragma unroll
-      for (int k = 0; k < NQ; ++k) {
-        const int32_t id = act ? nidx[k * NQ * NQ + node] : -1;
-        n_id[k] = id;
-        n_q[k] = (id >= 0) ? q[id] : 0.f;
-      }
-    }
-  };
-  if constexpr (PF) {
-    static_assert(STAGES == 2, "prefetching variant uses two stages");
-    cp_async_wait<0>();
-    __syncthreads();
-    gather_next(blockIdx.x, 0);
-  }
-
-  for (int64_t it = 0;; ++it) {
-    const int64_t grp = blockIdx.x + it * gridDim.x;
-    if (grp >= ngroups) break;
-    // this group's copies are complete, and after the barrier no thread still reads the
-    // stage of the previous group, which the next copy then refills
-    if constexpr (!PF) cp_async_wait<STAGES - 2>();
-    __syncthreads();
-    issue(grp + (int64_t)(STAGES - 1) * gridDim.x, (int)((it + STAGES - 1) % STAGES));
-    const unsigned char* base = smem + (it % STAGES) * STAGE_BYTES + el * L::ELEM_BYTES;
-    const G* sg = reinterpret_cast<const G*>(base);
-    const int32_t* sidx = reinterpret_cast<const int32_t*>(base + L::GEO_BYTES);
-    const int64_t ei = grp * EPB + el;
-    const bool active = ei < Nelements;
-    const int64_t e = active ? (elementList ? (int64_t)elementList[ei] : ei) : 0;
-
-    float r_q[NQ], r_Aq[NQ], qt[NQ], Gqt[NQ];
-    int32_t r_id[NQ];
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) {
-      if constexpr (PF) {
-        r_id[k] = n_id[k];
-        r_q[k] = n_q[k];
-      } else {
-        const int32_t id = active ? sidx[k * NQ * NQ + node] : -1;
-        r_id[k] = id;
-        r_q[k] = (id >= 0) ? q[id] : 0.f;
-      }
-    }
-    (void)sidx;
-    const float lam = (lambdaE && active) ? lambdaE[e] : lambda;
-    // t-direction of the pencil: qt = D r_q (rows of D are broadcast reads)
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) qt[k] = row_dot<NQ, VEC>(&s_D[k][0], r_q);
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) {
-      const int off = k * NQ * NQ + node;
-      const float G00 = geo_to_float(sg[0 * NP + off]), G01 = geo_to_float(sg[1 * NP + off]);
-      const float G02 = geo_to_float(sg[2 * NP + off]), G11 = geo_to_float(sg[3 * NP + off]);
-      const float G12 = geo_to_float(sg[4 * NP + off]), G22 = geo_to_float(sg[5 * NP + off]);
-      float GwJ = 0.f;
-      if constexpr (MASS) GwJ = geo_to_float(sg[6 * NP + off]);
-      const int b = k & 1;
-      s_q[b][el][j][i] = r_q[k];
-      s_qT[b][el][i][j] = r_q[k];
-      elem_sync<NQ>(el);
-      const float qr = row_dot<NQ, VEC>(&s_q[b][el][j][0], Dr);    // sum_m D[i][m] q(m,j)
-      const float qs = row_dot<NQ, VEC>(&s_qT[b][el][i][0], Ds);   // sum_m D[j][m] q(i,m)
-      s_GqsT[b][el][i][j] = G01 * qr + G11 * qs + G12 * qt[k];
-      s_Gqr[b][el][j][i] = G00 * qr + G01 * qs + G02 * qt[k];
-      Gqt[k] = G02 * qr + G12 * qs + G22 * qt[k];
-      float Auk = 0.f;
-      if constexpr (MASS) Auk = GwJ * lam * r_q[k];
-      elem_sync<NQ>(el);
-      Auk += row_dot<NQ, VEC>(&s_GqsT[b][el][i][0], DTj);       // sum_m D[m][j] Gqs(i,m)
-      Auk += row_dot<NQ, VEC>(&s_Gqr[b][el][j][0], DTi);        // sum_m D[m][i] Gqr(m,j)
-      r_Aq[k] = Auk;
-      if constexpr (PF) {
-        if (k == NQ / 2) {
-          cp_async_wait<0>();
-          __syncthreads();   // the next group's copy (both elements of the CTA) is visible
-          gather_next(grp + gridDim.x, (int)((it + 1) % STAGES));
-        }
-      }
-    }
-    // transposed t-direction: r_Aq[m] += sum_k D[k][m] Gqt[k]
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) {
-#pragma unroll
-      for (int m = 0; m < NQ; m += (VEC ? 4 : 1)) {
-        if constexpr (VEC) {
-          const float4 d = *reinterpret_cast<const float4*>(&s_D[k][m]);
-          r_Aq[m] += d.x * Gqt[k];
-          r_Aq[m + 1] += d.y * Gqt[k];
-          r_Aq[m + 2] += d.z * Gqt[k];
-          r_Aq[m + 3] += d.w * Gqt[k];
-        } else {
-          r_Aq[m] += s_D[k][m] * Gqt[k];
-        }
-      }
-    }
-    if (active) {
-#pragma unroll
-      for (int k = 0; k < NQ; ++k)
-        if (r_id[k] >= 0) atomicAdd(out + r_id[k], outScale * r_Aq[k]);
-    }
-  }
-  cp_async_wait<0>();
 }
 
 // ---------------------------------------------------------------- FP64 block fixed-point kernel
@@ -1179,59 +1032,6 @@ int ax_hex_dw(const AxArgs<double, float2>& a, cudaStream_t s) {
   return LPG_OK;
 }
 
-template <int NQ, typename T, typename G, int EPB, int STAGES, bool PF = false, bool MASS = true>
-static int launch_staged(const AxArgs<T, G>& a, cudaStream_t s) {
-  using L = StagedLayout<NQ, G>;
-  constexpr int smem = STAGES * EPB * L::ELEM_BYTES;
-  static PerDeviceConfig perDevice;   // per instantiation: dynamic shared memory opt-in, occupancy
-  auto kern = ax_hex_staged_kernel<NQ, T, G, EPB, STAGES, PF, MASS>;
-  KernelConfig cfg;
-  const int rc = perDevice.get(
-      [&](int, KernelConfig& c) {
-        LPG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        LPG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c.ctasPerSM, kern, NQ * NQ * EPB, smem));
-        if (c.ctasPerSM < 1) return set_error(LPG_ERR_UNSUPPORTED, "staged Ax: kernel does not fit on an SM");
-        return (int)LPG_OK;
-      },
-      &cfg);
-  if (rc) return rc;
-  const int64_t groups = (a.Nelements + EPB - 1) / EPB;
-  const int64_t grid = std::min<int64_t>(groups, (int64_t)cfg.numSMs * cfg.ctasPerSM);
-  if (grid <= 0) return LPG_OK;
-  kern<<<(unsigned)grid, dim3(NQ, NQ, EPB), smem, s>>>(a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ,
-                                                        a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out,
-                                                        a.outScale);
-  LPG_LAUNCH_CHECK("ax_hex_staged_kernel");
-  return LPG_OK;
-}
-
-static int staged_variant() {
-  static int v = -2;
-  if (v == -2) {
-    const char* e = std::getenv("LPG_AX_STAGED");
-    v = -1;
-    if (e) {
-      if (!std::strcmp(e, "off")) v = 0;
-      else if (!std::strcmp(e, "2x2")) v = 22;
-      else if (!std::strcmp(e, "2x3")) v = 23;
-      else if (!std::strcmp(e, "4x2")) v = 42;
-      else if (!std::strcmp(e, "4x3")) v = 43;
-      else if (!std::strcmp(e, "2x2pf")) v = 122;
-    }
-  }
-  return v;
-}
-
-// the staged kernel needs 16-byte aligned rows (even Nq) and aligned strides/pointers
-template <int NQ, typename T, typename G>
-static bool staged_ok(const AxArgs<T, G>& a) {
-  using L = StagedLayout<NQ, G>;
-  if (!L::ok) return false;
-  auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-  return al(a.ggeo) && al(a.wJ) && al(a.g2l) && ((a.geoStride * (int64_t)sizeof(G)) % 16 == 0) &&
-         ((a.wJStride * (int64_t)sizeof(G)) % 16 == 0);
-}
-
 // LPG_AX_FP64 = direct: tuning override back to the direct-contraction FP64 kernel (ax_hex_kernel)
 static bool fp64_direct_override() {
   static const bool direct = [] {
@@ -1282,40 +1082,34 @@ static int launch_line(const AxArgs<float, G>& a, cudaStream_t s) {
     kern<<<(unsigned)blocks, L::NT, 0, s>>>(a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride,
                                             a.D, a.lambda, a.lambdaE, a.q, a.out, a.outScale);
   };
-  if (a.lambda == 0 && !a.lambdaE) go(ax_hex_line_kernel<NQ, G, false>);
-  else go(ax_hex_line_kernel<NQ, G, true>);
+  const bool noMass = a.lambda == 0 && !a.lambdaE;
+  // BF16 factors at Nq = 8, where they start on 16-byte boundaries, are copied: 48^3 322 us against
+  // 357 read where they are used. FP32 factors need twice the shared memory, so fewer CTAs fit: 400
+  // against 383.
+  if constexpr (NQ == 8 && std::is_same<G, __nv_bfloat16>::value) {
+    if (((uintptr_t)a.ggeo & 15) == 0 && ((uintptr_t)a.wJ & 15) == 0 && a.geoStride % 8 == 0 && a.wJStride % 8 == 0) {
+      if (noMass) go(ax_hex_line_kernel<NQ, G, false, true>);
+      else go(ax_hex_line_kernel<NQ, G, true, true>);
+      LPG_LAUNCH_CHECK("ax_hex_line_kernel");
+      return LPG_OK;
+    }
+  }
+  if (noMass) go(ax_hex_line_kernel<NQ, G, false, false>);
+  else go(ax_hex_line_kernel<NQ, G, true, false>);
   LPG_LAUNCH_CHECK("ax_hex_line_kernel");
   return LPG_OK;
 }
 
-// FP32 vectors: the staged kernel at Nq = 8, and at Nq = 4 with FP32 geometry, on 16-byte
-// aligned rows; the line kernel elsewhere. Measured, staged against line, FP32 geometry:
-// 40^3, N = 7 251 against 300 us; 60^3, N = 3 109 against 112; 40^3, N = 5 148 against 141;
-// 100^3, N = 1 222 against 68; BF16 geometry: 60^3, N = 3 107 against 101; 40^3, N = 5 123
-// against 119. The one-layer-at-a-time kernel that served the odd Nq before the line kernel:
-// 48^3, N = 4 151 against 120 us; 30^3, N = 6 130 against 99; 24^3, N = 8 195 against 113;
-// 80^3, N = 2 125 against 118.
+// FP32 vectors. Measured against the kernels before this one, which copied a persistent CTA's
+// next elements to shared memory (Nq = 4, 8) or read D once per direction (the other Nq), us.
+// FP32 geometry: 100^3, N = 1 68.5 -> 66.2; 80^3, N = 2 118 -> 110; 100^3, N = 3 491 -> 411;
+// 48^3, N = 4 119 -> 110; 40^3, N = 5 142 -> 110; 30^3, N = 6 100 -> 83; 48^3, N = 7 425 -> 379;
+// 24^3, N = 8 113 -> 96. BF16 geometry: 60^3, N = 3 101 -> 87; 40^3, N = 5 120 -> 101; 48^3,
+// N = 7 410 -> 323.
 template <int NQ, int INMODE, int OUTMODE, typename G>
 static int launch_ax(const AxArgs<float, G>& a, cudaStream_t s) {
   if constexpr (INMODE == IN_GATHER && OUTMODE == OUT_ASSEMBLE) {
     if (a.Nelements <= 0) return LPG_OK;
-    constexpr bool F32 = std::is_same<G, float>::value;
-    if constexpr (NQ == 8 || (NQ == 4 && F32)) {
-      // LPG_AX_STAGED = off | EPBxSTAGES (2x2, 2x3, 4x2, 4x3) | 2x2pf: tuning override
-      const int v = staged_variant();
-      if (v != 0 && staged_ok<NQ, float, G>(a)) {
-        if (v == 22) return launch_staged<NQ, float, G, 2, 2>(a, s);
-        if (v == 23) return launch_staged<NQ, float, G, 2, 3>(a, s);
-        if (v == 43) return launch_staged<NQ, float, G, 4, 3>(a, s);
-        if (v == 42) return launch_staged<NQ, float, G, 4, 2>(a, s);
-        if (v == 122) return launch_staged<NQ, float, G, 2, 2, true>(a, s);
-        // measured best at N=7: FP32 geometry with the next group's q gathered half-way
-        // through the current group (0.997 vs 1.112 ms at 64^3); BF16 geometry without it
-        // (lambda = 0 without a lambda field: the instantiation without the mass term and wJ copy)
-        const bool noMass = (a.lambda == 0 && !a.lambdaE);
-        return noMass ? launch_staged<NQ, float, G, 2, 2, F32, false>(a, s) : launch_staged<NQ, float, G, 2, 2, F32>(a, s);
-      }
-    }
     return launch_line<NQ, G>(a, s);
   } else {
     return set_error(LPG_ERR_UNSUPPORTED, "ax: FP32 vectors are provided for the assembled operator only");

@@ -128,3 +128,41 @@ def test_scaled_derivative(N, scale):
     mag = _apply(np.abs(G), W, np.abs(D).astype(LD), np.zeros(E, LD), np.abs(u), top=True)
     err = np.abs(out.cpu().numpy().astype(LD) - ref.reshape(-1))
     assert np.all(err <= (2 * Nq + 8 + 1) * 2.0 ** -53 * mag.reshape(-1))
+
+
+@pytest.mark.parametrize("N", range(1, 9))
+@pytest.mark.parametrize("prec", ["f32", "bf16g"])
+@pytest.mark.parametrize("form", ["one", "list", "nomass", "nomass_list"])
+def test_fp32_line_kernel(N, prec, form):
+    """One element, a partly empty last block, aligned element lists, no mass term."""
+    rng = np.random.default_rng(10 * N + len(form))
+    Nq, E = N + 1, 1 if form == "one" else 75
+    Np = Nq ** 3
+    tgeo = torch.bfloat16 if prec == "bf16g" else torch.float32
+    D = rng.uniform(-2, 2, (Nq, Nq)).astype(np.float32)
+    geo = torch.tensor(rng.uniform(-1, 1, (E, 7, Nq, Nq, Nq))).to(tgeo).double().numpy()
+    g2l = rng.integers(-1, 5 * Np, E * Np).astype(np.int32)
+    q = rng.uniform(-1, 1, 5 * Np).astype(np.float32)
+    lam = 0.0 if "nomass" in form else 0.7
+    elems = rng.permutation(E)[:41] if "list" in form else np.arange(E)
+    dG = _off(geo, tgeo, 0)
+    out = torch.empty(5 * Np, dtype=torch.float32, device="cuda")
+    lst = torch.tensor(elems.astype(np.int32), device="cuda") if "list" in form else None
+    lpg.ax_hex(prec, N, len(elems), _off(g2l, torch.int32, 0), dG, 7 * Np, dG[6 * Np:], 7 * Np,
+               _off(D, torch.float32, 0), lam, _off(q, torch.float32, 0), out, 5 * Np, element_list=lst)
+    torch.cuda.synchronize()
+    LD = np.longdouble
+    lams = np.full(len(elems), lam, dtype=np.float32).astype(LD)
+    idx = g2l.reshape(E, Np)[elems]
+    u = np.where(idx < 0, 0, q[np.maximum(idx, 0)]).astype(LD).reshape(-1, Nq, Nq, Nq)
+    G, W, Dl = geo[elems][:, :6].astype(LD), geo[elems][:, 6].astype(LD), D.astype(LD)
+
+    def gather(f):
+        r = np.zeros(5 * Np + 1, dtype=LD)
+        np.add.at(r, np.where(idx < 0, 5 * Np, idx).reshape(-1), f.reshape(-1))
+        return r[:-1]
+
+    ref = gather(_apply(G, W, Dl, lams, u))
+    mag = gather(_apply(np.abs(G), np.abs(W), np.abs(Dl), lams, np.abs(u)))
+    copies = np.bincount(idx[idx >= 0], minlength=5 * Np).max()
+    assert np.all(np.abs(out.cpu().numpy().astype(LD) - ref) <= (2 * Nq + 8 + copies) * 2.0 ** -24 * mag)
