@@ -963,13 +963,12 @@ def main():
     # DRAM bytes per launch: the ncu capture's bytes per element (24^3 case, traffic
     # grows with the element count) times this workload's elements
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", {"f64": "ax_hex_f64_64cubed_N7.txt",
-                                            "f32": "ax_hex_staged_f32_24cubed_N7_full.txt",
-                                            "df64": "ax_hex_dw_24cubed_N7_full.txt",
-                                            "bf16g": "ax_hex_staged_bf16g_24cubed_N7_full.txt"}[a.prec])
+    tfile = os.path.join(ROOT, "profiles", "ax_hex_dw_24cubed_N7_full.txt" if a.prec == "df64"
+                         else "ax_hex_fx_line_24cubed_N7.txt")
+    key = ("" if a.prec == "df64" else a.prec + " ") + "traffic_bytes_per_element:"
     if os.path.exists(tfile) and a.N == 7:
         for line in open(tfile):
-            if line.startswith("traffic_bytes_per_element:"):
+            if line.startswith(key):
                 traffic = float(line.split(":")[1].split()[0]) * a.nx ** 3
     value = job_throughput(Nl, world, ms)
     out = {
@@ -984,7 +983,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
                      "algorithmic_bytes_per_launch": alg_bytes, "launch_ms": launch_ms},
-        "compute": {"arith": {"f64": "fp64", "df64": "double-fp32 words"}.get(a.prec, "fp32"),
+        "compute": {"arith": {"f64": "fp64 (contractions in 64-bit fixed point)", "df64": "double-fp32 words"}.get(a.prec, "fp32"),
                     "flops_per_launch": flops,
                     "achieved_tflops": flops / (launch_ms * 1e-3) / 1e12,
                     "nominal_fp64_tflops": 1.25},

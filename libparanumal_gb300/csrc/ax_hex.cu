@@ -1,16 +1,15 @@
 // Matrix-free screened-Poisson operator on hexahedra (sum-factorised, GLL collocation)
 // with the gather-scatter assembly fused into the kernel.
 //
-// Same arithmetic as ellipticPartialAxHex3D (solvers/elliptic/okl/ellipticAxHex3D.okl:156-295):
-// per element, pencils q(i,j,0:N) live in registers, one k-layer at a time is shared,
-// r/s derivatives come from shared memory, the metric product G*grad is formed per node,
-// and the transposed derivatives accumulate back into the register pencil.
-// Differences for GB300:
-//   * several elements per CTA (NQ*NQ threads each) so a CTA has ~256 threads;
+// Same operator as ellipticPartialAxHex3D (solvers/elliptic/okl/ellipticAxHex3D.okl:156-295):
+// the r, s and t derivatives of an element's lines, the metric product G*grad per node, the
+// transposed derivatives and the mass term. Differences for GB300:
+//   * lines are contracted by one thread each from line-contiguous copies in shared memory,
+//     FP64 ones in block fixed point (ax_hex_fx_kernel, ax_hex_line_kernel);
 //   * the assembled result is accumulated straight into Aq with atomics (the reference
 //     writes AqL, then an ogs Gather kernel re-reads it);
 //   * geometric-factor offsets are 64-bit (the reference's int offsets overflow at 112^3, N=7);
-//   * per-element lambda; FP64, FP32 and BF16-storage variants from one template.
+//   * per-element lambda; FP64, double-word, FP32 and BF16-storage kernels.
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
@@ -150,7 +149,7 @@ template <> __device__ __forceinline__ float geo_to_float<__nv_bfloat16>(__nv_bf
 // memory, contracted in place; a row of D is read once for the three. Two passes (D, D^T) with
 // the metric product between them, 4 barriers an element. Many small CTAs: while some wait for
 // their loads, others compute. 48^3, N = 7 with FP32 factors moves 2.26 GB in 357 us, 0.93 of
-// the measured copy rate; with BF16 factors shared memory bounds it (80 % of its cycles).
+// the measured copy rate (379 with the clearing of out); with BF16 factors shared memory bounds it (80 % of its cycles).
 template <int NQ>
 struct LineLayout {
   static constexpr int NP = NQ * NQ * NQ, NL = NQ * NQ;
