@@ -578,19 +578,23 @@ int MultiGrid::smooth(PLevel& L, const T* r, T* X, bool xIsZero, cudaStream_t s)
   const double invTheta = 1.0 / theta;
   const double sigma = theta / delta;
   double rho_n = 1. / sigma, rho_np1;
-  // same recurrence as the reference's loop (x += d before each application of A, and
-  // once at the end), with each x += d fused into the pass that produced d
-  if (!xIsZero && (rc = op<T>(L.el, X, RES, s))) return rc;
   // C0 levels (but with the double-word operator): the smoother keeps the unscaled residual
   // u = r - A x, which the operator updates in place (u -= A d, assembled straight into it): no
   // A d vector and no clearing of it, and each step pass reads 4 vectors and writes 2 instead
   // of 5 and 3
   bool fused = !L.el->ipdg && !cheb_unfused();
   if constexpr (std::is_same<T, double>::value) fused = fused && L.el->can_subtract();
-  if (fused)
-    rc = cheb_start_u<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s);
-  else
+  // same recurrence as the reference's loop (x += d before each application of A, and
+  // once at the end), with each x += d fused into the pass that produced d, and on x = 0 the
+  // first x = d into the first step
+  const bool deferX = xIsZero && opt.chebDegree > 0;
+  if (fused) {
+    if (!xIsZero && (rc = residual<T>(L.el, r, X, RES, s))) return rc;
+    rc = cheb_start_u<T>(N, invDiag, xIsZero ? r : nullptr, RES, d, deferX ? nullptr : X, (T)invTheta, s);
+  } else {
+    if (!xIsZero && (rc = op<T>(L.el, X, RES, s))) return rc;
     rc = cheb_start<T>(N, invDiag, r, xIsZero ? nullptr : RES, RES, d, X, (T)invTheta, xIsZero, s);
+  }
   if (rc) return rc;
   for (int k = 0; k < opt.chebDegree; ++k) {
     rho_np1 = 1.0 / (2. * sigma - rho_n);
@@ -600,7 +604,9 @@ int MultiGrid::smooth(PLevel& L, const T* r, T* X, bool xIsZero, cudaStream_t s)
       if constexpr (std::is_same<T, float>::value) rc = L.el->OperatorF32(d, RES, opt.prec, s, -1.f);
       else rc = L.el->OperatorSubtract(d, RES, s);
       if (rc) return rc;
-      if ((rc = cheb_step_u<T>(N, invDiag, RES, d, X, (T)(rho_np1 * rho_n), (T)rhoDivDelta, s, last))) return rc;
+      if ((rc = cheb_step_u<T>(N, invDiag, RES, d, X, (T)(rho_np1 * rho_n), (T)rhoDivDelta, s,
+                               deferX && k == 0, last)))
+        return rc;
       rho_n = rho_np1;
       continue;
     }

@@ -172,13 +172,13 @@ template <typename T>
 int cheb_step(int64_t N, const T* invDiag, const T* Ad, T* res, T* d, T* x, T a, T b, cudaStream_t s,
               bool last = false);
 // the same on the unscaled residual u = r - A x, which the operator updates in place
-// (u -= A d): start u = r - Ax (or r), d = invTheta invDiag u, x = d or x += d; step
-// d = a d + b invDiag u, x += d (last: d not written)
+// (u -= A d): start on x = 0 (r given; x null leaves x = d to the first step) u = r,
+// d = invTheta invDiag u, x = d; on x != 0 (r null, u there) d likewise, x += d; step
+// d = a d + b invDiag u, x += d (first: x = old d + d; last: d not written)
 template <typename T>
-int cheb_start_u(int64_t N, const T* invDiag, const T* r, const T* Ax, T* u, T* d, T* x, T invTheta, bool xIsZero,
-                 cudaStream_t s);
+int cheb_start_u(int64_t N, const T* invDiag, const T* r, T* u, T* d, T* x, T invTheta, cudaStream_t s);
 template <typename T>
-int cheb_step_u(int64_t N, const T* invDiag, const T* u, T* d, T* x, T a, T b, cudaStream_t s, bool last = false);
+int cheb_step_u(int64_t N, const T* invDiag, const T* u, T* d, T* x, T a, T b, cudaStream_t s, bool first, bool last);
 
 // ---------------------------------------------------------------- p-multigrid transfers
 // xC = assembled sum over coarse copies of P^T (weightF .* xF) per element (xC overwritten)
