@@ -326,7 +326,8 @@ ipdg_ax_kernel(const T* __restrict__ vgeo, const T* __restrict__ sgeo, const int
 //   rows at the face nodes, the transposed derivatives, and the value terms.
 // A face node needs of its neighbour the value and the normal derivative alone: the two
 // outward normals of a conforming face are opposite, so n . grad q_P is minus the neighbour's
-// own. With f = n . grad q_M + n . grad q_P + tau hinv (q_P - q_M) and g = WsJ / 2 (q_P - q_M)
+// own (a boundary face that the mesh file does not tag is its own neighbour, and takes its own
+// value as it is). With f = n . grad q_M + n . grad q_P + tau hinv (q_P - q_M) and g = WsJ / 2 (q_P - q_M)
 // a face node adds (n . grad r, n . grad s, n . grad t) g to the rows and -WsJ / 2 f to the
 // value.
 //
@@ -435,7 +436,8 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
     const double2 M = tr[f * NL];
     double2 P = trace[mP[f]];
     const int bc = EToB[e * 6 + f];
-    P.x = -P.x;
+    // a face without a neighbour and without a boundary tag pairs with itself: same normal
+    if (mP[f] != (int32_t)(e * NS + f * NL + l)) P.x = -P.x;
     // homogeneous boundary state B (Dirichlet: q = 0, grad kept; Neumann: q kept, grad = 0),
     // mirror state 2B - M
     if (bc > 0) P = bc == 1 ? make_double2(M.x, -M.y) : make_double2(-M.x, M.y);
