@@ -199,23 +199,13 @@ ax_hex_line_kernel(const int64_t Nelements, const int32_t* __restrict__ elementL
   const int64_t nodeBase = e * NP + l;
   if constexpr (!COPY) {
     if ((MASS || NQ < 4) && !elementList && geoStride <= 7 * NP) {
-      // one thread asks for the factors of the CTA's run of elements in L2 (whole 16-byte
-      // units inside the run: the rows need not be aligned)
-      if (tid == 0) {
-        const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
-        const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
-        const uintptr_t hi = (uintptr_t)(ggeo + (e + n) * geoStride) & ~(uintptr_t)15;
-        if (hi > lo) prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
-      }
+      // one thread asks for the factors of the CTA's run of elements in L2
+      if (tid == 0)
+        prefetch_l2_bulk(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride,
+                                       NP, sizeof(G), Nelements - e < EPB ? Nelements - e : EPB, MASS));
     } else if (NQ >= 4 && l == 0 && active) {
-      const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
-      const uintptr_t hi = (uintptr_t)(ggeo + e * geoStride + 6 * NP) & ~(uintptr_t)15;
-      prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
-      if constexpr (MASS) {
-        const uintptr_t lw = ((uintptr_t)(wJ + e * wJStride) + 15) & ~(uintptr_t)15;
-        const uintptr_t hw = (uintptr_t)(wJ + e * wJStride + NP) & ~(uintptr_t)15;
-        prefetch_l2_bulk((const void*)lw, (unsigned)(hw - lw));
-      }
+      prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(G));
+      if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(G));
     }
   }
   int32_t id[NQ];
@@ -419,7 +409,8 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
     }
   } else if (tid == 0 && !elementList && geoStride <= 7 * NP) {
     const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
-    prefetch_l2_bulk(ggeo + e * geoStride, (unsigned)(n * geoStride * sizeof(double)));
+    prefetch_l2_bulk(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride, NP,
+                                   sizeof(double), n, MASS));
     if (MASS && wJStride == NP) prefetch_l2_bulk(wJ + e * NP, (unsigned)(n * NP * sizeof(double)));
   }
   bool plain;
