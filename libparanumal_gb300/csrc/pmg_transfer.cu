@@ -100,59 +100,92 @@ struct LineMatrix<NIN, NOUT, float> {
   }
 };
 
+// The end nodes (and the midpoints, where both degrees are even) are nodes of both levels:
+// their rows of P are rows of the identity. Such values are passed on in FP64, and the integers
+// hold the other entries only, so that every entry of a line counts in every sum and the error is
+// relative to the terms of the sum (rows of P differ by 66 times at most among the others). A P
+// of another kind is contracted in FP64.
 template <int NIN, int NOUT>
 struct LineMatrix<NIN, NOUT, double> {
   // bits of a value and of an entry (fx_hex.cuh, FxLayout): NIN products of each kind per sum
   static constexpr int FS = 7, DS = NIN >= 8 ? 6 : 7, RS = (NIN + 1) & ~1, OFF = 2088 + FS + DS - 1086;
+  static constexpr bool UP = NIN < NOUT;   // prolongation
+  static constexpr int LO = UP ? NIN : NOUT, HI = UP ? NOUT : NIN;
   fx_half tab[NOUT * RS];
-  double c[NOUT * NIN];   // for lines outside the integers' range
+  double c[NOUT * NIN];   // for lines left to FP64
   int ex[NOUT];
+  // the coarse node at fine node i, or -1
+  __host__ __device__ static constexpr int shared(int i) {
+    return i == 0 ? 0 : i == HI - 1 ? LO - 1 : HI % 2 && LO % 2 && 2 * i == HI - 1 ? (LO - 1) / 2 : -1;
+  }
   __device__ __forceinline__ void fill(const double* M, int rs, int cs, int tid, int threads) {
     for (int w = tid; w < NOUT * NIN; w += threads) {
       const int t = w / NIN, m = w % NIN;
-      unsigned key = 0;
+      unsigned key = 0, least = 0x7fffffffu;
+      bool nodal = true;
 #pragma unroll
-      for (int k = 0; k < NIN; ++k) key = max(key, fx_key(M[t * rs + k * cs]));
+      for (int k = 0; k < NIN; ++k) {
+        const double v = M[t * rs + k * cs];
+        const int s = shared(UP ? t : k);
+        if (s >= 0) nodal = nodal && v == (s == (UP ? k : t) ? 1.0 : 0.0);
+        else least = min(least, fx_key(v));
+        if (UP || s < 0) key = max(key, fx_key(v));
+      }
       const int eR = max((int)(key >> 20), 960);
       c[w] = M[t * rs + m * cs];
       tab[t * RS + m] = fx_split(fx_from_double<DS + 1>(c[w], eR));
-      if (m == 0) ex[t] = eR > 1086 || (key >> 20) < 960 ? -1 : eR;
+      if (m == 0) {
+        const bool even = least == 0x7fffffffu || (int)(key >> 20) - (int)(least >> 20) <= 10;
+        ex[t] = !nodal || !even || eR > 1086 || (key >> 20) < 960 ? -1 : eR;
+      }
     }
   }
   template <typename F>
   __device__ __forceinline__ void apply(const double (&x)[NIN], F&& emit) const {
-    unsigned key = 0;
+    unsigned key = 0, ends = 0;
     int lo = 0, plain = 0;
 #pragma unroll
-    for (int m = 0; m < NIN; ++m) key = max(key, fx_key(x[m]));
+    for (int m = 0; m < NIN; ++m) {
+      if (!UP && shared(m) >= 0) {
+        ends = max(ends, fx_key(x[m]));
+        continue;
+      }
+      key = max(key, fx_key(x[m]));
+      lo |= __double2loint(x[m]);
+    }
 #pragma unroll
     for (int t = 0; t < NOUT; ++t) plain |= ex[t];
     const int eL = (int)(key >> 20);
-    if (fx_ordinary(eL) && plain >= 0) {
+    const bool zero = key == 0 && lo == 0;
+    if ((zero || fx_ordinary(eL)) && ends < 0x7ff00000u && plain >= 0) {
       fx_half f[NIN];
 #pragma unroll
-      for (int m = 0; m < NIN; ++m) f[m] = fx_split(fx_from_double<FS + 1>(x[m], eL));
+      for (int m = 0; m < NIN; ++m)
+        if (UP || shared(m) < 0) f[m] = fx_split(fx_from_double<FS + 1>(x[m], eL));
 #pragma unroll
       for (int t = 0; t < NOUT; ++t) {
+        if (UP && shared(t) >= 0) {
+          emit(t, x[UP ? shared(t) : 0]);
+          continue;
+        }
         fx_acc A(0x40000000ll);
         fx_half d[NIN];
 #pragma unroll
         for (int m = 0; m < NIN; ++m) {
+          if (!UP && shared(m) >= 0) continue;
           d[m] = tab[t * RS + m];
           A.cross(f[m], d[m]);
         }
         A.fold();
 #pragma unroll
-        for (int m = 0; m < NIN; ++m) A.high(f[m], d[m]);
-        emit(t, fx_to_double(A.v, fx_base(eL + ex[t] - OFF)));
+        for (int m = 0; m < NIN; ++m)
+          if (UP || shared(m) < 0) A.high(f[m], d[m]);
+        double y = zero ? 0.0 : fx_to_double(A.v, fx_base(eL + ex[t] - OFF));
+#pragma unroll
+        for (int m = 0; m < NIN; ++m)
+          if (!UP && shared(m) == t) y += x[m];
+        emit(t, y);
       }
-      return;
-    }
-#pragma unroll
-    for (int m = 0; m < NIN; ++m) lo |= __double2loint(x[m]);
-    if (key == 0 && lo == 0) {
-#pragma unroll
-      for (int t = 0; t < NOUT; ++t) emit(t, 0.0);
       return;
     }
 #pragma unroll
