@@ -366,6 +366,7 @@ __device__ __forceinline__ void elem_sync(const int el) {
 // lines 1.37 against 1.37 ms.
 // MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
 // UNIT: lambda == 1 without a lambda field, the mass term is wJ q
+// flags: bit 31 the sign bit for out -= A q, bit 0 this library's D
 // W = 3: three threads a line position, each with one direction of the derivatives and a third
 // of the layers, for problems too small to fill the GPU otherwise
 template <int NQ, int W>
@@ -381,7 +382,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
                  const int32_t* __restrict__ g2l, const double* __restrict__ ggeo, const int64_t geoStride,
                  const double* __restrict__ wJ, const int64_t wJStride, const double* __restrict__ Dg,
                  const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
-                 double* __restrict__ out, const int outSign) {
+                 double* __restrict__ out, const unsigned flags) {
   using L = FxLayout<NQ, EO>;
   constexpr int NP = L::NP, NL = L::NL, EPB = FxThreads<NQ, W>::EPB, KN = (NQ + W - 1) / W;
   extern __shared__ __align__(16) unsigned char fx_smem[];
@@ -426,7 +427,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
 #pragma unroll
       for (int i = 0; i < KN; ++i) v[i] = active && inside(i) ? q[nodeBase + layer(i) * NL] : 0.0;
     }
-    plain = fx_tables<NQ, EO>(Dg, tid, FxThreads<NQ, W>::NT, s_tab, s_e);   // while the gather is in flight
+    plain = fx_tables<NQ, EO>(Dg, tid, FxThreads<NQ, W>::NT, s_tab, s_e, flags & 1);   // while the gather is in flight
 #pragma unroll
     for (int i = 0; i < KN; ++i)
       if (inside(i)) E.r(E.a, E.b, layer(i)) = E.s(E.a, E.b, layer(i)) = E.t(E.a, E.b, layer(i)) = v[i];
@@ -485,8 +486,8 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
       r = fma(UNIT ? wp[k * NL] : wp[k * NL] * lam, v, r);
     }
     if constexpr (OUTMODE == OUT_ASSEMBLE) {
-      // outSign: the sign bit for out -= A q
-      if (id[i] >= 0) atomicAdd(out + id[i], __hiloint2double(__double2hiint(r) ^ outSign, __double2loint(r)));
+      if (id[i] >= 0)
+        atomicAdd(out + id[i], __hiloint2double(__double2hiint(r) ^ (int)(flags & 0x80000000u), __double2loint(r)));
     } else if constexpr (OUTMODE == OUT_LOCAL) {
       out[nodeBase + k * NL] = r;
     } else {
@@ -1058,7 +1059,7 @@ static int launch_fx(const AxArgs<double, double>& a, cudaStream_t s) {
   if (blocks > 0x7fffffffLL) return set_error(LPG_ERR_INVALID, "ax: too many elements");
   ax_hex_fx_kernel<NQ, EO, W, INMODE, OUTMODE, MASS, UNIT><<<(unsigned)blocks, L::NT, smem, s>>>(
       a.Nelements, a.elementList, a.g2l, a.ggeo, a.geoStride, a.wJ, a.wJStride, a.D, a.lambda, a.lambdaE, a.q, a.out,
-      a.outScale < 0 ? (int)0x80000000 : 0);
+      (a.outScale < 0 ? 0x80000000u : 0u) | (a.mirrored ? 1u : 0u));
   LPG_LAUNCH_CHECK("ax_hex_fx_kernel");
   return LPG_OK;
 }

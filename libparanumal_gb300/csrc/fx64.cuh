@@ -17,7 +17,9 @@
 // (61 and 1.9 measured), so the three take a tenth of the time of the FP64 FMA they replace.
 //
 // Lines whose largest entry is not in [2^-895, 2^897) (Inf, NaN, subnormals, zero) are left
-// to the caller (fx_ordinary).
+// to the caller (fx_ordinary), and so should be those where one entry outweighs all others
+// together: a sum of which that entry is no part is exact to the unit of the line only, not to
+// that of its own terms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,8 +37,9 @@ __device__ __forceinline__ bool fx_ordinary(int eL) { return (unsigned)(eL - 128
 // the line's largest that nothing is left, zeros and subnormals among them, shift to 0: the
 // PTX shift clamps its amount). Negative values are complemented, not negated: one unit of
 // 2 F, the size of the cut.
+// mag: the high word of the magnitude of 2 F (in [2^(20 + SH), 2^(21 + SH)) for the largest).
 template <int SH>
-__device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
+__device__ __forceinline__ int64_t fx_from_double(double v, int eL, unsigned& mag) {
   const int hi = __double2hiint(v), lo = __double2loint(v);
   const int n = eL - (int)(fx_key(v) >> 20);
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
@@ -45,19 +48,25 @@ __device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
       ".reg .u32 h, l;\n"
       ".reg .s32 s;\n"
       ".reg .u64 m;\n"
-      "shf.l.wrap.b32 h, %2, %1, %5;\n"
-      "shl.b32 l, %2, %5;\n"
+      "shf.l.wrap.b32 h, %3, %2, %6;\n"
+      "shl.b32 l, %3, %6;\n"
       "mov.b64 m, {l, h};\n"
-      "shr.u64 m, m, %3;\n"
-      "shr.s32 s, %4, 31;\n"
+      "shr.u64 m, m, %4;\n"
+      "shr.s32 s, %5, 31;\n"
       "mov.b64 {l, h}, m;\n"
+      "mov.u32 %1, h;\n"
       "xor.b32 l, l, s;\n"
       "xor.b32 h, h, s;\n"
       "mov.b64 %0, {l, h};\n"
       "}\n"
-      : "=l"(F)
+      : "=l"(F), "=r"(mag)
       : "r"(mh), "r"(lo), "r"(n), "r"(hi), "n"(SH));
   return F;
+}
+template <int SH>
+__device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
+  unsigned mag;
+  return fx_from_double<SH>(v, eL, mag);
 }
 
 // base word of fx_to_double for R * 2^(E - 1086), 64 <= E <= 1982 (a normal result)

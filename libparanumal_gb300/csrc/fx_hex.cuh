@@ -68,6 +68,15 @@ struct FxLayout {
   static constexpr int EXP = 2088 + FS + DS + (EO ? 1 : 0);   // of fx_line's unit
   static constexpr int EPB = NL >= 128 ? 1 : (128 + NL / 2) / NL;   // about 128 threads
   static constexpr int NT = NL * EPB;
+  // A line is left to FP64 where the magnitudes of all entries but the largest add up to less
+  // than 2^-T of the power of two under the largest: the derivative at an interior GLL point
+  // leaves the point's own value out (D[i][i] = 0), so the largest entry's own output is made of
+  // the others alone. The largest error of an output relative to its terms is then at most 1.5
+  // times that of an FP64 chain on lines and metric factors over 15 decades (without it, up to
+  // 10^9 times). Of uniform data on a box about 1 line in 30,000 goes that way at N >= 6, 1 in
+  // 10,000 at N = 2. It costs 1 to 3 %: 64^3, N = 7 3.07 -> 3.17 ms; 31 x 23 x 29, N = 5 111.8 ->
+  // 112.9 us. N = 1: every entry of D counts in both outputs.
+  static constexpr int T = NQ == 3 ? 8 : NQ == 4 ? 5 : NQ == 5 ? 4 : NQ == 6 ? 3 : 2;
   // resident CTAs per SM to compile for (registers): measured best of 5 to 10
   static constexpr int MINB = NQ == 9 ? 5 : NQ <= 4 ? 10 : 7;
 };
@@ -91,15 +100,26 @@ __device__ __forceinline__ fx_half fx_table_entry(const double* __restrict__ Dg,
 }
 
 // emit(t, sum_m table[t][m] q[m]) for the outputs t of one line, as integers in units of
-// 2^(eL + eR[t] - EXP)
+// 2^(eL + eR[t] - EXP); key: of the line's largest entry, eL its exponent. false, and nothing
+// emitted, where the line is left to FP64 (T).
 template <int NQ, bool EO, typename F>
-__device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, const fx_half* __restrict__ tab,
+__device__ __forceinline__ bool fx_line(const double (&q)[NQ], const unsigned key, const fx_half* __restrict__ tab,
                                         F&& emit) {
   using L = FxLayout<NQ, EO>;
-  constexpr int N = NQ - 1, H = L::H;
+  constexpr int N = NQ - 1, H = L::H, SH = L::FS + 1;
+  constexpr int HALF = (NQ << (SH - 3)) > 256 ? 1 : 0;   // NQ high words below 2^(21 + SH) add up within 32 bits
   int64_t f[NQ];
+  unsigned sum = 0;
 #pragma unroll
-  for (int m = 0; m < NQ; ++m) f[m] = fx_from_double<L::FS + 1>(q[m], eL);
+  for (int m = 0; m < NQ; ++m) {
+    unsigned mag;
+    f[m] = fx_from_double<SH>(q[m], (int)(key >> 20), mag);
+    sum += mag >> HALF;
+  }
+  if constexpr (NQ > 2) {
+    const unsigned top = ((key & 0xfffffu) | 0x100000u) << (SH - HALF);   // the largest, but for its lowest bits
+    if (sum - top < 1u << (20 + SH - HALF - L::T)) return false;
+  }
   fx_half x[NQ];
   if constexpr (L::EO) {
 #pragma unroll
@@ -164,11 +184,12 @@ __device__ __forceinline__ void fx_line(const double (&q)[NQ], const int eL, con
       emit(t, A.v);
     }
   }
+  return true;
 }
 
 // a line of zeros (as the masked lines of Dirichlet faces are): no magnitude bit is set
 template <int NQ>
-__device__ __forceinline__ bool fx_zero(const double (&v)[NQ], const unsigned key) {
+__device__ __forceinline__ bool fx_zero(const double* v, const unsigned key) {
   int lo = 0;
 #pragma unroll
   for (int m = 0; m < NQ; ++m) lo |= __double2loint(v[m]);
@@ -198,23 +219,29 @@ struct FxElement {
 };
 
 // tables of D and D^T with the exponents of their rows, by the threads of a CTA; true where
-// a row whose largest entry lies outside [2^-63, 2^63] leaves every line to FP64
+// every line is left to FP64: a row's largest entry lies outside [2^-63, 2^63], or an entry off
+// the diagonal is 0 or below 2^-10 of it (a GLL matrix has 2^-6 and more), so that more than its
+// own node's value can be missing in an output
 template <int NQ, bool EO>
 __device__ __forceinline__ bool fx_tables(const double* __restrict__ Dg, const int tid, const int threads,
                                           fx_half (&tab)[2][FxLayout<NQ, EO>::ROWS * FxLayout<NQ, EO>::RS],
-                                          int (&ex)[2][FxLayout<NQ, EO>::ROWS]) {
+                                          int (&ex)[2][FxLayout<NQ, EO>::ROWS], const bool gll) {
   using L = FxLayout<NQ, EO>;
   constexpr int TAB = L::ROWS * NQ;
   bool plain = false;
   for (int w = tid; w < 2 * TAB; w += threads) {
     const int tr = w / TAB, t = (w % TAB) / NQ, c = w % NQ;
-    unsigned key = 0;
+    unsigned key = 0, least = 0x7fffffffu;
 #pragma unroll
-    for (int m = 0; m < NQ; ++m) key = max(key, fx_key(Dg[tr ? m * NQ + t : t * NQ + m]));
+    for (int m = 0; m < NQ; ++m) {
+      const unsigned k = fx_key(Dg[tr ? m * NQ + t : t * NQ + m]);
+      key = max(key, k);
+      if (!gll && (m != t || NQ == 2)) least = min(least, k);
+    }
     const int eR = max((int)(key >> 20), 960) + (L::EO ? 1 : 0);   // 2 Dp, 2 Dm reach twice the row's maximum
     tab[tr][t * L::RS + c] = fx_table_entry<NQ, EO>(Dg, tr, t, c, eR);
     if (c == 0) ex[tr][t] = eR;
-    plain |= eR > 1086 || (key >> 20) < 960;
+    plain |= eR > 1086 || (key >> 20) < 960 || (!gll && (int)(key >> 20) - (int)(least >> 20) > 10);
   }
   return plain;
 }
@@ -236,14 +263,16 @@ __device__ __forceinline__ void fx_forward(const FxElement<NQ>& E, const fx_half
     }
     const int eL = (int)(key >> 20);
     asm volatile("" ::: "memory");   // keeps the table reads of all directions out of registers
-    if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ, EO>(v, eL, tab, [&](int t, int64_t r) {
-        o[t] = fx_to_double(r, fx_base(eL + ex[fx_row<NQ, EO>(t)] - (L::EXP - 1086)));
-      });
-    } else if (fx_zero<NQ>(v, key)) {
+    if (fx_ordinary(eL) && !plain && fx_line<NQ, EO>(v, key, tab, [&](int t, int64_t r) {
+          o[t] = fx_to_double(r, fx_base(eL + ex[fx_row<NQ, EO>(t)] - (L::EXP - 1086)));
+        }))
+      continue;
+    if (fx_zero<NQ>(o, key)) {
 #pragma unroll
       for (int t = 0; t < NQ; ++t) o[t] = 0.0;
     } else {
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) v[m] = o[m];   // not held over the conversion
 #pragma unroll 1
       for (int t = 0; t < NQ; ++t) {
         double r = 0;
@@ -275,15 +304,17 @@ __device__ __forceinline__ bool fx_transposed(const FxElement<NQ>& E, const fx_h
     const int eL = (int)(key >> 20);
     int xl = eL;
     asm volatile("" ::: "memory");
-    if (fx_ordinary(eL) && !plain) {
-      fx_line<NQ, EO>(v, eL, tab, [&](int t, int64_t r) { o[t] = __longlong_as_double(r); });
-    } else if (fx_zero<NQ>(v, key)) {
+    if (fx_ordinary(eL) && !plain &&
+        fx_line<NQ, EO>(v, key, tab, [&](int t, int64_t r) { o[t] = __longlong_as_double(r); })) {
+    } else if (fx_zero<NQ>(o, key)) {
       xl = 128;
 #pragma unroll
       for (int t = 0; t < NQ; ++t) o[t] = 0.0;
     } else {
       xl = -1;
       fp = true;
+#pragma unroll
+      for (int m = 0; m < NQ; ++m) v[m] = o[m];   // not held over the conversion
 #pragma unroll 1
       for (int t = 0; t < NQ; ++t) {
         double r = 0;

@@ -353,7 +353,7 @@ ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, 
     double v[NQ];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
-    plain = fx_tables<NQ, true>(Dg, tid, L::NT, s_tab, s_e);
+    plain = fx_tables<NQ, true>(Dg, tid, L::NT, s_tab, s_e, true);
 #pragma unroll
     for (int k = 0; k < NQ; ++k) S.r(S.a, S.b, k) = S.s(S.a, S.b, k) = S.t(S.a, S.b, k) = v[k];
   }
@@ -407,7 +407,7 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
     double v[NQ];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
-    plain = fx_tables<NQ, true>(Dg, tid, L::NT, s_tab, s_e);
+    plain = fx_tables<NQ, true>(Dg, tid, L::NT, s_tab, s_e, true);
     if (l == 0) s_val[el][4 * NL] = 0.0;
 #pragma unroll
     for (int k = 0; k < NQ; ++k) S.r(a, b, k) = S.s(a, b, k) = S.t(a, b, k) = v[k];
