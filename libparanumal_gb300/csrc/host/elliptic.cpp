@@ -402,29 +402,36 @@ int Elliptic::setup_ipdg(const MeshConfig& c, int N, const std::vector<double>* 
     boxMesh = box_hex_mesh(c.nx, c.ny, c.nz, c.bcflag);
     hm = &boxMesh;
   }
-  std::vector<int32_t> vP, mP;
-  if ((rc = hex_traces(*hm, N, mesh.r1d, vP, mP))) return rc;
+  std::vector<int32_t> mP;
+  if ((rc = hex_traces(*hm, N, mesh.r1d, mP))) return rc;
   hasDirichlet = false;
   for (int b : hm->EToB) hasDirichlet = hasDirichlet || (b == 1);
   EToE_h = hm->EToE;
   std::vector<int32_t> iota(Nlocal);
   for (int64_t n = 0; n < Nlocal; ++n) iota[n] = (int32_t)n;
-  DevBuf<double> hfac;
   if ((rc = g2l.alloc(Nlocal)) || (rc = owner.alloc(Nlocal)) || (rc = weightG.alloc(Nlocal)) ||
-      (rc = vgeo.alloc(E * 10 * Np)) || (rc = sgeo.alloc(E * 5 * 6 * Nfp)) || (rc = fcoef.alloc(E * 5 * 6 * Nfp)) ||
-      (rc = trace.alloc(2 * E * 6 * Nfp)) || (rc = vmapP.alloc(E * 6 * Nfp)) || (rc = mapP.alloc(E * 6 * Nfp)) || (rc = EToB.alloc(E * 6)) ||
-      (rc = hfac.alloc(E * 6 * Nfp)))
+      (rc = vgeo.alloc(E * 10 * Np)) || (rc = sgeo.alloc(E * 5 * 6 * Nfp)) || (rc = trace.alloc(ipdg_trace_size(N, E))) ||
+      (rc = mapP.alloc(E * 6 * Nfp)) || (rc = EToB.alloc(E * 6)))
     return rc;
   if ((rc = g2l.upload(iota.data(), Nlocal, s)) || (rc = owner.upload(iota.data(), Nlocal, s)) ||
-      (rc = vmapP.upload(vP.data(), E * 6 * Nfp, s)) || (rc = mapP.upload(mP.data(), E * 6 * Nfp, s)) ||
+      (rc = mapP.upload(mP.data(), E * 6 * Nfp, s)) ||
       (rc = EToB.upload(hm->EToB.data(), E * 6, s)) || (rc = fill<double>(Nlocal, 1.0, weightG.p, s)))
     return rc;
   tau = 2.0 * (N + 1) * (N + 3);
   IpdgArgs a = ipdg_args();
-  a.hfac = hfac.p;
+  a.hfac = trace.p;   // scratch, as the traces are
   if ((rc = ipdg_geometry(a, s))) return rc;
   if ((rc = finish_setup(lamE, s))) return rc;   // synchronises before the host vectors go
   return LPG_OK;
+}
+
+int Elliptic::make_volume_map(cudaStream_t s) {
+  if (vmapP.p) return LPG_OK;
+  int rc = vmapP.alloc(mapP.n);
+  if (rc) return rc;
+  IpdgArgs a = ipdg_args();
+  a.vmapP = vmapP.p;
+  return ipdg_volume_map(a, s);
 }
 
 IpdgArgs Elliptic::ipdg_args() const {
@@ -433,11 +440,11 @@ IpdgArgs Elliptic::ipdg_args() const {
   a.E = mesh.E;
   a.EX = mesh.EX.p; a.EY = mesh.EY.p; a.EZ = mesh.EZ.p;
   a.D = mesh.D_d.p; a.r1d = mesh.r1d_d.p; a.w1d = mesh.w1d_d.p;
-  a.geo = mesh.geo.p; a.vgeo = vgeo.p; a.sgeo = sgeo.p; a.fcoef = fcoef.p;
+  a.geo = mesh.geo.p; a.vgeo = vgeo.p; a.sgeo = sgeo.p;
   a.mapP = mapP.p; a.EToB = EToB.p;
   a.lambda = lambda; a.tau = tau;
   a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
-  a.trace = reinterpret_cast<double2*>(trace.p);
+  a.trace = trace.p;
   return a;
 }
 
@@ -463,6 +470,7 @@ int Elliptic::make_f32(bool bf16, cudaStream_t s) {
     // FP32 copies of the IPDG volume and surface factors (the C0 geometric factors are not used)
     if (bf16) return set_error(LPG_ERR_UNSUPPORTED, "BF16 geometry is defined for CONTINUOUS only");
     const int64_t E = mesh.E, Np = mesh.Np, Nfp = (int64_t)mesh.Nq * mesh.Nq;
+    if ((rc = make_volume_map(s))) return rc;
     if (!vgeo32.p) {
       if ((rc = vgeo32.alloc(E * 10 * Np)) || (rc = sgeo32.alloc(E * 5 * 6 * Nfp)) || (rc = g4_32.alloc(4 * Nlocal)))
         return rc;
@@ -487,6 +495,7 @@ int Elliptic::make_f32(bool bf16, cudaStream_t s) {
 int Elliptic::OperatorIpdgDW(const double* q, double* Aq, cudaStream_t s) {
   int rc;
   const int64_t E = mesh.E, Np = mesh.Np, Nfp = (int64_t)mesh.Nq * mesh.Nq;
+  if ((rc = make_volume_map(s))) return rc;
   if (!vgeoDW.p) {
     if ((rc = vgeoDW.alloc(E * 10 * Np)) || (rc = sgeoDW.alloc(E * 5 * 6 * Nfp)) || (rc = g8.alloc(8 * Nlocal)))
       return rc;

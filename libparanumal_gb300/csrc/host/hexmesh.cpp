@@ -274,14 +274,12 @@ struct FacePairing {
 
 }  // namespace
 
-int hex_traces(const HexMeshData& m, int N, const std::vector<double>& r1d, std::vector<int32_t>& vmapP,
-               std::vector<int32_t>& mapP) {
+int hex_traces(const HexMeshData& m, int N, const std::vector<double>& r1d, std::vector<int32_t>& mapP) {
   const int Nq = N + 1, Np = Nq * Nq * Nq, Nfp = Nq * Nq;
   const int64_t E = m.E;
   if (E * Np >= (int64_t)INT32_MAX || E * 6 * Nfp >= (int64_t)INT32_MAX)
     return set_error(LPG_ERR_UNSUPPORTED, "more than 2^31 local nodes");
   FacePairing fp(N, r1d);
-  vmapP.resize(E * 6 * Nfp);
   mapP.resize(E * 6 * Nfp);
   for (int64_t e = 0; e < E; ++e)
     for (int f = 0; f < 6; ++f) {
@@ -291,14 +289,7 @@ int hex_traces(const HexMeshData& m, int N, const std::vector<double>& r1d, std:
       if (eP >= 0 && !T) return set_error(LPG_ERR_INVALID, "mesh: face nodes of connected faces do not match");
       for (int n = 0; n < Nfp; ++n) {
         const int64_t id = (e * 6 + f) * Nfp + n;
-        if (eP < 0) {
-          vmapP[id] = (int32_t)(e * Np + fp.faceNodes[f * Nfp + n]);
-          mapP[id] = (int32_t)id;
-        } else {
-          const int q = (*T)[n];
-          vmapP[id] = (int32_t)(eP * Np + fp.faceNodes[fP * Nfp + q]);
-          mapP[id] = (int32_t)((eP * 6 + fP) * Nfp + q);
-        }
+        mapP[id] = eP < 0 ? (int32_t)id : (int32_t)((eP * 6 + fP) * Nfp + (*T)[n]);
       }
     }
   return LPG_OK;

@@ -174,13 +174,14 @@ struct Elliptic {
   // IPDG: unknowns are the local nodes (GlobalToLocal is the identity); face data
   bool ipdg = false;
   double tau = 0;
-  DevBuf<double> vgeo, sgeo, fcoef, trace;   // trace: two values per face node (scratch)
+  DevBuf<double> vgeo, sgeo, trace;     // trace: flux and value per face node (scratch)
   DevBuf<float> vgeo32, sgeo32, g4_32;  // FP32 copies and gradient scratch (preconditioner levels)
   DevBuf<float2> vgeoDW, sgeoDW;        // (hi, lo) copies for OPERATOR PRECISION DF64
   DevBuf<float> g8;                     // double-word gradients, 8 floats per node
   int OperatorIpdgDW(const double* q, double* Aq, cudaStream_t s);
   int64_t nOps = 0;   // applications through Operator and OperatorF32 (any precision)
-  DevBuf<int32_t> vmapP, mapP;
+  DevBuf<int32_t> mapP, vmapP;          // vmapP: made with the first FP32 or double-word copies
+  int make_volume_map(cudaStream_t s);
   DevBuf<int> EToB;
   std::vector<int64_t> EToE_h;     // element neighbours (host), for the matrix probing
   int setup_ipdg(const MeshConfig& c, int N, const std::vector<double>* lamE, cudaStream_t s);

@@ -9,9 +9,9 @@
 //
 // Layout (per element, structure of arrays): vgeo [e][10][Np] = rx ry rz sx sy sz tx ty tz JW;
 // sgeo [e][5][6 Nfp] = nx ny nz WsJ hinv for the face nodes of faces 0..5 (local index order);
-// fcoef [e][5][6 Nfp] = n . grad r, n . grad s, n . grad t, WsJ / 2, tau hinv of the FP64
-// operator. The FP32 preconditioner levels run a gradient and an operator kernel on FP32
-// copies of vgeo and sgeo with float4 gradients.
+// the FP64 operator reads the metric factors of the volume term (geo [e][7][Np]) and WsJ, hinv.
+// The FP32 preconditioner levels run a gradient and an operator kernel on FP32 copies of vgeo
+// and sgeo with float4 gradients.
 //
 // Those kernels run one CTA per element with one thread per node. A node owns its accumulators:
 // the face terms of every face it lies on are added by that node's thread, in the face
@@ -163,25 +163,14 @@ __global__ void ipdg_hinv_kernel(const int64_t nFaceNodes, const int nfpAll, con
   }
 }
 
-// coefficients of the FP64 operator's face terms (n . grad of the reference coordinates,
-// WsJ / 2, tau hinv), so that it needs neither the nine volume factors nor the physical
-// gradient
+// volume node of the paired face node (the FP32 and double-word operators gather volume data)
 template <int NQ>
 __global__ void __launch_bounds__(256)
-ipdg_face_coef_kernel(const int64_t E, const double* __restrict__ vgeo, const double* __restrict__ sgeo,
-                      const double tau, double* __restrict__ fcoef) {
-  constexpr int NP = NQ * NQ * NQ, NFP = NQ * NQ, NS = 6 * NFP;
-  for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < E * NS; id += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = id / NS;
-    const int c = (int)(id % NS);
-    const double* vg = vgeo + e * kVgeo * NP + face_node<NQ>(c / NFP, c % NFP);
-    const double* sg = sgeo + e * kSgeo * NS + c;
-    double* fc = fcoef + e * 5 * NS + c;
-    const double nx = sg[0], ny = sg[NS], nz = sg[2 * NS];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) fc[d * NS] = nx * vg[3 * d * NP] + ny * vg[(3 * d + 1) * NP] + nz * vg[(3 * d + 2) * NP];
-    fc[3 * NS] = 0.5 * sg[3 * NS];
-    fc[4 * NS] = tau * sg[4 * NS];
+ipdg_volume_map_kernel(const int64_t E, const int32_t* __restrict__ mapP, int32_t* __restrict__ vmapP) {
+  constexpr int NP = NQ * NQ * NQ, NFP = NQ * NQ;
+  for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < E * 6 * NFP; id += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t p = mapP[id], face = p / NFP;
+    vmapP[id] = face / 6 * NP + face_node<NQ>(face % 6, p % NFP);
   }
 }
 
@@ -320,26 +309,79 @@ ipdg_ax_kernel(const T* __restrict__ vgeo, const T* __restrict__ sgeo, const int
 
 // ---------------------------------------------------------------- FP64 operator
 // Two kernels with the contractions in block fixed point (fx_hex.cuh), both on the reference
-// derivatives (D_r q, D_s q, D_t q):
-//   traces: (n . grad q, q) at every face node of an element, with its own outward normal;
+// derivatives (D_r q, D_s q, D_t q) and the metric factors G of the volume term alone:
+//   traces: the flux w_end WsJ n . grad q and q at every face node of an element, with its own
+//   outward normal n;
 //   operator: the volume term G . grad q of the C0 operator, the face terms added to the three
 //   rows at the face nodes, the transposed derivatives, and the value terms.
-// A face node needs of its neighbour the value and the normal derivative alone: the two
-// outward normals of a conforming face are opposite, so n . grad q_P is minus the neighbour's
-// own (a boundary face that the mesh file does not tag is its own neighbour, and takes its own
-// value as it is). With f = n . grad q_M + n . grad q_P + tau hinv (q_P - q_M) and g = WsJ / 2 (q_P - q_M)
-// a face node adds (n . grad r, n . grad s, n . grad t) g to the rows and -WsJ / 2 f to the
-// value.
-//
-// Bounded by the FP64 pipe: 9 FP64 operations a node for the metric product, 9 a face node
-// (0.75 face nodes a node at N = 7) and 3 for its trace, 2 or 3 for the sum; against 84 a node
-// of the kernels replaced, which formed physical gradients from the nine volume factors.
+// On the face of direction d (r, s or t) with the outward sign s the normal is s grad d / |grad d|
+// and WsJ = |grad d| J w_a w_b, so WsJ n . grad x = s G_dx / w_end for x = r, s, t, with w_end =
+// 2 / (N (N + 1)) the GLL weight of the face: the flux is s times row d of G . grad q there.
+// Of its neighbour a face node needs the value and the flux: the two outward normals of a
+// conforming face are opposite, so the flux of q_P along this element's normal is minus the
+// neighbour's own (a boundary face that the mesh file does not tag is its own neighbour, and
+// takes its own flux as it is). A face node adds s G_dx / (2 w_end) (q_P - q_M) to the rows x,
+// which is what s / (2 w_end) (q_P - q_M) added to the derivative in direction d becomes in the
+// metric product, and -(flux_M + flux_P) / (2 w_end) - WsJ / 2 tau hinv (q_P - q_M) to the value.
+template <int NQ>
+struct FxFace {
+  static constexpr int N = NQ - 1, NL = NQ * NQ;
+  static constexpr double HALF_INV_W = 0.25 * N * (N + 1);   // 1 / (2 w_end)
+  // rows of G (00, 01, 02, 11, 12, 22) that make row d
+  static __device__ __forceinline__ constexpr int row(int d, int x) { return d + x + (d > 0 && x > 0 ? 1 : 0); }
+  static __device__ __forceinline__ constexpr int dir(int f) { return f == 0 || f == 5 ? 2 : f == 1 || f == 3 ? 1 : 0; }
+  static __device__ __forceinline__ constexpr double sign(int f) { return f == 0 || f == 1 || f == 4 ? -1.0 : 1.0; }
+  // face node (a, b) of face f: its node, and that node's coordinates
+  static __device__ __forceinline__ constexpr int i(int f, int a) { return f == 2 ? N : f == 4 ? 0 : a; }
+  static __device__ __forceinline__ constexpr int j(int f, int a, int b) { return f == 1 ? 0 : f == 3 ? N : f == 2 || f == 4 ? a : b; }
+  static __device__ __forceinline__ constexpr int k(int f, int b) { return f == 0 ? 0 : f == 5 ? N : b; }
+  static __device__ __forceinline__ constexpr int node(int f, int a, int b) { return i(f, a) + NQ * j(f, a, b) + NL * k(f, b); }
+};
+
+// The traces (flux, q): a pair per face node; for N = 1, where every node lies on three faces,
+// the fluxes of all face nodes and then the values of all nodes (less memory: 32 bytes a node
+// instead of 48)
+template <int NQ>
+struct FxTrace {
+  using Face = FxFace<NQ>;
+  static constexpr int NL = NQ * NQ, NS = 6 * NL, NP = NL * NQ;
+  static __device__ __forceinline__ void put(double* trace, int64_t E, int64_t e, int f, int l, int node, double flux, double q) {
+    if constexpr (NQ == 2) {
+      trace[e * NS + f * NL + l] = flux;
+      if (f == 0 || f == 5) trace[E * NS + e * NP + node] = q;
+    } else {
+      reinterpret_cast<double2*>(trace)[e * NS + f * NL + l] = make_double2(flux, q);
+    }
+  }
+  // of face node id; of this element's face node l of face f at `node`
+  static __device__ __forceinline__ double2 get(const double* trace, int64_t E, int32_t id) {
+    if constexpr (NQ == 2) {
+      // node of face node c = id % 24, four bits each
+      const int e = id / NS, c = id - e * NS;
+      const unsigned nodes = c < 8 ? node8(0) : c < 16 ? node8(8) : node8(16);
+      return make_double2(trace[id], trace[E * NS + (int64_t)e * NP + (nodes >> 4 * (c & 7) & 15u)]);
+    } else {
+      return reinterpret_cast<const double2*>(trace)[id];
+    }
+  }
+  static __device__ __forceinline__ double2 own(const double* trace, int64_t E, int64_t e, int f, int l, int node) {
+    if constexpr (NQ == 2) return make_double2(trace[e * NS + f * NL + l], trace[E * NS + e * NP + node]);
+    else return reinterpret_cast<const double2*>(trace)[e * NS + f * NL + l];
+  }
+  static __device__ __forceinline__ constexpr unsigned node8(int c0) {
+    unsigned w = 0;
+    for (int c = c0; c < c0 + 8; ++c) w |= (unsigned)Face::node(c / NL, c % NL % NQ, c % NL / NQ) << 4 * (c - c0);
+    return w;
+  }
+};
+
 template <int NQ>
 __global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB)
-ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, const double* __restrict__ Dg,
-                     const double* __restrict__ q, double2* __restrict__ trace) {
+ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ geo, const double* __restrict__ Dg,
+                     const double* __restrict__ q, double* __restrict__ trace) {
   using L = FxLayout<NQ>;
-  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
+  using Face = FxFace<NQ>;
+  constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB;
   extern __shared__ __align__(16) unsigned char fx_smem[];
   __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::RS];
   __shared__ int s_e[2][L::ROWS];
@@ -348,6 +390,7 @@ ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, 
   const int64_t e = (int64_t)blockIdx.x * EPB + el;
   const bool active = e < Nelements;
   const double* qe = q + e * NP;
+  if (active && l == 0) prefetch_l2_bulk(geo + e * 7 * NP, 3 * NP * sizeof(double));   // the r faces' strided rows
   bool plain;
   {
     double v[NQ];
@@ -361,27 +404,27 @@ ipdg_fx_trace_kernel(const int64_t Nelements, const double* __restrict__ fcoef, 
   fx_forward<NQ, true>(S, s_tab[0], s_e[0], plain, Dg);
   ax_fx_sync<NQ, EPB>(el);
   if (!active) return;
-  const double* fc = fcoef + e * 5 * NS + l;
-  double2* tr = trace + e * NS + l;
+  const double* gp = geo + e * 7 * NP;
 #pragma unroll
   for (int f = 0; f < 6; ++f) {
-    const int i = f == 2 ? N : f == 4 ? 0 : S.a;
-    const int j = f == 1 ? 0 : f == 3 ? N : (f == 2 || f == 4) ? S.a : S.b;
-    const int k = f == 0 ? 0 : f == 5 ? N : S.b;
-    const double* c = fc + f * NL;
-    tr[f * NL] = make_double2(c[0] * S.r(i, j, k) + c[NS] * S.s(i, j, k) + c[2 * NS] * S.t(i, j, k),
-                              qe[i + NQ * j + NL * k]);
+    const int d = Face::dir(f), i = Face::i(f, S.a), j = Face::j(f, S.a, S.b), k = Face::k(f, S.b);
+    const int node = Face::node(f, S.a, S.b);
+    const double* g = gp + node;
+    const double u = g[Face::row(d, 0) * NP] * S.r(i, j, k) + g[Face::row(d, 1) * NP] * S.s(i, j, k) +
+                     g[Face::row(d, 2) * NP] * S.t(i, j, k);
+    FxTrace<NQ>::put(trace, Nelements, e, f, l, node, Face::sign(f) < 0 ? -u : u, qe[node]);
   }
 }
 
 // MASS = false: lambda == 0 and no lambda field
 template <int NQ, bool MASS>
 __global__ void __launch_bounds__(FxLayout<NQ>::NT, FxLayout<NQ>::MINB > 6 ? 6 : FxLayout<NQ>::MINB)
-ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const double* __restrict__ fcoef,
+ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const double* __restrict__ sgeo,
                   const int32_t* __restrict__ mapP, const int* __restrict__ EToB, const double* __restrict__ Dg,
-                  const double lambda, const double* __restrict__ lambdaE, const double* __restrict__ q,
-                  const double2* __restrict__ trace, double* __restrict__ Aq) {
+                  const double halfTau, const double lambda, const double* __restrict__ lambdaE,
+                  const double* __restrict__ q, const double* __restrict__ trace, double* __restrict__ Aq) {
   using L = FxLayout<NQ>;
+  using Face = FxFace<NQ>;
   constexpr int NP = L::NP, NL = L::NL, EPB = L::EPB, N = NQ - 1, NS = 6 * NL;
   extern __shared__ __align__(16) unsigned char fx_smem[];
   __shared__ __align__(16) fx_half s_tab[2][L::ROWS * L::RS];
@@ -395,18 +438,20 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
   const int64_t e = active ? (int64_t)blockIdx.x * EPB + el : 0;
   const double* qe = q + e * NP;
   const double* gp = geo + e * 7 * NP + l;
-  const double* fc = fcoef + e * 5 * NS + l;
-  const double2* tr = trace + e * NS + l;
+  const double* sg = sgeo + (e * kSgeo + 3) * NS;   // WsJ, hinv
   if (active && l == 0) {
     prefetch_l2_bulk(geo + e * 7 * NP, (MASS ? 7 : 6) * NP * sizeof(double));
-    prefetch_l2_bulk(fcoef + e * 5 * NS, 5 * NS * sizeof(double));
+    prefetch_l2_bulk(sg, 2 * NS * sizeof(double));
     prefetch_l2_bulk(mapP + e * NS, NS * sizeof(int32_t));
   }
+  int32_t mP[6];
   bool plain;
   {
     double v[NQ];
 #pragma unroll
     for (int k = 0; k < NQ; ++k) v[k] = active ? qe[l + k * NL] : 0.0;
+#pragma unroll
+    for (int f = 0; f < 6; ++f) mP[f] = __ldg(mapP + e * NS + f * NL + l);
     plain = fx_tables<NQ, true>(Dg, tid, L::NT, s_tab, s_e, true);
     if (l == 0) s_val[el][4 * NL] = 0.0;
 #pragma unroll
@@ -416,9 +461,31 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
   fx_forward<NQ, true>(S, s_tab[0], s_e[0], plain, Dg);
   ax_fx_sync<NQ, EPB>(el);
 
-  int32_t mP[6];   // in flight over the metric product
-#pragma unroll
-  for (int f = 0; f < 6; ++f) mP[f] = __ldg(mapP + e * NS + f * NL + l);
+  // face node l of face f: the jump into the derivative across the face, value term returned
+  auto face = [&](const int f) -> double {
+    const int d = Face::dir(f), i = Face::i(f, a), j = Face::j(f, a, b), k = Face::k(f, b);
+    const double pen = sg[f * NL + l] * (halfTau * sg[NS + f * NL + l]);
+    const int32_t mM = (int32_t)(e * NS + f * NL + l);
+    const double2 M = FxTrace<NQ>::own(trace, Nelements, e, f, l, Face::node(f, a, b));
+    double2 P = FxTrace<NQ>::get(trace, Nelements, mP[f]);
+    const int bc = EToB[e * 6 + f];
+    // a face without a neighbour and without a boundary tag pairs with itself: same normal
+    if (mP[f] != mM) P.x = -P.x;
+    // homogeneous boundary state B (Dirichlet: q = 0, grad kept; Neumann: q kept, grad = 0),
+    // mirror state 2B - M
+    if (bc > 0) P = bc == 1 ? make_double2(M.x, -M.y) : make_double2(-M.x, M.y);
+    const double dq = P.y - M.y;
+    double& u = d == 0 ? S.r(i, j, k) : d == 1 ? S.s(i, j, k) : S.t(i, j, k);
+    u = fma(Face::sign(f) * Face::HALF_INV_W, dq, u);
+    return fma(-pen, dq, -Face::HALF_INV_W * (M.x + P.x));
+  };
+  // no two faces touch the same derivative of a node
+  const double v0 = face(0), v5 = face(5);
+  s_val[el][l] = face(1);
+  s_val[el][NL + l] = face(3);
+  s_val[el][2 * NL + l] = face(2);
+  s_val[el][3 * NL + l] = face(4);
+  ax_fx_sync<NQ, EPB>(el);
 #pragma unroll 4
   for (int k = 0; k < NQ; ++k) {
     const double G00 = gp[0 * NP + k * NL], G01 = gp[1 * NP + k * NL], G02 = gp[2 * NP + k * NL];
@@ -429,33 +496,6 @@ ipdg_fx_ax_kernel(const int64_t Nelements, const double* __restrict__ geo, const
     us = G01 * qr + G11 * qs + G12 * qt;
     ut = G02 * qr + G12 * qs + G22 * qt;
   }
-  // face node l of face f at node (i, j, k): rows in shared memory, value term returned
-  auto face = [&](const int f, const int i, const int j, const int k) -> double {
-    const double* c = fc + f * NL;
-    const double c0 = c[0], c1 = c[NS], c2 = c[2 * NS], hw = c[3 * NS], th = c[4 * NS];
-    const double2 M = tr[f * NL];
-    double2 P = trace[mP[f]];
-    const int bc = EToB[e * 6 + f];
-    // a face without a neighbour and without a boundary tag pairs with itself: same normal
-    if (mP[f] != (int32_t)(e * NS + f * NL + l)) P.x = -P.x;
-    // homogeneous boundary state B (Dirichlet: q = 0, grad kept; Neumann: q kept, grad = 0),
-    // mirror state 2B - M
-    if (bc > 0) P = bc == 1 ? make_double2(M.x, -M.y) : make_double2(-M.x, M.y);
-    const double dq = P.y - M.y, g = hw * dq;
-    double &ur = S.r(i, j, k), &us = S.s(i, j, k), &ut = S.t(i, j, k);
-    ur = fma(c0, g, ur);
-    us = fma(c1, g, us);
-    ut = fma(c2, g, ut);
-    return -hw * fma(th, dq, M.x + P.x);
-  };
-  // opposite faces share no node; the t faces' nodes are this thread's own
-  const double v0 = face(0, a, b, 0), v5 = face(5, a, b, N);
-  ax_fx_sync<NQ, EPB>(el);
-  s_val[el][l] = face(1, a, 0, b);
-  s_val[el][NL + l] = face(3, a, N, b);
-  ax_fx_sync<NQ, EPB>(el);
-  s_val[el][2 * NL + l] = face(2, N, a, b);
-  s_val[el][3 * NL + l] = face(4, 0, a, b);
   ax_fx_sync<NQ, EPB>(el);
   bool fp = fx_transposed<NQ, true>(S, s_tab[1], plain, Dg, s_x[el]);
   fp = ax_fx_sync<NQ, EPB>(el, fp);
@@ -782,10 +822,10 @@ int launch_operator_fx(const IpdgArgs& a, cudaStream_t s) {
       &cfg);
   if (rc) return rc;
   const unsigned blocks = (unsigned)((a.E + L::EPB - 1) / L::EPB);
-  ipdg_fx_trace_kernel<NQ><<<blocks, L::NT, smem, s>>>(a.E, a.fcoef, a.D, a.q, a.trace);
+  ipdg_fx_trace_kernel<NQ><<<blocks, L::NT, smem, s>>>(a.E, a.geo, a.D, a.q, a.trace);
   LPG_LAUNCH_CHECK("ipdg_fx_trace_kernel");
-  ipdg_fx_ax_kernel<NQ, MASS><<<blocks, L::NT, smem, s>>>(a.E, a.geo, a.fcoef, a.mapP, a.EToB, a.D, a.lambda, a.lambdaE,
-                                                          a.q, a.trace, a.out);
+  ipdg_fx_ax_kernel<NQ, MASS><<<blocks, L::NT, smem, s>>>(a.E, a.geo, a.sgeo, a.mapP, a.EToB, a.D, 0.5 * a.tau,
+                                                          a.lambda, a.lambdaE, a.q, a.trace, a.out);
   LPG_LAUNCH_CHECK("ipdg_fx_ax_kernel");
   return LPG_OK;
 }
@@ -807,9 +847,9 @@ int launch_all(int which, const IpdgArgs& a, cudaStream_t s) {
       LPG_LAUNCH_CHECK("ipdg_rhs_bc_kernel");
       return LPG_OK;
     case 3:
-      ipdg_face_coef_kernel<NQ><<<(unsigned)std::min<int64_t>((a.E * 6 * NQ * NQ + 255) / 256, 152 * 16), 256, 0, s>>>(
-          a.E, a.vgeo, a.sgeo, a.tau, a.fcoef);
-      LPG_LAUNCH_CHECK("ipdg_face_coef_kernel");
+      ipdg_volume_map_kernel<NQ><<<(unsigned)std::min<int64_t>((a.E * 6 * NQ * NQ + 255) / 256, 152 * 16), 256, 0, s>>>(
+          a.E, a.mapP, a.vmapP);
+      LPG_LAUNCH_CHECK("ipdg_volume_map_kernel");
       return LPG_OK;
     default:
       ipdg_diag_kernel<NQ><<<E, NP, 0, s>>>(a.vgeo, a.sgeo, a.EToB, a.D, a.lambda, a.lambdaE, a.tau, a.out);
@@ -843,7 +883,7 @@ int ipdg_geometry(const IpdgArgs& a, cudaStream_t s) {
   const int64_t blocks = std::min<int64_t>((nf + 255) / 256, 152 * 16);
   ipdg_hinv_kernel<<<(unsigned)blocks, 256, 0, s>>>(nf, nfpAll, a.hfac, a.mapP, a.sgeo);
   LPG_LAUNCH_CHECK("ipdg_hinv_kernel");
-  return dispatch(3, a, s);
+  return LPG_OK;
 }
 int ipdg_operator(const IpdgArgs& a, cudaStream_t s) { return dispatch(1, a, s); }
 int ipdg_operator_dw(const IpdgArgsDW& a, cudaStream_t s) {
@@ -900,6 +940,7 @@ int ipdg_operator_f32(const IpdgArgsF32& a, cudaStream_t s) {
   }
 }
 int ipdg_rhs_bc(const IpdgArgs& a, cudaStream_t s) { return dispatch(2, a, s); }
+int ipdg_volume_map(const IpdgArgs& a, cudaStream_t s) { return dispatch(3, a, s); }
 int ipdg_diagonal(const IpdgArgs& a, cudaStream_t s) { return dispatch(4, a, s); }
 
 }  // namespace lpg

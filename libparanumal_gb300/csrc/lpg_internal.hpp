@@ -219,20 +219,21 @@ int nb_directions(int64_t N, double beta, const double* u, const double* w, doub
 // ---------------------------------------------------------------- IPDG
 // Interior-penalty DG operator pieces (DISCRETIZATION = IPDG); unknowns are the E*Np
 // local nodes. vgeo [e][10][Np] (rx..tz, JW), sgeo [e][5][6 Nfp] (nx, ny, nz, WsJ, hinv),
-// fcoef [e][5][6 Nfp] (ipdg_hex.cu), mapP [e][6][Nfp] (paired face node), EToB [e][6], geo
-// [e][7][Np] (G00..G22, wJ), trace [E 6 Nfp] scratch.
+// mapP [e][6][Nfp] (paired face node), vmapP [e][6][Nfp] (its volume node), EToB [e][6], geo
+// [e][7][Np] (G00..G22, wJ), trace scratch of ipdg_trace_size() doubles (E 6 Nfp at least).
 struct IpdgArgs {
   int N = 0;
   int64_t E = 0;
   const double *EX = nullptr, *EY = nullptr, *EZ = nullptr, *D = nullptr, *r1d = nullptr, *w1d = nullptr;
   const double* geo = nullptr;
-  double *vgeo = nullptr, *sgeo = nullptr, *fcoef = nullptr, *hfac = nullptr;
+  double *vgeo = nullptr, *sgeo = nullptr, *hfac = nullptr;
   const int32_t* mapP = nullptr;
+  int32_t* vmapP = nullptr;
   const int* EToB = nullptr;
   double lambda = 0, tau = 0;
   const double* lambdaE = nullptr;
   const double* q = nullptr;
-  double2* trace = nullptr;
+  double* trace = nullptr;
   double* out = nullptr;
 };
 // the operator on FP32 copies of vgeo, sgeo, D and lambdaE (preconditioner levels)
@@ -265,8 +266,12 @@ struct IpdgArgsDW {
   double* out = nullptr;
 };
 int ipdg_operator_dw(const IpdgArgsDW& a, cudaStream_t s);
-// vgeo, sgeo, fcoef (hfac = scratch [E][6 Nfp])
+// vgeo, sgeo (hfac = scratch [E][6 Nfp])
 int ipdg_geometry(const IpdgArgs& a, cudaStream_t s);
+inline int64_t ipdg_trace_size(int N, int64_t E) {
+  return N == 1 ? E * (24 + 8) : 2 * E * 6 * (N + 1) * (N + 1);
+}
+int ipdg_volume_map(const IpdgArgs& a, cudaStream_t s);  // vmapP from mapP
 int ipdg_operator(const IpdgArgs& a, cudaStream_t s);   // out = A q (trace scratch)
 int ipdg_rhs_bc(const IpdgArgs& a, cudaStream_t s);     // out -= boundary data terms
 int ipdg_diagonal(const IpdgArgs& a, cudaStream_t s);   // out = diag(A)
