@@ -71,12 +71,14 @@ struct FxLayout {
   // A line is left to FP64 where the magnitudes of all entries but the largest add up to less
   // than 2^-T of the power of two under the largest: the derivative at an interior GLL point
   // leaves the point's own value out (D[i][i] = 0), so the largest entry's own output is made of
-  // the others alone. The largest error of an output relative to its terms is then at most 1.5
+  // the others alone. The largest error of an output relative to its terms is then at most 3
   // times that of an FP64 chain on lines and metric factors over 15 decades (without it, up to
-  // 10^9 times). Of uniform data on a box about 1 line in 30,000 goes that way at N >= 6, 1 in
-  // 10,000 at N = 2. It costs 1 to 3 %: 64^3, N = 7 3.07 -> 3.17 ms; 31 x 23 x 29, N = 5 111.8 ->
-  // 112.9 us. N = 1: every entry of D counts in both outputs.
-  static constexpr int T = NQ == 3 ? 8 : NQ == 4 ? 5 : NQ == 5 ? 4 : NQ == 6 ? 3 : 2;
+  // 10^9 times), and below it for the metric of any usual element. N = 1: every entry of D counts
+  // in both outputs. One line in FP64 holds up its element by 1 to 2 us, so T is the largest that
+  // keeps the 3: with one less a problem of one wave has such a line and takes 5 to 8 % more (16^3,
+  // N = 5 and 4; 10^3, N = 6). The test itself costs 1 to 3 % of large problems: 64^3, N = 7
+  // 3.07 -> 3.17 ms; 31 x 23 x 29, N = 5 111.8 -> 112.9 us.
+  static constexpr int T = NQ == 3 ? 8 : NQ == 4 ? 6 : NQ == 5 ? 5 : NQ == 6 ? 4 : 3;
   // resident CTAs per SM to compile for (registers): measured best of 5 to 10
   static constexpr int MINB = NQ == 9 ? 5 : NQ <= 4 ? 10 : 7;
 };
