@@ -509,7 +509,8 @@ __device__ __forceinline__ void eo_sync(const int el) {
 }
 
 // ---------------------------------------------------------------- double-word variant
-// The even-odd kernel above with every FP64 value held as a double-FP32 word (df64.cuh):
+// Layer by layer, contracted through the mirror symmetry of D (even and odd parts of a line, its
+// two halves exchanged by shuffles), every value held as a double-FP32 word (df64.cuh):
 // FP64-accurate (48-bit significands, sums with absolute error of order 2^-48 times the
 // magnitudes summed) on GB300's FP32 pipe, which runs ~64x the FP64 rate. q is read as
 // FP64 and split with integer operations; the geometric factors come pre-split

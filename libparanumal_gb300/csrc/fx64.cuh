@@ -69,7 +69,8 @@ __device__ __forceinline__ int64_t fx_from_double(double v, int eL) {
   return fx_from_double<SH>(v, eL, mag);
 }
 
-// base word of fx_to_double for R * 2^(E - 1086), 64 <= E <= 1982 (a normal result)
+// base word of fx_to_double for R * 2^(E - 1086): a normal result for 64 <= E <= 2047 (a line's
+// exponent reaches 1919, a row's 1086: E <= 1990 in the operators and transfers)
 __device__ __forceinline__ int fx_base(int E) { return (E - 1) << 20; }
 
 // R * 2^(E - 1086), |R| < 2^63, rounded to nearest: |R| is shifted so that its leading bit

@@ -522,7 +522,7 @@ int Elliptic::OperatorDW(const double* q, double* Aq, cudaStream_t s, bool zeroe
   const int64_t Np = mesh.Np;
   a.N = mesh.N; a.Nelements = mesh.E; a.elementList = elemOrder.p; a.g2l = g2l.p;
   a.ggeo = mesh.geoDW.p; a.geoStride = 7 * Np; a.wJ = mesh.geoDW.p + 6 * Np; a.wJStride = 7 * Np;
-  a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
+  a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
   a.q = q; a.out = Aq; a.Nglobal = zeroed ? 0 : Nglobal;
   return ax_hex_dw(a, s);
 }
@@ -719,15 +719,15 @@ int Elliptic::OperatorHost(const double* qHost, double* AqHost, cudaStream_t s) 
       AxArgs<double, float2> a;
       a.N = mesh.N; a.Nelements = a1 - a0; a.g2l = g2l.p + a0 * Np;
       a.ggeo = mesh.geoDW.p + a0 * 7 * Np; a.geoStride = 7 * Np; a.wJ = a.ggeo + 6 * Np; a.wJStride = 7 * Np;
-      a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
+      a.D = mesh.D_d.p; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
       a.q = pipe->q.p; a.out = pipe->Aq.p; a.Nglobal = 0;   // accumulate: the pipeline zeroed Aq
       return ax_hex_dw(a, s);
     }
-    AxArgs<double, double> a;
-    a.N = mesh.N; a.Nelements = a1 - a0; a.g2l = g2l.p + a0 * Np;
-    a.ggeo = mesh.geo.p + a0 * 7 * Np; a.geoStride = 7 * Np; a.wJ = a.ggeo + 6 * Np; a.wJStride = 7 * Np;
-    a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p + a0 : nullptr;
-    a.q = pipe->q.p; a.out = pipe->Aq.p; a.Nglobal = Nglobal;
+    AxArgs<double, double> a = ax_args();
+    a.Nelements = a1 - a0; a.elementList = nullptr;
+    a.g2l += a0 * Np; a.ggeo += a0 * 7 * Np; a.wJ += a0 * 7 * Np;
+    if (a.lambdaE) a.lambdaE += a0;
+    a.q = pipe->q.p; a.out = pipe->Aq.p;
     return ax_hex<double, double>(a, AxMode::AccumulateAssembled, s);
   };
   return run_pipe<double>(*pipe, pipe->native, qHost, AqHost, pipe->q.p, pipe->Aq.p, Nglobal, s, launch);
@@ -801,11 +801,8 @@ int Elliptic::BuildRhs(double* r, cudaStream_t s) {
   }
   if (rhsKind == 0 && hasDirichlet && !ipdg) {
     // Dirichlet lifting rhs -= A_e g (ellipticRhsBCHex3D.okl:60-290)
-    AxArgs<double, double> a;
-    const int64_t Np = mesh.Np;
-    a.N = mesh.N; a.Nelements = mesh.E; a.g2l = g2l.p;
-    a.ggeo = mesh.geo.p; a.geoStride = 7 * Np; a.wJ = mesh.geo.p + 6 * Np; a.wJStride = 7 * Np;
-    a.D = mesh.D_d.p; a.mirrored = true; a.lambda = lambda; a.lambdaE = hasLambdaE ? lambdaE.p : nullptr;
+    AxArgs<double, double> a = ax_args();
+    a.elementList = nullptr;
     a.q = gL.p; a.out = rL.p;
     if ((rc = ax_hex<double, double>(a, AxMode::LocalInSubtract, s))) return rc;
   }

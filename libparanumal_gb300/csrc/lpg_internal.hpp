@@ -22,7 +22,7 @@ struct AxArgs {
   const G* wJ = nullptr;
   int64_t wJStride = 0;
   const T* D = nullptr;
-  bool mirrored = false;   // D[N-i][N-m] == -D[i][m] exactly (this library's D)
+  bool mirrored = false;   // D[N-i][N-m] == -D[i][m] exactly (this library's D); read by the FP64 kernels
   T lambda = 0;
   const T* lambdaE = nullptr;
   const T* q = nullptr;
