@@ -356,13 +356,13 @@ __device__ __forceinline__ void elem_sync(const int el) {
 //   transposed derivatives as integers (exponents in s_x), summed on their common exponent.
 // q is gathered again for the mass term.
 //
-// What bounds it (N = 7): the FP64 pipe again, at the 9 FP64 operations a node of the metric
-// product and 1 of the mass term against 50 of the FP64 kernel it replaced, closely followed
-// by the integer pipe (shifts, logic and multiply-adds share 64 lanes a clock; 520
-// instructions a node in all). 48^3, N = 7: 1.31 ms (lambda = 0: 1.20)
-// against 4.78 (4.56); 28^3, N = 5: 156 us against 406 us; 64^3, N = 3: 340 us against 1037 us
-// of the direct kernel. Measured and not kept at 48^3: L2 prefetch of a later element's factors
-// (one wave ahead) 1.53 against 1.37 ms; eight CTAs per SM with swizzled instead of pitched
+// What bounds it (N = 7): the FP64 pipe, at the 9 FP64 operations a node of the metric product and
+// 1 of the mass term against 50 of the FP64 kernel it replaced, closely followed by the integer
+// pipe (shifts, logic and multiply-adds share 64 lanes a clock; 537 instructions a node in all): 64
+// and 57 % busy, with barriers between the two. 48^3, N = 7: 1.36 ms (lambda = 0: 1.22) against
+// 4.79 (4.70) of that kernel; 28^3, N = 5: 134 us against 406; 64^3, N = 3: 334 us against 1099;
+// 20^3, N = 8: 199 us against 699. Measured and not kept at 48^3: L2 prefetch of a later element's
+// factors (one wave ahead) 1.53 against 1.37 ms; eight CTAs per SM with swizzled instead of pitched
 // lines 1.37 against 1.37 ms.
 // MASS = false: lambda == 0 and no lambda field, the mass term and its wJ reads are left out
 // UNIT: lambda == 1 without a lambda field, the mass term is wJ q

@@ -323,6 +323,12 @@ ipdg_ax_kernel(const T* __restrict__ vgeo, const T* __restrict__ sgeo, const int
 // takes its own flux as it is). A face node adds s G_dx / (2 w_end) (q_P - q_M) to the rows x,
 // which is what s / (2 w_end) (q_P - q_M) added to the derivative in direction d becomes in the
 // metric product, and -(flux_M + flux_P) / (2 w_end) - WsJ / 2 tau hinv (q_P - q_M) to the value.
+//
+// What bounds them (24^3, N = 7, 333 us against 947 of the gradient and ax kernels before): the
+// operator the FP64 pipe (82 % busy), at 9 FP64 operations a node for the metric product, 2 or 3 for
+// the sum and 8 a face node (0.75 face nodes a node at N = 7); the traces the integer pipe (55 %)
+// and the latency of their loads. With stored coefficients of the face terms (n . grad r, s, t, WsJ / 2,
+// tau hinv) instead the two took 331 us and 33 bytes a node more.
 template <int NQ>
 struct FxFace {
   static constexpr int N = NQ - 1, NL = NQ * NQ;

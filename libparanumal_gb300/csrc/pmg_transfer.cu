@@ -67,10 +67,10 @@ pmg_coarsen_kernel(const int NqF, const int NqC, const int32_t* __restrict__ g2l
 //
 // FP64 contracts in block fixed point (fx64.cuh): with FP64 products the 7 <-> 3 transfers were
 // bound by the FP64 pipe (8 operations a fine node). 20^3 elements, FP64, us before -> now:
-// restriction 64.8 -> 31.8, prolongation 68.3 -> 43.8, 3 <-> 1 9.7 -> 8.4 and 9.6 -> 9.6; 32^3, FP32
+// restriction 65.9 -> 31.5, prolongation 65.8 -> 31.0, 3 <-> 1 12.4 -> 11.4 and 10.4 -> 8.3; 32^3, FP32
 // (strided shared-memory operands before): 65.2 -> 36.6, 85.1 -> 47.6, 10.5 -> 9.3, 13.0 -> 9.7.
 // Now bound by the gathers: the prolongation of 20^3 in FP64 moves at least 85 MB in
-// 43.8 us. All other pairs take the generic kernels.
+// 31.0 us. All other pairs take the generic kernels.
 template <int NQF, int NQC>
 struct TransferLayout {
   static constexpr int NL = NQF * NQF, P = NQF | 1;        // fine lines; odd pitch of every line
