@@ -201,11 +201,17 @@ ax_hex_line_kernel(const int64_t Nelements, const int32_t* __restrict__ elementL
     if ((MASS || NQ < 4) && !elementList && geoStride <= 7 * NP) {
       // one thread asks for the factors of the CTA's run of elements in L2
       if (tid == 0)
-        prefetch_l2_bulk(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride,
+        prefetch_l2_run(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride,
                                        NP, sizeof(G), Nelements - e < EPB ? Nelements - e : EPB, MASS));
     } else if (NQ >= 4 && l == 0 && active) {
-      prefetch_l2_bulk(ggeo + e * geoStride, 6 * NP * sizeof(G));
-      if constexpr (MASS) prefetch_l2_bulk(wJ + e * wJStride, NP * sizeof(G));
+      const uintptr_t lo = ((uintptr_t)(ggeo + e * geoStride) + 15) & ~(uintptr_t)15;
+      const uintptr_t hi = (uintptr_t)(ggeo + e * geoStride + 6 * NP) & ~(uintptr_t)15;
+      prefetch_l2_bulk((const void*)lo, (unsigned)(hi - lo));
+      if constexpr (MASS) {
+        const uintptr_t lw = ((uintptr_t)(wJ + e * wJStride) + 15) & ~(uintptr_t)15;
+        const uintptr_t hw = (uintptr_t)(wJ + e * wJStride + NP) & ~(uintptr_t)15;
+        prefetch_l2_bulk((const void*)lw, (unsigned)(hw - lw));
+      }
     }
   }
   int32_t id[NQ];
@@ -410,7 +416,7 @@ ax_hex_fx_kernel(const int64_t Nelements, const int32_t* __restrict__ elementLis
     }
   } else if (tid == 0 && !elementList && geoStride <= 7 * NP) {
     const int64_t n = Nelements - e < EPB ? Nelements - e : EPB;
-    prefetch_l2_bulk(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride, NP,
+    prefetch_l2_run(l2_factor_run((uint64_t)(ggeo + e * geoStride), geoStride, (uint64_t)(wJ + e * wJStride), wJStride, NP,
                                    sizeof(double), n, MASS));
     if (MASS && wJStride == NP) prefetch_l2_bulk(wJ + e * NP, (unsigned)(n * NP * sizeof(double)));
   }

@@ -21,13 +21,15 @@
 
 namespace lpg {
 
-// L2 prefetch of whole 16-byte units of global memory, as the bulk prefetch requires
-__device__ __forceinline__ void prefetch_l2_bulk(const L2Run r) {
+// L2 prefetch of `bytes` (a multiple of 16) from global memory; skipped unless the address
+// is 16-byte aligned, as the bulk prefetch requires
+__device__ __forceinline__ void prefetch_l2_bulk(const void* gmem, unsigned bytes) {
+  if (((uintptr_t)gmem & 15u) == 0 && (bytes & 15u) == 0)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2_run(const L2Run r) {
   if (r.bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(r.lo), "r"((unsigned)r.bytes) : "memory");
-}
-__device__ __forceinline__ void prefetch_l2_bulk(const void* gmem, unsigned bytes) {
-  prefetch_l2_bulk(l2_units((uint64_t)gmem, bytes));
 }
 // Barrier over the threads of one element where they are whole warps, else over the CTA;
 // returns whether `any` was set by one of them. The barrier numbers are immediates: a number
